@@ -36,7 +36,7 @@ extern "C" {
 #define IRS_FULLFADDEEVA  3
 
 /* arithmetic of the line sum */
-#define IRS_FP64          0   /* FP64 everywhere: the plain GPU kernel                  */
+#define IRS_FP64          0   /* FP64 everywhere (distant lines' wings interpolated to rounding) */
 #define IRS_MIXED         1   /* FP32 Faddeeva + Kahan-compensated FP32 line sum; the far
                                  wings of lines >= 640 grid points from a 256-point block
                                  are summed at 8 Chebyshev nodes and interpolated        */

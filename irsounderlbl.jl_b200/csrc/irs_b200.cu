@@ -12,6 +12,7 @@
 #include "irs_internal.h"
 #include "lineparams.cuh"
 #include "linesum.cuh"
+#include "linesum_tree64.cuh"
 #include "rte_ils.cuh"
 #include "jacobian.cuh"
 #include "oe.cuh"
@@ -173,11 +174,82 @@ static std::vector<ListDev> list_descs(irs_ctx* ctx) {
     return v;
 }
 
+// tree64: points per leaf (one warp).  128 points cost the least per point, but a short
+// grid then has too few leaves to fill the chip; the rule counts the leaves of one
+// profile's layers (not of the batch, so that a profile's result does not depend on it).
+// Measured as whole calls, 32- against 128-point leaves: cross sections of 20,000 lines on
+// 5,501 points 152 / 184 us (0.01 cm^-1 steps 165 / 262), 100,000 points 263 / 281,
+// 300,000 points 474 / 487; 846,001 points (6,610 leaves of 128) 1309 / 1212; 34,801 points
+// x 49 layers (13,328 leaves) 2.9 / 1.1 ms.
+static int t64_leaf_points(int64_t n_nu, int L) { return (n_nu + 127) / 128 * (int64_t)L >= 148 * 16 ? 128 : 32; }
+static size_t t64_cell_bytes(bool lm) { return kT64Nodes * sizeof(double) * (lm ? 2 : 1) + sizeof(int4); }
+static int64_t t64_groups(int64_t n_nu, int leaf) { return 4 * ((n_nu + 16 * leaf - 1) / (16 * leaf)); }
+
+// The FP64 line sum on a uniform grid (linesum_tree64.cuh): the far-field pre-pass and the
+// leaf kernel, in groups of profile-layers whose node values fit ctx->strip_buf_max (one
+// profile-layer beyond it runs without the pre-pass, every far line at its leaf's nodes).
+// With d_uniform the kernels return at once unless *d_uniform is set.
+static void tree64_launch(irs_ctx* ctx, const Plan& pl, const std::vector<int>& first, const SegDev* d_segs,
+                          const int* d_count, const unsigned* d_reach, const int2* d_pl, const LpOutF64& o64,
+                          const double* d_grid, int64_t n_nu, double grid0, double dnu, const irs_fm_options& o,
+                          double* d_tau, double* d_pert, long long pstride, unsigned long long* d_eval,
+                          const int* d_uniform) {
+    static_assert(sizeof(T64Tables) == kT64TableDoubles * sizeof(double), "table layout");
+    cudaStream_t st = ctx->stream;
+    const bool have = ctx->work.count("t64_tables") != 0;
+    T64Tables* d_tab = (T64Tables*)workspace(ctx, "t64_tables", sizeof(T64Tables));
+    if (!have) {
+        std::vector<double> h(kT64TableDoubles);
+        t64_tables(h.data());
+        IRS_CUDA(cudaMemcpyAsync(d_tab, h.data(), sizeof(T64Tables), cudaMemcpyHostToDevice, st));
+        IRS_CUDA(cudaStreamSynchronize(st));
+    }
+    const bool lm = o.line_mixing == IRS_LM_PER_LINE_Y;
+    const int npl = pl.n_prof * pl.L, leaf = t64_leaf_points(n_nu, pl.L);
+    const int n_groups = (int)t64_groups(n_nu, leaf);
+    const size_t cell_bytes = t64_cell_bytes(lm);
+    const size_t max_cells = std::min((size_t)first[npl] * n_groups, ctx->strip_buf_max / cell_bytes);
+    char* buf = (char*)workspace(ctx, "t64_far", max_cells * cell_bytes);
+    for (int pa = 0; pa < npl;) {
+        int pb = pa;
+        const int s_a = first[pa];
+        while (pb < npl && (size_t)(first[pb + 1] - s_a) * n_groups <= max_cells) ++pb;
+        if (pb == pa) pb = pa + 1;
+        const int ns = first[pb] - s_a;
+        const size_t cells = (size_t)ns * n_groups;
+        double *far = nullptr, *farD = nullptr;
+        int4* rng = nullptr;
+        if (cells <= max_cells && ns > 0) {
+            rng = (int4*)buf;
+            far = (double*)(buf + cells * sizeof(int4));
+            farD = lm ? far + cells * kT64Nodes : nullptr;
+            const dim3 gf(n_groups / 4, ns);
+            if (lm) tree64_far_kernel<true><<<gf, 32 * kT64Warps, 0, st>>>(d_segs, d_count, d_reach, o64, grid0, dnu, o.cutoff, leaf, d_tab, far, farD, rng, s_a, d_uniform, d_eval);
+            else tree64_far_kernel<false><<<gf, 32 * kT64Warps, 0, st>>>(d_segs, d_count, d_reach, o64, grid0, dnu, o.cutoff, leaf, d_tab, far, farD, rng, s_a, d_uniform, d_eval);
+            check_launch(ctx);
+        }
+        const dim3 gl((unsigned)((n_nu + 4 * leaf - 1) / (4 * leaf)), pb - pa);
+#define IRS_T64(M, Q, LMX)                                                                                                  tree64_leaf_kernel<M, Q, LMX><<<gl, 32 * kT64LeafWarps, sizeof(T64Leaf<Q, LMX>) * kT64LeafWarps, st>>>(                     d_segs, d_count, d_reach, d_pl, o64, d_grid, n_nu, grid0, dnu, o.cutoff, o.x_far, d_tab, far, farD, rng, n_groups,         pa, s_a, d_tau, d_pert, pstride, d_uniform, d_eval)
+        if (leaf == 128) {
+            if (o.method == IRS_WEIDEMAN) IRS_T64(1, 4, false);
+            else if (lm) IRS_T64(3, 4, true);
+            else IRS_T64(3, 4, false);
+        } else {
+            if (o.method == IRS_WEIDEMAN) IRS_T64(1, 1, false);
+            else if (lm) IRS_T64(3, 1, true);
+            else IRS_T64(3, 1, false);
+        }
+#undef IRS_T64
+        check_launch(ctx);
+        pa = pb;
+    }
+}
+
 // Runs the line-parameter passes and the line sum for the plan; returns the
 // device tau buffer ([n_prof * L][n_nu], FP32 for mixed or FP64 for plain).
 static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n_nu, double grid0,
                          double dnu_g, const irs_fm_options& o, int ev_mid, double* d_pert = nullptr,
-                         long long pstride = 0) {
+                         long long pstride = 0, const int* d_uniform = nullptr) {
     cudaStream_t st = ctx->stream;
     const int nseg = (int)pl.segs.size();
     std::vector<SegDev> sd(std::max(nseg, 1));
@@ -228,13 +300,17 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
     LpOutMixed om{};
     const size_t S = (size_t)pl.slots;
     if (!mixed) {
-        double* base = (double*)workspace(ctx, "lp64", S * 6 * sizeof(double));
+        double* base = (double*)workspace(ctx, "lp64", S * kLpF64 * sizeof(double));
         o64.nu0 = base; o64.f = base + S; o64.y = base + 2 * S; o64.Sn = base + 3 * S;
         o64.Hc = base + 4 * S; o64.YSn = base + 5 * S;
-        lp_write_kernel<0><<<g1, kLpThreads, 0, st>>>(d_segs, d_lists, tp, cfg, d_keep, d_chunk, n_chunks,
-                                                      d_count, o64, om, d_pairs, nullptr);
+        o64.b = base + 6 * S; o64.k0 = base + 7 * S; o64.g = base + 8 * S;
     }
-    unsigned* d_reach = nullptr;  // per segment: the largest Faddeeva-core half-width, grid units
+    // per segment: the largest Faddeeva-core half-width, in grid units (mixed) or cm^-1 (FP64)
+    unsigned* d_reach = (unsigned*)workspace(ctx, "core_reach", sizeof(unsigned) * std::max(nseg, 1));
+    IRS_CUDA(cudaMemsetAsync(d_reach, 0, sizeof(unsigned) * std::max(nseg, 1), st));
+    if (!mixed)
+        lp_write_kernel<0><<<g1, kLpThreads, 0, st>>>(d_segs, d_lists, tp, cfg, d_keep, d_chunk, n_chunks,
+                                                      d_count, o64, om, d_pairs, d_reach);
     if (mixed) {
         char* base = (char*)workspace(ctx, "lpmx", S * (8 + 8 + 16 + 16 + 16));
         om.V = (double*)base;
@@ -242,22 +318,28 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
         om.p0 = (float4*)(base + S * 16);
         om.p1 = (float4*)(base + S * 32);
         om.p2 = (float4*)(base + S * 48);
-        d_reach = (unsigned*)workspace(ctx, "core_reach", sizeof(unsigned) * std::max(nseg, 1));
-        IRS_CUDA(cudaMemsetAsync(d_reach, 0, sizeof(unsigned) * std::max(nseg, 1), st));
         lp_write_kernel<1><<<g1, kLpThreads, 0, st>>>(d_segs, d_lists, tp, cfg, d_keep, d_chunk, n_chunks,
                                                       d_count, o64, om, d_pairs, d_reach);
     }
     check_launch(ctx);
     IRS_CUDA(cudaEventRecord(ctx->ev[ev_mid], st));
     const int npl = pl.n_prof * pl.L;
+    std::vector<int> first(npl + 1, 0);  // first segment of each profile-layer (emitted in order)
+    for (int q = 0; q < npl; ++q) first[q + 1] = first[q] + pl.pl_segs[q].y;
     if (!mixed) {
-        dim3 g2((unsigned)((n_nu + 255) / 256), npl);
-        if (o.method == 1)
-            linesum_f64_kernel<1><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride);
-        else if (o.method == 2)
-            linesum_f64_kernel<2><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride);
-        else
-            linesum_f64_kernel<3><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride);
+        const bool tree = o.method != IRS_PSEUDOVOIGT && dnu_g > 0.0;
+        if (tree) tree64_launch(ctx, pl, first, d_segs, d_count, d_reach, d_pl, o64, d_grid, n_nu, grid0, dnu_g, o,
+                                (double*)d_tau, d_pert, pstride, d_pairs + 2, d_uniform);
+        if (!tree || d_uniform) {  // PseudoVoigt, and a caller's grid that is not uniform
+            dim3 g2((unsigned)((n_nu + 255) / 256), npl);
+            const int* du = tree ? d_uniform : nullptr;
+            if (o.method == 1)
+                linesum_f64_kernel<1><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride, du);
+            else if (o.method == 2)
+                linesum_f64_kernel<2><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride, du);
+            else
+                linesum_f64_kernel<3><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride, du);
+        }
     } else {
         dim3 g2((unsigned)((n_nu + kMxStrip - 1) / kMxStrip), npl);
         const float cut_g = (float)(o.cutoff / dnu_g);
@@ -281,8 +363,6 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
             strip_table_kernel<<<(nM + 255) / 256, 256, 0, st>>>(d_M);
             check_launch(ctx);
         }
-        std::vector<int> first(npl + 1, 0);  // first segment of each profile-layer (emitted in order)
-        for (int q = 0; q < npl; ++q) first[q + 1] = first[q] + pl.pl_segs[q].y;
         for (int pa = 0; pa < npl;) {
             // this launch: profile-layers [pa, pb) and their segments [s_a, first[pb])
             int pb = npl;
@@ -506,7 +586,7 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
         workspace(ctx, "I", (size_t)n_prof * n_nu * sizeof(double));
         workspace(ctx, "grid", n_nu * sizeof(double));
         if (slots > 0) {
-            workspace(ctx, mixed ? "lpmx" : "lp64", (size_t)slots * (mixed ? 64 : 48));
+            workspace(ctx, mixed ? "lpmx" : "lp64", (size_t)slots * (mixed ? 64 : kLpF64 * sizeof(double)));
             workspace(ctx, "keep", (size_t)slots);
             workspace(ctx, "chunk_count", sizeof(int) * (size_t)nseg * ((max_list + kLpChunk - 1) / kLpChunk));
         }
@@ -517,7 +597,12 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
             workspace(ctx, "strip_far", std::min((size_t)nseg * n_strips, ctx->strip_buf_max / cb) * cb);
             workspace(ctx, "strip_M", sizeof(float) * kMxWarps * kFarNodes * kCtaNodes);
         }
-        if (mixed) workspace(ctx, "core_reach", sizeof(unsigned) * nseg);
+        if (!mixed && o.method != IRS_PSEUDOVOIGT) {
+            const size_t cb = t64_cell_bytes(o.line_mixing == IRS_LM_PER_LINE_Y);
+            const size_t cells = (size_t)nseg * t64_groups(n_nu, t64_leaf_points(n_nu, L));
+            workspace(ctx, "t64_far", std::min(cells, ctx->strip_buf_max / cb) * cb);
+        }
+        workspace(ctx, "core_reach", sizeof(unsigned) * nseg);
         workspace(ctx, "lrt", std::max<size_t>(lrt.size(), 1) * sizeof(LayerRT));
         workspace(ctx, "prt", std::max<size_t>(prt.size(), 1) * sizeof(ProfileRT));
     }
@@ -942,7 +1027,7 @@ static void forward_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, c
     int64_t total_lines = 0;
     for (auto& l : ctx->lists) total_lines += l.n;
     const bool mixed = o.precision != IRS_FP64;
-    const size_t per_prof = (size_t)L * total_lines * (mixed ? 65 : 49) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
+    const size_t per_prof = (size_t)L * total_lines * (mixed ? 65 : 1 + kLpF64 * sizeof(double)) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
                             (size_t)ig.g.n * 8;
     const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
@@ -1490,7 +1575,15 @@ int irs_cross_sections(irs_ctx* ctx, int species, const double* grid, int64_t n_
     IRS_CUDA(cudaEventRecord(ctx->ev[0], st));
     double* d_grid = (double*)workspace(ctx, "grid", n_nu * sizeof(double));
     IRS_CUDA(cudaMemcpyAsync(d_grid, grid, n_nu * sizeof(double), cudaMemcpyHostToDevice, st));
-    void* d_tau = run_linesum(ctx, pl, d_grid, n_nu, grid[0], dnu_g, o, 1);
+    // the FP64 line sum takes its grid as it is: uniform or not is found on the device
+    int* d_uni = nullptr;
+    if (precision == IRS_FP64) {
+        d_uni = (int*)workspace(ctx, "grid_uniform", sizeof(int));
+        IRS_CUDA(cudaMemsetAsync(d_uni, 1, sizeof(int), st));
+        grid_uniform_kernel<<<(unsigned)((n_nu + 255) / 256), 256, 0, st>>>(d_grid, n_nu, grid[0], dnu_g, d_uni);
+        check_launch(ctx);
+    }
+    void* d_tau = run_linesum(ctx, pl, d_grid, n_nu, grid[0], dnu_g, o, 1, nullptr, 0, d_uni);
     IRS_CUDA(cudaEventRecord(ctx->ev[2], st));
     if (precision != IRS_FP64) {
         std::vector<float> tmp(n_nu);

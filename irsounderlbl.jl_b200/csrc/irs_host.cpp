@@ -258,6 +258,37 @@ void jacobian_weights(const irs_profile& P, const irs_fm_options& o, int species
     }
 }
 
+// --------------------------------------- interpolation tables (FP64 line sum)
+// 32 Chebyshev nodes on [-1, 1] (as rounded to double, which is where the kernels evaluate)
+// and the Lagrange weights at the nodes of the block's four quarters and at the points of
+// 128- and 32-point blocks, products in extended precision.
+void t64_tables(double* out) {
+    constexpr int N = 32;
+    long double xk[N], wk[N];
+    for (int k = 0; k < N; ++k) {
+        out[k] = (double)std::cos((2 * k + 1) * 3.14159265358979323846264338327950288L / (2 * N));
+        xk[k] = out[k];
+    }
+    for (int k = 0; k < N; ++k) {
+        wk[k] = 1.0L;
+        for (int l = 0; l < N; ++l)
+            if (l != k) wk[k] *= xk[k] - xk[l];
+    }
+    auto weight = [&](int k, long double x) {
+        long double p = 1.0L;
+        for (int l = 0; l < N; ++l)
+            if (l != k) p *= x - xk[l];
+        return (double)(p / wk[k]);
+    };
+    double* o = out + N;
+    for (int q = 0; q < 4; ++q)
+        for (int k = 0; k < N; ++k)
+            for (int j = 0; j < N; ++j) *o++ = weight(k, (2 * q - 3 + xk[j]) / 4.0L);
+    for (int P : {128, 32})
+        for (int k = 0; k < N; ++k)
+            for (int i = 0; i < P; ++i) *o++ = weight(k, (2.0L * i - (P - 1)) / P);
+}
+
 // --------------------------------------------------- Faddeeva constants
 static void weideman_coefficients(int N, double* L_out, double* a_out) {
     const int M = 2 * N, M2 = 2 * M;

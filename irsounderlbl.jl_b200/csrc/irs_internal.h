@@ -29,6 +29,10 @@ struct Error {
         if (!(cond)) throw ::irs::Error{IRS_E_ARG, std::string(msg)}; \
     } while (0)
 
+// Tables of the FP64 line sum's interpolation (T64Tables, linesum_tree64.cuh) as one array
+constexpr int kT64TableDoubles = 32 + 4 * 32 * 32 + 32 * 128 + 32 * 32;
+void t64_tables(double* out);
+
 // ------------------------------------------------------------------ grids
 // Julia's float range a:s:b (src/Utils/wavenumber_grid.jl:23-26): start, step and
 // stop are rationalised (n/den) when they have exact small-denominator forms and the
@@ -109,8 +113,8 @@ struct DevBuf {
 };
 
 // Per-line parameter arrays for the line sum (one slot per (segment, line)).
-struct LineParamsF64 {  // plain FP64 kernel; PseudoVoigt reuses f=gV, y=eta, Sn=S, Hc=base
-    double *nu0, *f, *y, *Sn, *Hc, *YSn;
+struct LineParamsF64 {  // FP64 kernels; PseudoVoigt reuses f=gV, y=eta, Sn=S, Hc=base
+    double *nu0, *f, *y, *Sn, *Hc, *YSn, *b, *k0, *g;
 };
 struct LineParamsMixed {  // FP32 kernel, grid units relative to the grid start
     double* V;            // unshifted centre (sorted key)

@@ -190,7 +190,9 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_keep_kernel(
 
 struct LpOutF64 {
     double *nu0, *f, *y, *Sn, *Hc, *YSn;
+    double *b, *k0, *g;  // gamma_L = y/f, Sn/(sqrt(pi) f), YSn/(sqrt(pi) f): far wings in cm^-1
 };
+constexpr int kLpF64 = 9;  // doubles per line
 struct LpOutMixed {
     double* V;   // unshifted centre, grid units (the sorted key of the window searches)
     float2* U;   // shifted centre, grid units, as hi + lo: hi = (float)U, lo = (float)(U - hi)
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
     __syncthreads();
     long long run = s_off;
     unsigned long long pairs = 0, core = 0;
-    float reach = 0.f;  // x_far / fx in grid units: the Faddeeva core's half-width
+    float reach = 0.f;  // the Faddeeva core's half-width: x_far / fx in grid units, x_far / f in FP64
     const double isp = kInvSqrtPi;
     const SegPhys g = seg_phys(L.mol, sg.T, sg.p_atm, sg.vs);
     const double inv_dg = 1.0 / cfg.dnu_g, inv_gran = 1.0 / cfg.u_gran;  // u_gran: a power of two
@@ -323,6 +325,9 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
                 if (PREC == 0) {
                     o64.nu0[slot] = ph.nu0s; o64.f[slot] = f; o64.y[slot] = y;
                     o64.Sn[slot] = Sn; o64.Hc[slot] = Hc; o64.YSn[slot] = YSn;
+                    const double rf = gd * (1.0 / kSqrtLn2);  // 1 / f
+                    o64.b[slot] = ph.gl; o64.k0[slot] = ph.S * (isp * isp); o64.g[slot] = YSn * isp * rf;
+                    reach = fmaxf(reach, (float)fmin(cfg.x_far * rf, 1.0e30) * 1.000001f);  // cm^-1
                 } else {
                     const double dg = cfg.dnu_g, co = sg.coef;
                     const double fx = f * dg;         // x per grid unit

@@ -4,10 +4,12 @@
 // (src/Sensor/sounder.jl:283-307); with VP_Y line mixing the CO2 term is
 // max(sigma_V + sum_j YSn_j Im w, 0) (line_mixing.jl:1166-1186, :1351-1369).
 //
-// Two kernels:
+// Two kernels here, and linesum_tree64.cuh:
 //  * linesum_f64_kernel -- the plain FP64 GPU kernel: one thread per grid point,
 //    a binary search per point and species for the window on the shifted centres,
-//    FP64 arithmetic and IEEE division, exactly the reference kernel's structure.
+//    FP64 arithmetic and IEEE division, exactly the reference kernel's structure.  It
+//    serves PseudoVoigt and grids that are not uniform; the FP64 sum of the other methods
+//    on a uniform grid is tree64_leaf_kernel's.
 //  * linesum_mixed_kernel -- FP32 + Kahan: a CTA owns a 2048-point strip of one
 //    (profile, layer); each warp owns 256 contiguous points (8 per lane,
 //    interleaved so stores are 128-byte coalesced); line tiles of 256 lines are
@@ -45,7 +47,8 @@ template <int METHOD>
 __global__ void __launch_bounds__(256) linesum_f64_kernel(
     const SegDev* __restrict__ segs, const int* __restrict__ seg_count, const int2* __restrict__ pl_segs,
     LpOutF64 lp, const double* __restrict__ grid, long long n_nu, double cutoff, double x_far,
-    double* __restrict__ tau, double* __restrict__ pert, long long pstride) {
+    double* __restrict__ tau, double* __restrict__ pert, long long pstride, const int* __restrict__ uniform) {
+    if (uniform && *uniform) return;  // taken by tree64_leaf_kernel
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int pl = blockIdx.y;
     if (i >= n_nu) return;
