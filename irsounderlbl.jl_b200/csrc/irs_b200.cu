@@ -425,6 +425,36 @@ static void ensure_ils(irs_ctx* ctx, double dnu, double opd, double fwhm, int ap
     ctx->ils_n = n;
 }
 
+// ChanNodes of the channel grid on the internal grid: both are (a + i s)/den with integers
+// in double, so equal rationals are equal doubles and the resampling weight is exactly 0.
+static ChanNodes chan_nodes(const GridSpec& g, const GridSpec& ch) {
+    ChanNodes c{0, 0};
+    if (!g.den || !ch.den || g.n >= ((int64_t)1 << 30)) return c;
+    const __int128 gs = (__int128)(int64_t)g.s_n * ch.den, cs = (__int128)(int64_t)ch.s_n * g.den;
+    const __int128 off = (__int128)(int64_t)ch.a_n * g.den - (__int128)(int64_t)g.a_n * ch.den;
+    if (gs <= 0 || cs % gs != 0 || off < 0 || off % gs != 0) return c;
+    const __int128 step = cs / gs, first = off / gs;
+    if (step < 16 || step > kChanThreads || first + (ch.n - 1) * step > g.n - 1) return c;
+    c.first = (int)first;
+    c.step = (int)step;
+    return c;
+}
+
+// The ILS at the channels, R and BT [np][n_ch]
+static void launch_ils(irs_ctx* ctx, const double* d_I, int64_t n_nu, int np, const InternalGrid& ig, const GridSpec& ch,
+                       int with_ils, double* d_R, double* d_BT) {
+    const double* d_kern = with_ils ? (const double*)ctx->work["ils"].p : nullptr;
+    const int64_t n_taps = with_ils ? ctx->ils_n : 0;
+    const ChanNodes cn = with_ils ? chan_nodes(ig.g, ch) : ChanNodes{0, 0};
+    if (cn.step)
+        ils_nodes_kernel<<<dim3((unsigned)((ch.n + kIlsChan - 1) / kIlsChan), np), kChanThreads, 0, ctx->stream>>>(
+            d_I, (int)n_nu, d_kern, (int)n_taps, ig.dnu_hi, to_dev(ch), cn, d_R, d_BT);
+    else
+        ils_bt_kernel<<<dim3((unsigned)((ch.n * 32 + 255) / 256), np), 256, 0, ctx->stream>>>(
+            d_I, n_nu, d_kern, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), with_ils, d_R, d_BT);
+    check_launch(ctx);
+}
+
 // Runs f(0..n-1) on the host's cores.
 template <class F>
 static void parallel_for(int n, F&& f) {
@@ -676,11 +706,7 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
             rte_kernel<double><<<g3, 256, 0, st>>>((const double*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);
     check_launch(ctx);
     IRS_CUDA(cudaEventRecord(ctx->ev[3], st));
-    const double* d_kern = o.with_ils ? (const double*)ctx->work["ils"].p : nullptr;
-    dim3 g4((unsigned)((ch.n * 32 + 255) / 256), n_prof);
-    ils_bt_kernel<<<g4, 256, 0, st>>>(d_I, n_nu, d_kern, o.with_ils ? ctx->ils_n : 0, ig.dnu_hi, to_dev(ig.g),
-                                       to_dev(ch), o.with_ils, d_R, d_BT);
-    check_launch(ctx);
+    launch_ils(ctx, d_I, n_nu, n_prof, ig, ch, o.with_ils, d_R, d_BT);
     IRS_CUDA(cudaEventRecord(ctx->ev[4], st));
 }
 
@@ -913,9 +939,7 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
         check_launch(ctx);
         const double* d_kern = o.with_ils ? (const double*)ctx->work["ils"].p : nullptr;
         const int64_t n_taps = o.with_ils ? ctx->ils_n : 0;
-        ils_bt_kernel<<<dim3((unsigned)((n_ch * 32 + 255) / 256), np), 256, 0, st>>>(
-            d_I, n_nu, d_kern, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), o.with_ils, d_RB, d_RB + (size_t)np * n_ch);
-        check_launch(ctx);
+        launch_ils(ctx, d_I, n_nu, np, ig, ch, o.with_ils, d_RB, d_RB + (size_t)np * n_ch);
         if (adjoint) {  // the pullback: radiance cotangent on the grid, then the adjoint sweep
             double* d_dy = (double*)workspace(ctx, "vjp_dy", (size_t)np * n_ch * sizeof(double));
             IRS_CUDA(cudaMemcpyAsync(d_dy, dy_h + (size_t)p0 * n_ch, (size_t)np * n_ch * sizeof(double),
@@ -946,10 +970,15 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             IRS_CUDA(cudaStreamSynchronize(st));
             continue;
         }
-        jg_channel_kernel<<<dim3((unsigned)((n_ch * 32 + 255) / 256), (unsigned)n_state, np), 256, 0, st>>>(
-            d_D, n_nu, (int)n_state, o.with_ils ? (const float*)ctx->work["ils_f"].p : nullptr, n_taps, ig.dnu_hi,
-            to_dev(ig.g), to_dev(ch), o.with_ils, d_RB,
-            sp.observable, d_K);
+        const float* d_kernf = o.with_ils ? (const float*)ctx->work["ils_f"].p : nullptr;
+        const ChanNodes cn = o.with_ils ? chan_nodes(ig.g, ch) : ChanNodes{0, 0};
+        if (cn.step)
+            jg_channel_nodes_kernel<<<dim3((unsigned)((n_ch + kJgChan - 1) / kJgChan), (unsigned)n_state, np), kChanThreads, 0, st>>>(
+                d_D, (int)n_nu, (int)n_state, d_kernf, (int)n_taps, ig.dnu_hi, to_dev(ch), cn, d_RB, sp.observable, d_K);
+        else
+            jg_channel_kernel<<<dim3((unsigned)((n_ch * 32 + 255) / 256), (unsigned)n_state, np), 256, 0, st>>>(
+                d_D, n_nu, (int)n_state, d_kernf, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), o.with_ils, d_RB,
+                sp.observable, d_K);
         check_launch(ctx);
         if (!K_dev) {
             Kf.resize((size_t)np * n_state * n_ch);

@@ -1151,6 +1151,12 @@ __global__ void __launch_bounds__(128) jg_rte_kernel(
 }
 
 // ------------------------------------------------------------------ channel tail
+__device__ __forceinline__ double dbt_dr(double nu, double R) {  // vmr_jacobian.jl:120-125
+    if (R <= 0.0) return 0.0;
+    const double A = 1.191042953e-5 * (nu * nu * nu), Lg = log1p(A / R);
+    return 1.4387769 * nu * A / ((Lg * Lg) * R * (R + A));
+}
+
 // K[x][c] = dBT/dR_c * resample(ILS(D[x]))_c, vmr_jacobian.jl:359-380.  One warp per
 // (state element, channel); the ILS taps (kernf: the normalised FP64 taps rounded to
 // FP32) run over lanes (FP32 products, FP32 sums).  A window that lies inside the grid,
@@ -1199,15 +1205,25 @@ __global__ void __launch_bounds__(256) jg_channel_kernel(const float* __restrict
     }
     if (lane == 0) {
         double scale = 1.0;
-        if (observable == 0) {  // vmr_jacobian.jl:120-125
-            const double Rc = R[(size_t)p * ch.n + wid];
-            if (Rc <= 0.0) scale = 0.0;
-            else {
-                const double A = 1.191042953e-5 * (nu * nu * nu), Lg = log1p(A / Rc);
-                scale = 1.4387769 * nu * A / ((Lg * Lg) * Rc * (Rc + A));
-            }
-        }
+        if (observable == 0) scale = dbt_dr(nu, R[(size_t)p * ch.n + wid]);
         K[((size_t)p * n_state + x) * ch.n + wid] = (float)(v * scale);
+    }
+}
+
+// The same for channels on grid nodes: 16 channels of one state element per CTA, FP32
+// products and sums as above (chan_sums: two loads per 16 products).
+constexpr int kJgChan = 16;
+__global__ void __launch_bounds__(kChanThreads) jg_channel_nodes_kernel(
+    const float* __restrict__ D, int n_nu, int n_state, const float* __restrict__ kernf, int n_taps, double dnu_hi,
+    GridDev ch, ChanNodes nodes, const double* __restrict__ R, int observable, float* __restrict__ K) {
+    const int c0 = blockIdx.x * kJgChan, x = blockIdx.y, p = blockIdx.z;
+    const float v = chan_sums<float, kJgChan>(D + ((size_t)p * n_state + x) * n_nu, n_nu, kernf, n_taps,
+                                              nodes.first + c0 * nodes.step - (n_taps - 1) / 2, nodes.step);
+    const int c = c0 + (int)threadIdx.x;
+    if (threadIdx.x < kJgChan && c < ch.n) {
+        double scale = 1.0;
+        if (observable == 0) scale = dbt_dr(ch.at(c), R[(size_t)p * ch.n + c]);
+        K[((size_t)p * n_state + x) * ch.n + c] = (float)((double)v * dnu_hi * scale);
     }
 }
 
@@ -1228,15 +1244,7 @@ __global__ void __launch_bounds__(256) vjp_channel_kernel(const double* __restri
     if (c >= ch.n) return;
     const double nu = ch.at(c);
     const size_t pc = (size_t)p * ch.n + c;
-    double scale = 1.0;
-    if (observable == 0) {
-        const double Rc = R[pc];
-        if (Rc <= 0.0) scale = 0.0;
-        else {
-            const double A = 1.191042953e-5 * (nu * nu * nu), Lg = log1p(A / Rc);
-            scale = 1.4387769 * nu * A / ((Lg * Lg) * Rc * (Rc + A));
-        }
-    }
+    const double scale = observable == 0 ? dbt_dr(nu, R[pc]) : 1.0;
     const double rb = dy[pc] * scale;
     ChanAdj a{0, 0.0, 0.0};
     const double g0 = g.at(0), gl = g.at(n_nu - 1);

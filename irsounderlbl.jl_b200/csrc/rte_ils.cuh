@@ -13,7 +13,8 @@
 //  only in the cumulative optical depth and the transmittances, FP32 (Kahan-summed
 //  radiance) elsewhere.
 //
-//  ils_bt_kernel (one warp per channel and profile) restates apply_ils
+//  ils_bt_kernel (one warp per channel and profile; ils_nodes_kernel where the channels
+//  are grid nodes at a constant step) restates apply_ils
 //  (src/Sensor/ils.jl:131-153) evaluated at the grid nodes that the linear channel
 //  resampling reads (sounder.jl:372-377), then brightness_temperature
 //  (planck.jl:53-57).  Channel nodes are grid nodes for every sounder, so this is the
@@ -490,6 +491,97 @@ __global__ void ils_normalise_kernel(double* kern, long long n, double dnu) {
     for (long long k = threadIdx.x; k < n; k += blockDim.x) kern[k] /= tot;
 }
 
+// Channels on grid nodes at a constant step: channel c reads the convolution at node
+// first + c step, and the linear resampling (sounder.jl:372-377) has weight 0.  Found on
+// the host from the grids' exact rational forms; step 0 where it does not hold (or the
+// step is outside 16..256, where apod_at serves).
+struct ChanNodes {
+    int first, step;
+};
+constexpr int kChanThreads = 256;
+
+// The convolution at C consecutive channels, one CTA: sum[c] = sum_k X[base + c step + k]
+// kern[k], X zero outside [0, n_nu).  A thread takes one phase r of the step (of the
+// kChanThreads / T splits of the rows m) and walks the points r + m step; the taps that a
+// point meets in the C channels are C rows of the same phase, so a ring of C registers holds
+// them and each point costs two coalesced loads for C products.  One warp per channel and
+// two loads per product, as apod_at does it, left 221 channels of one scene waiting on 400
+// dependent loads (94 us, now 13) and the Jacobian's states on L2: a 151-element IASI
+// Jacobian's contraction took 4.76 ms, now 2.10 (16 scenes x 101 x 221: 1.51, now 0.61).
+// Returns the sum of channel threadIdx.x to the first C threads.
+template <typename T, int C>
+__device__ __forceinline__ T chan_sums(const T* __restrict__ X, int n_nu, const T* __restrict__ kern, int n_taps,
+                                       int base, int step) {
+    __shared__ T part[kChanThreads / 32][C];
+    const int lanes = (step + 31) & ~31;            // threads per split
+    const int splits = kChanThreads / lanes;
+    const int r = threadIdx.x % lanes, sp = threadIdx.x / lanes;
+    const int M = (n_taps + step - 1) / step + C - 1;  // rows m in which some tap is met
+    const int per = ((M + splits - 1) / splits + C - 1) / C * C;
+    T acc[C], ring[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = ring[c] = T(0);
+    if (r < step && sp < splits) {
+        const int m0 = sp * per, m1 = min(M, m0 + per);
+#pragma unroll
+        for (int u = 1; u < C; ++u) {  // the rows before this split's
+            const int m = m0 - C + u, k = r + m * step;
+            if (m >= 0 && k < n_taps) ring[u] = kern[k];
+        }
+        for (int mb = m0; mb < m1; mb += C) {
+            T x[C];
+#pragma unroll
+            for (int u = 0; u < C; ++u) {
+                const int j = base + r + (mb + u) * step;
+                x[u] = (mb + u < m1 && (unsigned)j < (unsigned)n_nu) ? X[j] : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < C; ++u) {
+                const int k = r + (mb + u) * step;
+                ring[u] = k < n_taps ? kern[k] : T(0);
+#pragma unroll
+                for (int c = 0; c < C; ++c) acc[c] = fma(x[u], ring[(u - c + C) % C], acc[c]);
+            }
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        T v = acc[c];
+#pragma unroll
+        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        if (lane == 0) part[warp][c] = v;
+    }
+    __syncthreads();
+    T tot = T(0);
+    if (threadIdx.x < C) {
+#pragma unroll
+        for (int w = 0; w < kChanThreads / 32; ++w) tot += part[w][threadIdx.x];
+    }
+    return tot;
+}
+
+__device__ __forceinline__ double brightness_t(double nu, double R) {  // planck.jl:53-57
+    return R <= 0.0 ? 0.0 : 1.4387769 * nu / log1p(1.191042953e-5 * (nu * nu * nu) / R);
+}
+
+// R and BT of 8 channels per CTA (channels on grid nodes, with the ILS)
+constexpr int kIlsChan = 8;
+__global__ void __launch_bounds__(kChanThreads) ils_nodes_kernel(const double* __restrict__ I, int n_nu,
+                                                                 const double* __restrict__ kern, int n_taps,
+                                                                 double dnu_hi, GridDev ch, ChanNodes nodes,
+                                                                 double* __restrict__ R, double* __restrict__ BT) {
+    const int c0 = blockIdx.x * kIlsChan, p = blockIdx.y;
+    const double v = chan_sums<double, kIlsChan>(I + (size_t)p * n_nu, n_nu, kern, n_taps,
+                                                 nodes.first + c0 * nodes.step - (n_taps - 1) / 2, nodes.step);
+    const int c = c0 + (int)threadIdx.x;
+    if (threadIdx.x < kIlsChan && c < ch.n) {
+        const double Rv = v * dnu_hi;
+        R[(size_t)p * ch.n + c] = Rv;
+        BT[(size_t)p * ch.n + c] = brightness_t(ch.at(c), Rv);
+    }
+}
+
 __device__ double apod_at(const double* __restrict__ Ip, long long n_nu, const double* __restrict__ kern,
                           long long n_taps, long long i, int lane) {
     const long long half = (n_taps - 1) / 2;
@@ -532,8 +624,7 @@ __global__ void __launch_bounds__(256) ils_bt_kernel(const double* __restrict__ 
     }
     if (lane == 0) {
         R[(size_t)p * ch.n + wid] = Rv;
-        BT[(size_t)p * ch.n + wid] =
-            Rv <= 0.0 ? 0.0 : 1.4387769 * nu / log1p(1.191042953e-5 * (nu * nu * nu) / Rv);
+        BT[(size_t)p * ch.n + wid] = brightness_t(nu, Rv);
     }
 }
 
