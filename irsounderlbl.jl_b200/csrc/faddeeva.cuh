@@ -211,6 +211,26 @@ __device__ __forceinline__ float2 faddeeva_cf2(float x, float y, float y2) {
     return wz_ratio32(ur - 1.f, ui, fmaf(x, cr, -y * ui), fmaf(x, ui, y * cr));
 }
 
+// The same with its derivative, as (H_x, H_y) = (Re w', -Im w'):
+//   w' = -(i/sqrt(pi)) (u^2 - 3/2 u + 3/2) / (u (u - 3/2)^2),
+// the derivative of the rational function, sharing its reciprocal.  w' = -2 z w + 2 i/sqrt(pi)
+// would lose 2 |z|^2 in relative accuracy here (1e-3 of H_y at |x| = 122 in FP32).
+__device__ __forceinline__ float2 faddeeva_cf2_grad(float x, float y, float y2, float2& grad) {
+    constexpr float k = (float)kInvSqrtPi;
+    const float ur = fmaf(x, x, -y2), ui = 2.f * x * y;  // u = z^2
+    const float cr = ur - 1.5f;                           // u - 3/2 = (cr, ui)
+    const float dr = fmaf(x, cr, -y * ui), di = fmaf(x, ui, y * cr);  // D = z (u - 3/2)
+    const float r = rcp_approx32(fmaf(dr, dr, di * di));
+    const float qr = dr * r, qi = -di * r;                // 1 / D
+    const float nr = ur - 1.f;
+    const float2 w = make_float2(-k * fmaf(nr, qi, ui * qr), k * fmaf(nr, qr, -ui * qi));
+    const float mr = fmaf(ur, cr, fmaf(-ui, ui, 1.5f)), mi = ui * (cr + ur);  // u (u - 3/2) + 3/2
+    const float sr = fmaf(qr, qr, -qi * qi), si = 2.f * qr * qi;
+    // w' = -(i k) m s: Re = k Im(m s), -Im = k Re(m s)
+    grad = make_float2(k * fmaf(mr, si, mi * sr), k * fmaf(mr, sr, -mi * si));
+    return w;
+}
+
 __device__ __forceinline__ float2 faddeeva32_inline(float x, float y) {
     const float s = fabsf(x) + y;
     if (s >= 15.0f) return faddeeva_cf2(x, y, y * y);
@@ -243,11 +263,16 @@ __device__ __forceinline__ float2 faddeeva32_inline(float x, float y) {
 static __device__ __noinline__ float2 faddeeva32(float x, float y) { return faddeeva32_inline(x, y); }
 
 
-// faddeeva32 with its |x| + y >= 15 branch (the two-level continued fraction) inlined
-// in real arithmetic; the CF4 and Weideman regions go through the shared routine
-__device__ __forceinline__ float2 faddeeva32_fast(float x, float y) {
-    if (fabsf(x) + y >= 15.0f) return faddeeva_cf2(x, y, y * y);
-    return faddeeva32(x, y);
+// w and (H_x, H_y): the two-level continued fraction and its derivative for |x| + y >= 15,
+// else faddeeva32 with w' = -2 z w + 2 i/sqrt(pi)
+__device__ __forceinline__ float2 wofz_grad32(float x, float y, float2 w) {
+    return make_float2(-2.f * x * w.x + 2.f * y * w.y, 2.f * (x * w.y + y * w.x) - 2.f * (float)kInvSqrtPi);
+}
+__device__ __forceinline__ float2 faddeeva32_grad(float x, float y, float2& grad) {
+    if (fabsf(x) + y >= 15.0f) return faddeeva_cf2_grad(x, y, y * y, grad);
+    const float2 w = faddeeva32(x, y);
+    grad = wofz_grad32(x, y, w);
+    return w;
 }
 
 // voigt.jl:105-117 (Float32 Weideman-24, IEEE division as Julia's Float32 `/`)

@@ -174,6 +174,49 @@ static std::vector<ListDev> list_descs(irs_ctx* ctx) {
     return v;
 }
 
+// granularity of the FP32 high part of the shifted centres: those within the grid plus its
+// cutoff margins have |U| < 2^24 u_gran
+static double u_granularity(int64_t n_nu, double cut_g) {
+    const double reach = (double)n_nu + 2.0 * cut_g + 64.0;
+    double g = 1.0 / 16.0;
+    while (reach >= 16777216.0 * g) g *= 2.0;
+    return g;
+}
+
+// Cell index (linesum_tree32.cuh) of rows of sorted keys V[off[r] .. + n[r]) over the grid
+// and `reach` (cutoff and margin) beyond each end: cells of 32 points, wider where the grid
+// and its margins would take more than a million.
+static CellIndex cell_index(irs_ctx* ctx, const double* d_V, const std::vector<long long>& off, const std::vector<int>& n,
+                            int64_t n_nu, double reach) {
+    const double span = (double)((n_nu + kTrStrip - 1) / kTrStrip * kTrStrip) + 2.0 * reach;
+    double cell = 32.0;
+    while (span / cell > 1048576.0) cell *= 2.0;
+    CellIndex ci;
+    const double o = std::ceil(reach / cell + 1.0) * cell;
+    ci.n = (int)((span + 2.0 * (o - reach)) / cell) + 3;
+    ci.inv_cell = (float)(1.0 / cell);
+    ci.off = (float)o;
+    int* d_idx = (int*)workspace(ctx, "cell_idx", off.size() * (size_t)ci.n * sizeof(int));
+    const long long* d_off = upload(ctx, "cell_off", off);
+    const int* d_n = upload(ctx, "cell_n", n);
+    cell_index_kernel<<<dim3((unsigned)((ci.n + 255) / 256), (unsigned)off.size()), 256, 0, ctx->stream>>>(d_V, d_off, d_n,
+                                                                                                  ci.n, cell, o, d_idx);
+    check_launch(ctx);
+    ci.idx = d_idx;
+    return ci;
+}
+static const TreeTables* tree_tables(irs_ctx* ctx) {
+    const bool have = ctx->work.count("tree32") != 0;
+    TreeTables* d = (TreeTables*)workspace(ctx, "tree32", sizeof(TreeTables));
+    if (!have) {
+        std::unique_ptr<TreeTables> h(new TreeTables);
+        tree32_tables(&h->M[0][0][0], &h->L[0][0]);
+        IRS_CUDA(cudaMemcpyAsync(d, h.get(), sizeof(TreeTables), cudaMemcpyHostToDevice, ctx->stream));
+        IRS_CUDA(cudaStreamSynchronize(ctx->stream));
+    }
+    return d;
+}
+
 // tree64: points per leaf (one warp).  128 points cost the least per point, but a short
 // grid then has too few leaves to fill the chip; the rule counts the leaves of one
 // profile's layers (not of the batch, so that a profile's result does not depend on it).
@@ -287,11 +330,7 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
     LpConfig cfg;
     cfg.cutoff = o.cutoff; cfg.x_far = o.x_far; cfg.dptmn = o.dptmn;
     cfg.grid0 = grid0; cfg.dnu_g = dnu_g; cfg.method = o.method; cfg.n_nu = n_nu;
-    {  // shifted centres within the grid plus its cutoff margins: |U| < 2^24 u_gran
-        const double reach = (double)n_nu + 2.0 * o.cutoff / dnu_g + 64.0;
-        cfg.u_gran = 1.0 / 16.0;
-        while (reach >= 16777216.0 * cfg.u_gran) cfg.u_gran *= 2.0;
-    }
+    cfg.u_gran = u_granularity(n_nu, o.cutoff / dnu_g);
     const TipsDev tp = tips_dev(ctx);
     dim3 g1(n_chunks, nseg);
     lp_keep_kernel<<<g1, kLpThreads, 0, st>>>(d_segs, d_lists, tp, cfg, d_keep, d_chunk, n_chunks);
@@ -497,7 +536,7 @@ struct RelmatPlan {
 };
 static_assert(sizeof(LmPole) == sizeof(LmPoleDev), "pole layouts differ");
 constexpr long long kPertAlign = 8192;  // rows padded to whole line-sum strips of either kernel
-static_assert(kPertAlign % kMxStrip == 0 && kPertAlign % kJgStrip == 0, "perturbation row padding");
+static_assert(kPertAlign % kMxStrip == 0 && kPertAlign % kTrLeaf == 0, "perturbation row padding");
 
 // Flags the LM species' segments SEG_RELMAT; false when relmat line mixing is off.
 static bool relmat_prepare(irs_ctx* ctx, Plan& pl, const irs_fm_options& o, RelmatPlan& rp) {
@@ -768,16 +807,9 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
     for (auto& l : ctx->lists) max_list = std::max<int64_t>(max_list, l.n);
     int64_t total_lines = 0;
     for (auto& l : ctx->lists) total_lines += l.n;
-    const size_t per_prof = (size_t)L * total_lines * 96 + (size_t)n_out * L * n_nu * 4 + (size_t)n_state * n_nu * 4 +
+    const size_t per_prof = (size_t)L * total_lines * kJgLineBytes + (size_t)n_out * L * n_nu * 4 + (size_t)n_state * n_nu * 4 +
                             (size_t)n_nu * 8 + (size_t)n_state * n_ch * 4;
-    int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
-    if (o.method == 3) {  // the strip far field's node values of a pass fit its buffer
-        int n_lists = 0;
-        for (auto& l : ctx->lists) n_lists += l.n > 0 ? 1 : 0;
-        const size_t strip_prof = (size_t)L * std::max(n_lists, 1) * (size_t)((n_nu + kJgStrip - 1) / kJgStrip) *
-                                  (kJgStripWords * sizeof(float) + sizeof(int4));
-        chunk = std::max(1, std::min<int>(chunk, (int)std::min<size_t>(ctx->strip_buf_max / strip_prof, n_prof)));
-    }
+    const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
     std::vector<float> Kf;
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
         const int np = std::min(chunk, n_prof - p0);
@@ -824,7 +856,9 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
         pl.pl_segs.assign((size_t)np * L, make_int2(0, 0));
         std::vector<SegDev> sd(std::max<size_t>(pl.segs.size(), 1));
         std::vector<SegW> sw(std::max<size_t>(pl.segs.size(), 1));
-        std::vector<int> sn(std::max<size_t>(pl.segs.size(), 1), 0);
+        unsigned modes = 0;  // kinds of segments present
+        std::vector<long long> row_off(ctx->lists.size(), 0);  // a segment of each list (its keys: the list's)
+        std::vector<int> row_n(ctx->lists.size(), 0);
         int64_t off = 0;
         for (size_t i = 0; i < pl.segs.size(); ++i) {
             Segment& g = pl.segs[i];
@@ -832,21 +866,34 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             if (pl.pl_segs[key].y == 0) pl.pl_segs[key].x = (int)i;
             pl.pl_segs[key].y++;
             g.out_off = off;
-            sn[i] = (int)ctx->lists[g.list].n;
-            off += sn[i];
+            row_off[g.list] = off;
+            row_n[g.list] = (int)ctx->lists[g.list].n;
+            off += ctx->lists[g.list].n;
             SegDev& d = sd[i];
             d.T = g.T; d.p_atm = g.p_atm; d.vs = g.vmr_self; d.coef = g.coef; d.margin_g = g.margin_g;
             d.off = g.out_off; d.list = g.list; d.flags = g.flags;
-            std::memset(&sw[i], 0, sizeof(SegW));
-            jacobian_weights(profs[p0 + g.prof], o, ctx->lists[g.list].species, g.layer, sp, sw[i].w);
+            float w[kJgMaxOut][4] = {};
+            const int species = ctx->lists[g.list].species;
+            jacobian_weights(profs[p0 + g.prof], o, species, g.layer, sp, w);
+            sw[i] = SegW{};
+            for (int k = 0; k < sp.n_retrieved; ++k)
+                if (sp.retrieved[k] == species) {
+                    sw[i].retr |= 1u << k;
+                    std::memcpy(sw[i].pair, w[3 + 2 * k], sizeof sw[i].pair);
+                }
+            std::memcpy(sw[i].base, w, sizeof sw[i].base);
+            for (int c = 0; c < n_out; ++c) {
+                if (w[c][2] != 0.f) d.flags |= SEG_NEED_P;
+                if (w[c][3] != 0.f) d.flags |= SEG_NEED_V;
+            }
+            modes |= 1u << jg_mode(d.flags);
         }
         const int nseg = (int)pl.segs.size();
         const size_t S = (size_t)std::max<int64_t>(off, 1);
-        char* base = (char*)workspace(ctx, "jg_params", S * 96);
+        char* base = (char*)workspace(ctx, "jg_params", S * kJgLineBytes);
         JgOut go;
-        go.V = (double*)base; go.U = (double*)(base + S * 8);
-        go.q0 = (float4*)(base + S * 16); go.q1 = (float4*)(base + S * 32); go.q2 = (float4*)(base + S * 48);
-        go.q3 = (float4*)(base + S * 64); go.q4 = (float4*)(base + S * 80);
+        go.q0 = (float4*)base; go.q1 = go.q0 + S; go.q2 = go.q0 + 2 * S; go.q3 = go.q0 + 3 * S; go.q4 = go.q0 + 4 * S;
+        go.V = (double*)(base + S * 80); go.U = (float2*)(base + S * 88); go.df = (float*)(base + S * 96);
         float* d_out = (float*)workspace(ctx, "jg_out", (size_t)np * L * n_out * n_nu * sizeof(float));
         float* d_D = adjoint ? nullptr : (float*)workspace(ctx, "jg_D", (size_t)np * n_state * n_nu * sizeof(float));
         double* d_I = (double*)workspace(ctx, "I", (size_t)np * n_nu * sizeof(double));
@@ -856,7 +903,6 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
                              : (float*)workspace(ctx, "jg_K", (size_t)np * n_state * n_ch * sizeof(float));
         SegDev* d_segs = upload(ctx, "segs", sd);
         SegW* d_sw = upload(ctx, "jg_w", sw);
-        int* d_sn = upload(ctx, "jg_n", sn);
         std::vector<ListDev> ld = list_descs(ctx);
         ListDev* d_lists = upload(ctx, "list_descs", ld);
         int2* d_pl = upload(ctx, "pl_segs", pl.pl_segs);
@@ -865,55 +911,73 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
         JgLayer* d_jl = upload(ctx, "jg_layer", jl);
         JgProfile* d_jp = upload(ctx, "jg_prof", jp);
         double* d_vlev = upload(ctx, "jg_vlev", vlev);
-        IRS_CUDA(cudaMemsetAsync(d_out, 0, (size_t)np * L * n_out * n_nu * sizeof(float), st));
+        if (nseg == 0) IRS_CUDA(cudaMemsetAsync(d_out, 0, (size_t)np * L * n_out * n_nu * sizeof(float), st));
         long long pstride = 0;
         const double* d_pert = relmat ? relmat_launch(ctx, rp, d_grid, n_nu, o.lm_cutoff, o.x_far, pstride) : nullptr;
         if (nseg > 0) {
             LpConfig cfg;
-            cfg.cutoff = o.cutoff; cfg.x_far = o.x_far; cfg.dptmn = 0.0; cfg.grid0 = ig.g.at(0); cfg.u_gran = 1.0 / 16.0;
+            cfg.cutoff = o.cutoff; cfg.x_far = o.x_far; cfg.dptmn = 0.0; cfg.grid0 = ig.g.at(0); cfg.u_gran = u_granularity(n_nu, o.cutoff / ig.dnu_hi);
             cfg.dnu_g = ig.dnu_hi; cfg.method = o.method; cfg.n_nu = n_nu;
             unsigned* d_reach = (unsigned*)workspace(ctx, "jg_reach", sizeof(unsigned) * nseg);
             IRS_CUDA(cudaMemsetAsync(d_reach, 0, sizeof(unsigned) * nseg, st));
             jg_params_kernel<<<dim3((unsigned)((max_list + 255) / 256), nseg), 256, 0, st>>>(d_segs, d_lists, tips_dev(ctx), cfg, go, d_reach);
             check_launch(ctx);
-            const dim3 g2((unsigned)((n_nu + kJgStrip - 1) / kJgStrip), np * L);
             const float cut_g = (float)(o.cutoff / ig.dnu_hi);
-            const bool lm = o.line_mixing == 1;
-            // strip far field (pre-pass): 1808 bytes per (segment, strip); the profile passes
-            // are sized so a pass fits ctx->strip_buf_max (a single profile beyond it runs without)
-            float* d_sfar = nullptr;
-            int4* d_srng = nullptr;
-            const int n_strips = (int)g2.x;
-            const size_t cells = (size_t)nseg * n_strips;
-            if (o.method == 3 && cells * (kJgStripWords * sizeof(float) + sizeof(int4)) <= ctx->strip_buf_max) {
-                char* b = (char*)workspace(ctx, "jg_strip", cells * (kJgStripWords * sizeof(float) + sizeof(int4)));
-                d_sfar = (float*)b;
-                d_srng = (int4*)(b + cells * kJgStripWords * sizeof(float));
-                constexpr int nM = kJgWarps * kJgFarNodes * kJgStripNodes;
-                float* d_M = (float*)workspace(ctx, "jg_strip_M", nM * sizeof(float));
-                jg_strip_table_kernel<<<(nM + 255) / 256, 256, 0, st>>>(d_M);
-                check_launch(ctx);
-                if (lm) jg_strip_kernel<true><<<g2, kJgWarps * 32, 0, st>>>(d_segs, d_sn, d_reach, d_pl, go, cut_g, n_strips, d_M, d_sfar, d_srng);
-                else jg_strip_kernel<false><<<g2, kJgWarps * 32, 0, st>>>(d_segs, d_sn, d_reach, d_pl, go, cut_g, n_strips, d_M, d_sfar, d_srng);
-                check_launch(ctx);
-            }
-#define IRS_JG(NO)                                                                                          \
-    do {                                                                                                    \
-        const size_t sm = jg_smem_bytes(NO);                                                                \
-        IRS_CUDA(cudaFuncSetAttribute(jg_linesum_kernel<true, NO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-        IRS_CUDA(cudaFuncSetAttribute(jg_linesum_kernel<false, NO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-        if (lm) jg_linesum_kernel<true, NO><<<g2, kJgWarps * 32, sm, st>>>(d_segs, d_sn, d_sw, d_pl, go, n_nu, cut_g, d_out, d_pert, pstride, d_sfar, d_srng, n_strips); \
-        else jg_linesum_kernel<false, NO><<<g2, kJgWarps * 32, sm, st>>>(d_segs, d_sn, d_sw, d_pl, go, n_nu, cut_g, d_out, d_pert, pstride, d_sfar, d_srng, n_strips); \
+            const bool lm = o.line_mixing == IRS_LM_PER_LINE_Y;
+            double margin = 0.0;
+            for (auto& g : pl.segs) margin = std::max(margin, g.margin_g);
+            const CellIndex ci = cell_index(ctx, go.V, row_off, row_n, n_nu, cut_g + margin);
+            const TreeTables* d_tab = tree_tables(ctx);
+            // far field (jg_tree_kernel), in groups of profile-layers whose node values fit
+            // ctx->strip_buf_max (one profile-layer beyond it runs without)
+            const int npl = np * L, n_strips = (int)((n_nu + kTrStrip - 1) / kTrStrip), n_leaves = n_strips * kTrLeaves;
+            std::vector<int> first(npl + 1, 0);
+            for (int q = 0; q < npl; ++q) first[q + 1] = first[q] + pl.pl_segs[q].y;
+            const size_t cell_bytes = (size_t)jg_sums(lm) * kTrNodes * sizeof(float) + sizeof(int4);
+            const size_t max_cells = std::min((size_t)nseg * n_leaves, ctx->strip_buf_max / cell_bytes);
+            char* fbuf = (char*)workspace(ctx, "jg_far", max_cells * cell_bytes);
+            for (int pa = 0; pa < npl;) {
+                int pb = pa;
+                const int s_a = first[pa];
+                while (pb < npl && (size_t)(first[pb + 1] - s_a) * n_leaves <= max_cells) ++pb;
+                if (pb == pa) pb = pa + 1;
+                const size_t cells = (size_t)(first[pb] - s_a) * n_leaves;
+                float* d_far = nullptr;
+                int4* d_rng = nullptr;
+                if (cells <= max_cells && cells > 0) {
+                    d_rng = (int4*)fbuf;
+                    d_far = (float*)(fbuf + cells * sizeof(int4));
+                    const dim3 g1(n_strips, first[pb] - s_a);
+#define IRS_JGT(LMX)                                                                                                   \
+    do {                                                                                                               \
+        IRS_CUDA(cudaFuncSetAttribute(jg_tree_kernel<LMX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jg_tree_smem(LMX))); \
+        jg_tree_kernel<LMX><<<g1, kJgWarps * 32, jg_tree_smem(LMX), st>>>(d_segs, d_reach, ci, go, cut_g, n_nu, n_leaves, d_tab, \
+                                                                          d_far, d_rng, s_a);                          \
     } while (0)
-            switch (n_out) {
-                case 3: IRS_JG(3); break;
-                case 5: IRS_JG(5); break;
-                case 7: IRS_JG(7); break;
-                case 9: IRS_JG(9); break;
-                default: IRS_JG(11); break;
+                    if (lm) IRS_JGT(true);
+                    else IRS_JGT(false);
+#undef IRS_JGT
+                    check_launch(ctx);
+                }
+                const dim3 g2((unsigned)((n_nu + kJgWarps * kJgWarpPts - 1) / (kJgWarps * kJgWarpPts)), pb - pa);
+                int store = 1;  // the first launch stores the layer channels
+#define IRS_JGK(MODE)                                                                                                  \
+    if (modes >> MODE & 1u) {                                                                                          \
+        const size_t sm = jg_smem_bytes(MODE >= kJgLm2, n_out);                                                        \
+        IRS_CUDA(cudaFuncSetAttribute(jg_linesum_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+        jg_linesum_kernel<MODE><<<g2, kJgWarps * 32, sm, st>>>(d_segs, d_sw, d_pl, ci, go, n_nu, cut_g, n_out, store, jg_sums(lm), \
+                                                               d_out, d_pert, pstride, d_tab, d_far, d_rng, n_leaves, pa, s_a);    \
+        check_launch(ctx);                                                                                             \
+        store = 0;                                                                                                     \
+    }
+                IRS_JGK(kJg2)
+                IRS_JGK(kJg3)
+                IRS_JGK(kJg4)
+                IRS_JGK(kJgLm2)
+                IRS_JGK(kJgLm3)
+#undef IRS_JGK
+                pa = pb;
             }
-#undef IRS_JG
-            check_launch(ctx);
         }
         ContDev cd = cont_dev(ctx, o);
         if (o.apply_continuum) {

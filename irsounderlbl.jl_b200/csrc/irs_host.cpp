@@ -289,6 +289,31 @@ void t64_tables(double* out) {
             for (int i = 0; i < P; ++i) *o++ = weight(k, (2.0L * i - (P - 1)) / P);
 }
 
+// ------------------------------------ interpolation tables (FP32 line sums' tree)
+// 16 Chebyshev nodes as rounded to FP32 (where the kernels evaluate): weights at the nodes
+// of a block's two halves, M[half][k][j], and at the 128 points of a leaf, L[k][i].
+void tree32_tables(double* M, float* L) {
+    constexpr int N = 16;
+    long double xk[N], wk[N];
+    for (int k = 0; k < N; ++k) xk[k] = (float)std::cos((2 * k + 1) * 3.14159265358979323846264338327950288L / (2 * N));
+    for (int k = 0; k < N; ++k) {
+        wk[k] = 1.0L;
+        for (int l = 0; l < N; ++l)
+            if (l != k) wk[k] *= xk[k] - xk[l];
+    }
+    auto weight = [&](int k, long double x) {
+        long double p = 1.0L;
+        for (int l = 0; l < N; ++l)
+            if (l != k) p *= x - xk[l];
+        return p / wk[k];
+    };
+    for (int h = 0; h < 2; ++h)
+        for (int k = 0; k < N; ++k)
+            for (int j = 0; j < N; ++j) *M++ = (double)weight(k, (2 * h - 1 + xk[j]) / 2.0L);
+    for (int k = 0; k < N; ++k)
+        for (int i = 0; i < 128; ++i) *L++ = (float)weight(k, (2.0L * i - 127) / 128);
+}
+
 // --------------------------------------------------- Faddeeva constants
 static void weideman_coefficients(int N, double* L_out, double* a_out) {
     const int M = 2 * N, M2 = 2 * M;

@@ -32,6 +32,8 @@ struct Error {
 // Tables of the FP64 line sum's interpolation (T64Tables, linesum_tree64.cuh) as one array
 constexpr int kT64TableDoubles = 32 + 4 * 32 * 32 + 32 * 128 + 32 * 32;
 void t64_tables(double* out);
+// ... and of the FP32 line sums' tree (TreeTables, linesum_tree32.cuh): M, then L
+void tree32_tables(double* M, float* L);
 
 // ------------------------------------------------------------------ grids
 // Julia's float range a:s:b (src/Utils/wavenumber_grid.jl:23-26): start, step and
@@ -69,7 +71,9 @@ struct Segment {
 };
 // SEG_LM: per-line Y dispersive sum fused into the line sum; SEG_RELMAT: the
 // relaxation-matrix perturbation of this (profile, layer) is added before the clamp.
-enum { SEG_DPTMIN = 1, SEG_LM = 2, SEG_RELMAT = 4 };
+// SEG_NEED_P, SEG_NEED_V (Jacobian): the pressure and self-broadening derivatives have a
+// non-zero weight in some layer channel of the segment (retrieved species only).
+enum { SEG_DPTMIN = 1, SEG_LM = 2, SEG_RELMAT = 4, SEG_NEED_P = 8, SEG_NEED_V = 16 };
 
 // Per (profile, layer) inputs of the fused RTE/continuum kernel.
 struct LayerRT {

@@ -15,21 +15,27 @@
 #include "faddeeva.cuh"
 #include "lineparams.cuh"
 #include "linesum.cuh"
+#include "linesum_tree32.cuh"
 #include "rte_ils.cuh"
 
 namespace irs {
 
 constexpr int kJgMaxOut = 11;  // tau, T_lo, T_hi, and (lo, hi) for up to 4 retrieved species
 
-// Per-line primitives (FP64 physics, stored FP32 except the centres), grid units.
+// Per-line primitives (FP64 physics, stored FP32 except the sorted key), grid units.  q2
+// and q3 are written only for segments that need them (SEG_NEED_P, SEG_NEED_V), q4 with
+// line mixing.
 struct JgOut {
-    double *V, *U;          // sorted key, shifted centre
+    double* V;              // sorted key
+    float2* U;              // shifted centre as hi + lo (split_hi_lo)
+    float* df;              // core half-width x_far / fx
     float4 *q0;             // An, fx, y, Hc
     float4 *q1;             // An_T, fx_T, y_T, Hc_T
-    float4 *q2;             // y_p, u_p, Hc_p, dfar
+    float4 *q2;             // y_p, u_p, Hc_p, -
     float4 *q3;             // y_v, u_v, Hc_v, -
     float4 *q4;             // Yw, Yw_T, Yw_p, -
 };
+constexpr size_t kJgLineBytes = 8 + 8 + 4 + 5 * 16;
 
 // cross_section_jacobian.jl:43-56 in FP64 (H and its x, y gradient)
 __device__ __forceinline__ void h_and_grad64(double x, double y, double x_far, double& H, double& Hx, double& Hy) {
@@ -112,12 +118,15 @@ __global__ void __launch_bounds__(256) jg_params_kernel(const SegDev* __restrict
         }
     }
     o.V[slot] = (nu - cfg.grid0) / dg;
-    o.U[slot] = (nu0 - cfg.grid0) / dg;
+    o.U[slot] = split_hi_lo((nu0 - cfg.grid0) / dg, cfg.u_gran, 1.0 / cfg.u_gran);
+    o.df[slot] = (float)fmin(cfg.x_far / (f * dg), 1.0e30);
     o.q0[slot] = make_float4((float)(Sn * co), (float)(f * dg), (float)y, (float)Hc);
     o.q1[slot] = make_float4((float)(dSnT * co), (float)(df * dg), (float)dyT, (float)dHcT);
-    o.q2[slot] = make_float4((float)dyp, (float)(dn0p / dg), (float)dHcp, (float)fmin(cfg.x_far / (f * dg), 1.0e30));
-    o.q3[slot] = make_float4((float)dyv, (float)(dn0v / dg), (float)dHcv, 0.f);
-    o.q4[slot] = make_float4((float)Yw, (float)YwT, (float)Ywp, 0.f);
+    if (sg.flags & (SEG_NEED_P | SEG_NEED_V)) {
+        o.q2[slot] = make_float4((float)dyp, (float)(dn0p / dg), (float)dHcp, 0.f);
+        o.q3[slot] = make_float4((float)dyv, (float)(dn0v / dg), (float)dHcv, 0.f);
+    }
+    if (sg.flags & SEG_LM) o.q4[slot] = make_float4((float)Yw, (float)YwT, (float)Ywp, 0.f);
     if (core_reach) {  // the segment's largest core half-width (non-negative floats order as their bits)
         const unsigned mask = __activemask();
         const unsigned r = __reduce_max_sync(mask, __float_as_uint((float)fmin(cfg.x_far / (f * dg), 1.0e30)));
@@ -127,770 +136,829 @@ __global__ void __launch_bounds__(256) jg_params_kernel(const SegDev* __restrict
 
 // ------------------------------------------------------------------ line sum
 constexpr int kJgQ = 4;                        // points per lane
-constexpr int kJgWarpPts = 32 * kJgQ;          // 128 points per warp
+constexpr int kJgWarpPts = 32 * kJgQ;          // 128 points per warp: a leaf of the tree
 constexpr int kJgWarps = 8;
-constexpr int kJgStrip = kJgWarps * kJgWarpPts;
+static_assert(kJgWarpPts == kTrLeaf, "one warp per leaf");
 
-// Per pair: the value and derivative terms of one line at offset d (grid units).
-// H-ped and its derivatives; x = d fx, y; c1 = P/cut^2, c0 = -2P with P = An Hc.
-// Far wing: H = y/(sqrt(pi)(x^2+y^2)); core: FP32 Faddeeva with w' = -2 z w + 2i/sqrt(pi).
-template <bool LM>
-__device__ __forceinline__ void jg_pair(float d, bool core, const float4& q0, const float4& q1, const float4& q2,
-                                        const float4& q3, const float4& q4, float icut2, float& s, float& sT,
-                                        float& sp, float& sv, float& D, float& DT, float& Dp) {
-    const float An = q0.x, fx = q0.y, y = q0.z, Hc = q0.w;
-    const float x = d * fx;
-    const float xT = d * q1.y;          // u_T = 0
-    const float xp = -fx * q2.y, xv = -fx * q3.y;
-    float H, Hx, Hy, Lw = 0.f, Lx = 0.f, Ly = 0.f;
-    if (core) {
-        const float2 w = faddeeva32_fast(x, y);
-        H = w.x;
-        Hx = -2.f * x * w.x + 2.f * y * w.y;
-        Hy = 2.f * (x * w.y + y * w.x) - 2.f * (float)kInvSqrtPi;
-        if (LM) {
-            Lw = w.y;
-            Lx = -2.f * (x * w.y + y * w.x) + 2.f * (float)kInvSqrtPi;
-            Ly = Hx;
-        }
-    } else {
-        const float e = fmaf(x, x, y * y);
-        const float r = rcp_approx32(e);
-        const float r2 = r * r;
-        const float k = (float)kInvSqrtPi;
-        H = y * k * r;
-        Hx = -2.f * x * y * k * r2;
-        Hy = k * (x * x - y * y) * r2;
-        if (LM) {
-            Lw = x * k * r;
-            Lx = k * (y * y - x * x) * r2;
-            Ly = -2.f * x * y * k * r2;
-        }
-    }
-    // pedestal (2 - (d/cut)^2) Hc and its derivatives; the factor moves with the centre
-    const float pf = 2.f - d * d * icut2;
-    const float pfp = 2.f * d * q2.y * icut2, pfv = 2.f * d * q3.y * icut2;
-    const float Hm = H - pf * Hc;
-    s += An * Hm;
-    sT += q1.x * Hm + An * (Hx * xT + Hy * q1.z - pf * q1.w);
-    sp += An * (Hx * xp + Hy * q2.x - (pfp * Hc + pf * q2.z));
-    sv += An * (Hx * xv + Hy * q3.x - (pfv * Hc + pf * q3.z));
-    if (LM) {
-        D += q4.x * Lw;
-        DT += q4.y * Lw + q4.x * (Lx * xT + Ly * q1.z);
-        Dp += q4.z * Lw + q4.x * (Lx * xp + Ly * q2.x);
+// Segment weights onto the layer channels: channel o += w[0] s + w[1] s_T + w[2] s_p + w[3]
+// s_v, for channels 0..2 (tau, T_lo, T_hi) and, for a retrieved species, its two (lo, hi) at
+// 3 + 2 r for the bits r of retr.
+struct SegW {
+    float base[3][4], pair[2][4];
+    unsigned retr;
+};
+
+// The sums of a segment: NS of (value, d/dT, d/dp, d/dv_self), and with line mixing the
+// dispersive value, d/dT and (NS >= 3) d/dp.  Only the channels of a retrieved species read
+// d/dp, and only those of water d/dv (SegW): the other segments sum two terms a pair
+// instead of four (SEG_NEED_P, SEG_NEED_V).
+//
+// Per pair of the general form: H-ped and its derivatives; x = d fx, y; P = An Hc.
+// Far wing: H = y/(sqrt(pi)(x^2+y^2)); core: FP32 Faddeeva and its gradient (H_x, H_y).
+template <bool LM, int NS>
+__device__ __forceinline__ void jg_core_terms(float d, float2 w, float2 gr, const float4& q0, const float4& q1, const float4& q2,
+                                              const float4& q3, const float4& q4, float t[7]) {
+    const float An = q0.x, fx = q0.y, xT = d * q1.y, Hx = gr.x, Hy = gr.y;
+    t[0] = An * w.x;
+    t[1] = q1.x * w.x + An * (Hx * xT + Hy * q1.z);
+    if (NS >= 3) t[2] = An * (Hy * q2.x - Hx * (fx * q2.y));
+    if (NS >= 4) t[3] = An * (Hy * q3.x - Hx * (fx * q3.y));
+    if (LM) {  // L = Im w: L_x = -H_y, L_y = H_x
+        t[4] = q4.x * w.y;
+        t[5] = q4.y * w.y + q4.x * (Hx * q1.z - Hy * xT);
+        if (NS >= 3) t[6] = q4.z * w.y + q4.x * (Hy * (fx * q2.y) + Hx * q2.x);
     }
 }
 
-// Warp-private staging of one 32-line tile, compacted into the two line classes.
-// Fast lines (all 128 points of the warp inside the cutoff and outside the Faddeeva
-// core) carry closed-form coefficients of the far-wing terms in rho = 1/(d^2 + b2),
-// d the offset in grid units and b2 = (y/fx)^2:
+// The general form of a pair, pedestal included: (H - pf Hc) and its derivatives, the wing
+// from x and y themselves, so that where H and the pedestal nearly cancel (narrow cutoffs)
+// they carry the same roundings.
+template <bool LM, int NS>
+__device__ __forceinline__ void jg_pair(float d, bool core, const float4& q0, const float4& q1, const float4& q2,
+                                        const float4& q3, const float4& q4, float icut2, float t[7]) {
+    const float An = q0.x, fx = q0.y, y = q0.z, Hc = q0.w, x = d * fx, xT = d * q1.y;
+    float2 w, gr;
+    if (core) {
+        w = faddeeva32_grad(x, y, gr);
+    } else {
+        constexpr float k = (float)kInvSqrtPi;
+        const float r = rcp_approx32(fmaf(x, x, y * y)), r2 = r * r;
+        w = make_float2(y * k * r, x * k * r);
+        gr = make_float2(-2.f * x * y * k * r2, k * (x * x - y * y) * r2);
+    }
+    // pedestal (2 - (d/cut)^2) Hc and its derivatives; the factor moves with the centre
+    const float pf = 2.f - d * d * icut2, Hm = w.x - pf * Hc;
+    t[0] = An * Hm;
+    t[1] = q1.x * Hm + An * (gr.x * xT + gr.y * q1.z - pf * q1.w);
+    if (NS >= 3) t[2] = An * (gr.y * q2.x - gr.x * (fx * q2.y) - (2.f * d * q2.y * icut2 * Hc + pf * q2.z));
+    if (NS >= 4) t[3] = An * (gr.y * q3.x - gr.x * (fx * q3.y) - (2.f * d * q3.y * icut2 * Hc + pf * q3.z));
+    if (LM) {
+        t[4] = q4.x * w.y;
+        t[5] = q4.y * w.y + q4.x * (gr.x * q1.z - gr.y * xT);
+        if (NS >= 3) t[6] = q4.z * w.y + q4.x * (gr.y * (fx * q2.y) + gr.x * q2.x);
+    }
+}
+
+// The far wing of a line in rho = 1/(d^2 + b2), d the offset in grid units and b2 = (y/fx)^2:
 //   s  = a_s rho
 //   sT = aT1 rho + aT2 rho^2
 //   sp = ap1 rho + ap2 rho^2 + ap3 d rho^2        (sv likewise)
 //   D  = cD d rho,  DT = cT1 d rho + cT2 d rho^2,
 //   Dp = cp1 d rho + cp2 rho + cp3 rho^2 + cp4 d rho^2          (line mixing)
-// which follow from H = y/(sqrt(pi)(x^2+y^2)), its x and y derivatives and
-// x = d fx (x_T = d fx_T, x_p = -fx u_p); their pedestals are quadratics in the point
-// index summed over the tile.  Slow lines keep the general per-pair form (jg_pair).
-struct JgTile {
-    float4 fu[32];   // fast: uh, ul, b2, a_s
-    float4 fT[32];   // fast: aT1, aT2, ap1, ap2
-    float4 fp[32];   // fast: ap3, av1, av2, av3
-    float4 fL0[32];  // fast, line mixing: cD, cT1, cT2, cp1
-    float4 fL1[32];  // fast, line mixing: cp2, cp3, cp4, -
-    float4 su[32];   // slow: uh, ul, -, dfar2
-    float4 q0[32], q1[32], q2[32], q3[32], q4[32];  // slow: per-line primitives
-};
-
-// The far-wing coefficients of one line (the JgTile fast-line layout; fu = (-, -, b2,
-// a_s)) and its pedestal scales P[o] (value, d/dT, d/dp, d/dv) of -P pf,
-// pf = 2 - (i - u)^2 / c^2 (pf also moves with the centre for d/dp and d/dv).
-template <bool LM>
+// which follow from H = y/(sqrt(pi)(x^2+y^2)), its x and y derivatives and x = d fx
+// (x_T = d fx_T, x_p = -fx u_p).  f0 = (-, -, b2, a_s), f1 = (aT1, aT2, ap1, ap2),
+// f2 = (ap3, av1, av2, av3), l0 = (cD, cT1, cT2, cp1), l1 = (cp2, cp3, cp4, -), and the
+// pedestal scales P[o] of -P pf, pf = 2 - (i - u)^2 / c^2 (pf also moves with the centre for
+// d/dp and d/dv).  1/fx by the MUFU reciprocal (about 1 ulp).
+template <bool LM, int NS>
 __device__ __forceinline__ void jg_wing_coeffs(const float4& a0, const float4& a1, const float4& a2,
-                                               const float4& a3, const float4& a4, float4& fu, float4& fT,
-                                               float4& fp, float4& fL0, float4& fL1, float P[4]) {
+                                               const float4& a3, const float4& a4, float4& f0, float4& f1,
+                                               float4& f2, float4& l0, float4& l1, float P[4]) {
     constexpr float k = (float)kInvSqrtPi;
     const float An = a0.x, fx = a0.y, y = a0.z, Hc = a0.w;
     const float AnT = a1.x, fxT = a1.y, yT = a1.z, HcT = a1.w;
-    const float yp = a2.x, up = a2.y, Hcp = a2.z, yv = a3.x, uv = a3.y, Hcv = a3.z;
-    // 1/fx by the MUFU reciprocal (about 1 ulp) instead of IEEE divisions: these are
-    // far-wing coefficients of an FP32 sum
     const float ifx = rcp_fast(fx);
-    const float gg = ifx * ifx, b2 = y * y * gg, Aky = An * k * y;
-    fu = make_float4(0.f, 0.f, b2, Aky * gg);
+    const float gg = ifx * ifx, b2 = y * y * gg, Aky = An * k * y, Akg = An * k * gg;
     const float r_fx = fxT * ifx;
-    fT = make_float4(gg * k * (AnT * y + An * yT) - 2.f * Aky * r_fx * gg,
-                     2.f * Aky * b2 * r_fx * gg - 2.f * An * k * yT * b2 * gg, An * k * yp * gg,
-                     -2.f * An * k * yp * b2 * gg);
-    fp = make_float4(2.f * Aky * up * gg, An * k * yv * gg, -2.f * An * k * yv * b2 * gg, 2.f * Aky * uv * gg);
-    if (LM) {
-        const float Yw = a4.x, YwT = a4.y, Ywp = a4.z;
-        fL0 = make_float4(Yw * k * ifx, YwT * k * ifx - Yw * k * gg * fxT,
-                          2.f * Yw * k * gg * fxT * b2 - 2.f * Yw * k * y * fx * yT * gg * gg, Ywp * k * ifx);
-        fL1 = make_float4(Yw * k * up * ifx, -2.f * Yw * k * up * b2 * ifx, -2.f * Yw * k * y * fx * yp * gg * gg, 0.f);
-    }
-    // pedestals: -P0 pf, -PT pf, -An Hc pf_p - An Hc_p pf, ... with pf = 2 - (i - u)^2 / c^2
+    f0 = make_float4(0.f, 0.f, b2, Aky * gg);
+    f1 = make_float4(gg * k * (AnT * y + An * yT) - 2.f * Aky * r_fx * gg, 2.f * Aky * b2 * r_fx * gg - 2.f * Akg * yT * b2,
+                     0.f, 0.f);
     P[0] = An * Hc;
     P[1] = AnT * Hc + An * HcT;
-    P[2] = An * Hcp;
-    P[3] = An * Hcv;
+    if (NS >= 3) {
+        f1.z = Akg * a2.x;
+        f1.w = -2.f * Akg * a2.x * b2;
+        f2.x = 2.f * Aky * a2.y * gg;
+        P[2] = An * a2.z;
+    }
+    if (NS >= 4) {
+        f2.y = Akg * a3.x;
+        f2.z = -2.f * Akg * a3.x * b2;
+        f2.w = 2.f * Aky * a3.y * gg;
+        P[3] = An * a3.z;
+    }
+    if (LM) {
+        const float Yw = a4.x, YwT = a4.y, Ywp = a4.z;
+        l0 = make_float4(Yw * k * ifx, YwT * k * ifx - Yw * k * gg * fxT,
+                         2.f * Yw * k * gg * fxT * b2 - 2.f * Yw * k * y * fx * yT * gg * gg, Ywp * k * ifx);
+        if (NS >= 3)
+            l1 = make_float4(Yw * k * a2.y * ifx, -2.f * Yw * k * a2.y * b2 * ifx, -2.f * Yw * k * y * fx * a2.x * gg * gg, 0.f);
+    }
 }
 
 // A line's pedestals as quadratics in the point index i (value A + B i + C i^2, the
 // centre u in the same coordinates as i)
+template <int NS>
 __device__ __forceinline__ void jg_pedestal_quadratics(const float P[4], const float4& a0, const float4& a2,
-                                                       const float4& a3, float u, float icut2, float pA[4],
-                                                       float pB[4], float pC[4]) {
+                                                       const float4& a3, float u, float icut2, float pA[NS],
+                                                       float pB[NS], float pC[NS]) {
     const float e0 = 2.f - u * u * icut2, e1 = 2.f * u * icut2;
 #pragma unroll
-    for (int o = 0; o < 4; ++o) {
+    for (int o = 0; o < NS; ++o) {
         pA[o] = -P[o] * e0;
         pB[o] = -P[o] * e1;
         pC[o] = P[o] * icut2;
     }
     const float shp = 2.f * a0.x * a0.w * icut2;  // pf_p = 2 (i - u) u_p / c^2
-    pA[2] += shp * a2.y * u;
-    pB[2] -= shp * a2.y;
-    pA[3] += shp * a3.y * u;
-    pB[3] -= shp * a3.y;
-}
-
-// Far field of the Jacobian sums: as in the forward line sum, the fast lines whose
-// centres lie kJgFarDist or more points from the centre of the warp's 128-point block
-// are summed at the 8 Chebyshev nodes of the block (all seven sums: s, s_T, s_p, s_v
-// and the three dispersive ones) and interpolated; kJgFarDist / 64 = 5 gives the same
-// 1.6e-7 bound on one line's interpolation error as the forward kernel's 640 / 128.
-constexpr float kJgFarDist = 320.f;
-constexpr int kJgFarNodes = 8;
-struct JgFarTable {
-    float L[kJgFarNodes][kJgWarpPts];
-};
-__device__ __forceinline__ double jg_far_node(int k) {
-    return 63.5 + 63.5 * cos((2 * k + 1) * 3.14159265358979323846 / (2 * kJgFarNodes));
-}
-__device__ __forceinline__ void jg_far_table_init(JgFarTable& F) {
-    for (int idx = threadIdx.x; idx < kJgFarNodes * kJgWarpPts; idx += blockDim.x) {
-        const int kk = idx / kJgWarpPts, i = idx % kJgWarpPts;
-        double v = 1.0;
-        for (int j = 0; j < kJgFarNodes; ++j)
-            if (j != kk) v *= ((double)i - jg_far_node(j)) / (jg_far_node(kk) - jg_far_node(j));
-        F.L[kk][i] = (float)v;
+    if (NS >= 3) {
+        pA[2] += shp * a2.y * u;
+        pB[2] -= shp * a2.y;
+    }
+    if (NS >= 4) {
+        pA[3] += shp * a3.y * u;
+        pB[3] -= shp * a3.y;
     }
 }
 
-// ---------------------------------------------------------- strip far field
-// As for the forward line sum (strip_far_kernel): a line whose shifted centre lies
-// kJgStripR or more points from the centre of a 1024-point strip (the 8 warps of a CTA),
-// whose cutoff covers the strip and whose Faddeeva core stays off it, is evaluated once
-// per strip at 16 Chebyshev nodes, for the four sums (seven with VP_Y on the segment),
-// pedestals included (quadratics, reproduced by the interpolation); the degree-15
-// interpolants go to each warp's 8 nodes through the fixed matrix M and join the
-// warp's own far field.  Worst error of one line's term: 1.6e-8 of its largest value
-// on the strip (poles 2 half-widths or more from its centre).  Its lines are two index
-// ranges per (segment, strip), taken out of every warp's window.
-constexpr float kJgStripR = 1024.f;
-constexpr double kJgStripCentre = 0.5 * (kJgStrip - 1);  // 511.5
-constexpr int kJgStripNodes = 16;
-constexpr int kJgStripOut = 7;                                       // s, s_T, s_p, s_v, D, D_T, D_p
-constexpr int kJgStripWords = kJgWarps * kJgStripOut * kJgFarNodes;  // per (segment, strip)
-constexpr int kJgStripSegs = 4;                                      // segments per block-wide exchange
-// the nodes relative to the strip centre, 511.5 cos((2k+1) pi / 32), rounded to FP32
-__device__ __forceinline__ float jg_strip_node_f(int k) {
-    const int a = k < 8 ? k : 15 - k;
-    const float v = a == 0 ? 5.090369873e+02f : a == 1 ? 4.894749756e+02f : a == 2 ? 4.511027222e+02f
-                  : a == 3 ? 3.953948364e+02f : a == 4 ? 3.244921570e+02f : a == 5 ? 2.411194305e+02f
-                  : a == 6 ? 1.484806061e+02f : 5.013576889e+01f;
-    return k < 8 ? v : -v;
+// adds the wing's terms of two points (packed): dn their offsets, rho their reciprocals
+template <bool LM, int NS>
+__device__ __forceinline__ void jg_wing_add(float2 dn, float2 rho, const float4& f0, const float4& f1, const float4& f2,
+                                            const float4& l0, const float4& l1, float2 v[7]) {
+    const float2 rho2 = __fmul2_rn(rho, rho);
+    v[0] = __ffma2_rn(make_float2(f0.w, f0.w), rho, v[0]);
+    v[1] = __ffma2_rn(make_float2(f1.x, f1.x), rho, __ffma2_rn(make_float2(f1.y, f1.y), rho2, v[1]));
+    if (NS >= 3 || LM) {
+        const float2 drho2 = __fmul2_rn(dn, rho2);
+        if (NS >= 3)
+            v[2] = __ffma2_rn(make_float2(f1.z, f1.z), rho,
+                              __ffma2_rn(make_float2(f1.w, f1.w), rho2, __ffma2_rn(make_float2(f2.x, f2.x), drho2, v[2])));
+        if (NS >= 4)
+            v[3] = __ffma2_rn(make_float2(f2.y, f2.y), rho,
+                              __ffma2_rn(make_float2(f2.z, f2.z), rho2, __ffma2_rn(make_float2(f2.w, f2.w), drho2, v[3])));
+        if (LM) {
+            const float2 drho = __fmul2_rn(dn, rho);
+            v[4] = __ffma2_rn(make_float2(l0.x, l0.x), drho, v[4]);
+            v[5] = __ffma2_rn(make_float2(l0.y, l0.y), drho, __ffma2_rn(make_float2(l0.z, l0.z), drho2, v[5]));
+            if (NS >= 3)
+                v[6] = __ffma2_rn(make_float2(l0.w, l0.w), drho,
+                                  __ffma2_rn(make_float2(l1.x, l1.x), rho,
+                                             __ffma2_rn(make_float2(l1.y, l1.y), rho2,
+                                                        __ffma2_rn(make_float2(l1.z, l1.z), drho2, v[6]))));
+        }
+    }
+}
+// offsets and reciprocals of two points: xn their positions (natural), xs swapped; one MUFU
+// reciprocal of the product of the swapped denominators serves both
+__device__ __forceinline__ void jg_offsets(float2 xn, float2 xs, float uh, float ul, float b2, float2& dn, float2& rho) {
+    const float2 nu_ = make_float2(-uh, -uh), nl = make_float2(-ul, -ul);
+    dn = __fadd2_rn(__fadd2_rn(xn, nu_), nl);
+    const float2 ds = __fadd2_rn(__fadd2_rn(xs, nu_), nl);
+    const float2 es = __ffma2_rn(ds, ds, make_float2(b2, b2));
+    const float R = rcp_fast(es.x * es.y);
+    rho = __fmul2_rn(es, make_float2(R, R));
 }
 
-// M[w][j][k] = L_k(node j of warp w) for the strip nodes k; one thread per entry
-__global__ void jg_strip_table_kernel(float* __restrict__ M) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kJgWarps * kJgFarNodes * kJgStripNodes) return;
-    const int w = i / (kJgFarNodes * kJgStripNodes), j = (i / kJgStripNodes) % kJgFarNodes, k = i % kJgStripNodes;
-    const double x = (double)kJgWarpPts * w + jg_far_node(j) - kJgStripCentre;
-    const double xk = (double)jg_strip_node_f(k);
-    double v = 1.0;
-    for (int l = 0; l < kJgStripNodes; ++l)
-        if (l != k) v *= (x - (double)jg_strip_node_f(l)) / (xk - (double)jg_strip_node_f(l));
-    M[i] = (float)v;
+// The kinds of segments by their sums.  Line mixing is CO2's and d/dv_self water's, so they
+// do not meet.
+enum { kJg2, kJg3, kJg4, kJgLm2, kJgLm3, kJgModes };
+__host__ __device__ inline int jg_mode(int flags) {
+    if (flags & SEG_LM) return flags & (SEG_NEED_P | SEG_NEED_V) ? kJgLm3 : kJgLm2;
+    return flags & SEG_NEED_V ? kJg4 : flags & SEG_NEED_P ? kJg3 : kJg2;
 }
 
-// One CTA per (strip, profile-layer).  Per batch of segments: the index ranges
-// (rin = max(kJgStripR, core reach + 513) + margin, rout = cut - 512 - margin), then
-// each warp takes tiles warp, warp + 8, ... of the ranges' lines: the lanes stage their
-// lines' far-wing coefficients and sum their pedestal quadratics (the centre as offset
-// from the strip centre), and lane l evaluates nodes l % 8 and l % 8 + 8 (packed) over
-// every fourth staged line;
-// the warps' node and pedestal sums meet in shared memory, and each warp takes them
-// (the warps in a fixed order, pedestals evaluated at the nodes) through M to its own
-// line-sum warp's 8 nodes: far[(segment, strip)][warp][sum][node], and the ranges.
-template <bool ANY_LM>
-__global__ void __launch_bounds__(kJgWarps * 32, 2) jg_strip_kernel(
-    const SegDev* __restrict__ segs, const int* __restrict__ seg_n, const unsigned* __restrict__ core_reach,
-    const int2* __restrict__ pl_segs, JgOut g, float cut_g, int n_strips, const float* __restrict__ M,
-    float* __restrict__ far, int4* __restrict__ ranges) {
-    constexpr int NC = ANY_LM ? 7 : 4;            // sums
-    constexpr int kSlot = kJgStripOut * kJgStripNodes + 12;  // node sums, then A, B, C of the 4 pedestals
-    __shared__ float4 sfu[kJgWarps][32], sfT[kJgWarps][32], sfp[kJgWarps][32];
-    __shared__ float4 sL0[ANY_LM ? kJgWarps : 1][32], sL1[ANY_LM ? kJgWarps : 1][32];
-    __shared__ float slot[kJgStripSegs][kJgWarps][kSlot];
-    __shared__ int sj[kJgStripSegs][4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int strip = blockIdx.x, pl = blockIdx.y;
-    const double c = (double)strip * kJgStrip + kJgStripCentre;
-    const float icut2 = 1.f / (cut_g * cut_g);
-    const float xk = jg_strip_node_f(lane & (kJgStripNodes - 1));  // this lane's node (combining)
-    // this lane's node pair (np, np + 8), np = lane % 8, for the line evaluations
-    const float2 xp = make_float2(jg_strip_node_f(lane & 7), jg_strip_node_f((lane & 7) + 8));
+// sums in use: value, d/dT, [d/dp], [d/dv], then with line mixing D, D_T, [D_p]
+template <bool LM, int NS>
+__device__ __forceinline__ constexpr bool jg_used(int c) {
+    return c < NS || (LM && c >= 4 && c < (NS >= 3 ? 7 : 6));
+}
+
+// ------------------------------------------------------------------ far lines
+// One CTA per (strip of 4096 points, segment): the tree's levels from the strip down to the
+// 32 leaves, each level's own far lines (tree_list) spread over the warps, then the parents'
+// node values through M (FP64) and the next level.  Leaves far[(segment, leaf)][sum][node]
+// and the leaf's ranges.  Against the two levels it replaces (1024-point strips from 1024
+// points, then every warp's 8 nodes from 320 points): see the figures at jg_linesum_kernel.
+struct JgStage {
+    float4 f0[32], f1[32], f2[32];
+};
+struct JgStageLm {
+    float4 l0[32], l1[32];
+};
+__host__ __device__ constexpr int jg_sums(bool lm) { return lm ? 7 : 4; }
+constexpr size_t jg_tree_smem(bool lm) {
+    return (sizeof(JgStage) + (lm ? sizeof(JgStageLm) : 0)) * kJgWarps +
+           (size_t)2 * (kTrLeaves / 2) * jg_sums(lm) * kTrNodes * sizeof(double) +
+           (size_t)kTrLeaves * jg_sums(lm) * kTrNodes * sizeof(float) + 2 * (kTrLeaves / 2) * sizeof(int4);
+}
+
+// one warp's share of a block's far lines at its nodes, written to part[sum][node]
+template <bool LM, int NS>
+__device__ __forceinline__ void jg_block(const JgOut& g, long long off, const TreeList& TL, int first, int step, float cb,
+                                         float h, float icut2, int lane, JgStage& T, JgStageLm* TLm,
+                                         float (*__restrict__ part)[kTrNodes]) {
+    const float2 xp = make_float2(h * tree_node_f(lane & 7), h * tree_node_f((lane & 7) + 8));
     const float2 xps = make_float2(xp.y, xp.x);
-    const int2 rng = pl_segs[pl];
-    for (int s0 = rng.x; s0 < rng.x + rng.y; s0 += kJgStripSegs) {  // block-uniform
-        const int ns = min(kJgStripSegs, rng.x + rng.y - s0);
-        for (int i = warp; i < 4 * ns; i += kJgWarps) {  // search i: bound i % 4 of segment i / 4
-            const SegDev sg = segs[s0 + i / 4];
-            const double reach = (double)__uint_as_float(core_reach[s0 + i / 4]);
-            const double m = sg.margin_g, rin = fmax((double)kJgStripR, reach + 0.5 * kJgStrip + 1.0) + m;
-            const double rout = (double)cut_g - 0.5 * kJgStrip - m;
-            int j = 0;
-            if (rout > rin) {
-                const int b = i % 4;
-                const double v = b == 0 ? c - rout : b == 1 ? c - rin : b == 2 ? c + rin : c + rout;
-                j = (int)warp_lower_bound(g.V + sg.off, v, seg_n[s0 + i / 4], lane);
+    float2 v[7], vs[2], vc[2];  // the value (c = 0) and D (c = 4) compensated over tiles
+#pragma unroll
+    for (int c = 0; c < 7; ++c) v[c] = make_float2(0.f, 0.f);
+    vs[0] = vs[1] = vc[0] = vc[1] = make_float2(0.f, 0.f);
+    float QA[NS], QB[NS], QC[NS], QAc = 0.f, QBc = 0.f, QCc = 0.f;
+#pragma unroll
+    for (int o = 0; o < NS; ++o) QA[o] = QB[o] = QC[o] = 0.f;
+    for (int t0 = 32 * first; t0 < TL.n; t0 += 32 * step) {
+        const int nt = min(32, TL.n - t0);
+        __syncwarp();
+        if (lane < nt) {
+            const long long q = off + tree_line(TL, t0 + lane);
+            const float2 uf = g.U[q];
+            const float uh = (uf.x - cb) - (h - 0.5f), ul = uf.y;  // exact: see split_hi_lo
+            const float4 a0 = g.q0[q], a1 = g.q1[q];
+            float4 a2, a3, a4, f0, f1, f2, l0, l1;
+            if (NS >= 3) { a2 = g.q2[q]; a3 = g.q3[q]; }
+            if (LM) a4 = g.q4[q];
+            float P[4], pA[NS], pB[NS], pC[NS];
+            jg_wing_coeffs<LM, NS>(a0, a1, a2, a3, a4, f0, f1, f2, l0, l1, P);
+            T.f0[lane] = make_float4(uh, ul, f0.z, f0.w);
+            T.f1[lane] = f1;
+            if (NS >= 3) T.f2[lane] = f2;
+            if (LM) {
+                TLm->l0[lane] = l0;
+                if (NS >= 3) TLm->l1[lane] = l1;
             }
-            if (lane == 0) sj[i / 4][i % 4] = j;
+            jg_pedestal_quadratics<NS>(P, a0, a2, a3, uh + ul, icut2, pA, pB, pC);
+            kahan_add(QA[0], QAc, pA[0]);
+            kahan_add(QB[0], QBc, pB[0]);
+            kahan_add(QC[0], QCc, pC[0]);
+#pragma unroll
+            for (int o = 1; o < NS; ++o) {
+                QA[o] += pA[o];
+                QB[o] += pB[o];
+                QC[o] += pC[o];
+            }
+        }
+        __syncwarp();
+        for (int k = lane >> 3; k < nt; k += 4) {  // lane: nodes lane % 8 and + 8, every fourth line
+            const float4 f0 = T.f0[k], f1 = T.f1[k];
+            float4 f2, l0, l1;
+            if (NS >= 3) f2 = T.f2[k];
+            if (LM) {
+                l0 = TLm->l0[k];
+                if (NS >= 3) l1 = TLm->l1[k];
+            }
+            float2 dn, rho;
+            jg_offsets(xp, xps, f0.x, f0.y, f0.z, dn, rho);
+            jg_wing_add<LM, NS>(dn, rho, f0, f1, f2, l0, l1, v);
+        }
+#pragma unroll
+        for (int c = 0; c < (LM ? 2 : 1); ++c) {
+            kahan_add(vs[c].x, vc[c].x, v[4 * c].x);
+            kahan_add(vs[c].y, vc[c].y, v[4 * c].y);
+            v[4 * c] = make_float2(0.f, 0.f);
+        }
+    }
+    v[0] = vs[0];
+    if (LM) v[4] = vs[1];
+    const float xk = (lane & 8) ? xp.y : xp.x;  // node lane % 16
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+        if (!jg_used<LM, NS>(c)) continue;
+        float2 x = v[c];
+        x.x += __shfl_xor_sync(kFull, x.x, 8);
+        x.y += __shfl_xor_sync(kFull, x.y, 8);
+        x.x += __shfl_xor_sync(kFull, x.x, 16);
+        x.y += __shfl_xor_sync(kFull, x.y, 16);
+        float val = (lane & 8) ? x.y : x.x;
+        if (c < NS) {
+            const float A = warp_sum(c == 0 ? QA[0] - QAc : QA[c]), B = warp_sum(c == 0 ? QB[0] - QBc : QB[c]);
+            const float C = warp_sum(c == 0 ? QC[0] - QCc : QC[c]);
+            val += fmaf(xk, fmaf(xk, C, B), A);
+        }
+        if (lane < kTrNodes) part[c][lane] = val;
+    }
+}
+
+template <bool ANY_LM, bool LM, int NS>
+__device__ __forceinline__ void jg_tree_segment(const JgOut& g, long long off, const CellIndex& ci, const int* row,
+                                                float cut, float m, float reach, long long n_nu,
+                                                const TreeTables* __restrict__ tab, float* __restrict__ far,
+                                                int4* __restrict__ ranges, unsigned char* smem) {
+    constexpr int NC = jg_sums(ANY_LM);
+    JgStage* tiles = (JgStage*)smem;
+    JgStageLm* tiles_lm = (JgStageLm*)(tiles + kJgWarps);
+    double* F = (double*)(ANY_LM ? (void*)(tiles_lm + kJgWarps) : (void*)tiles_lm);  // [2][16][NC][16]
+    float(*part)[NC][kTrNodes] = (float(*)[NC][kTrNodes])(F + 2 * (kTrLeaves / 2) * NC * kTrNodes);  // [32]
+    int4* rg = (int4*)(part + kTrLeaves);  // [2][16]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long sb = (long long)blockIdx.x * kTrStrip;
+    const float icut2 = 1.f / (cut * cut);
+#pragma unroll 1
+    for (int l = 0; l < kTrLevels; ++l) {
+        const int nb = 1 << l, wpb = l < 3 ? kJgWarps >> l : 1, bpw = l < 3 ? 1 : nb / kJgWarps;
+        const float h = (float)(kTrStrip >> (l + 1));
+        int4* up = rg + ((l + 1) & 1) * (kTrLeaves / 2);
+        for (int i = 0; i < bpw; ++i) {
+            const int b = l < 3 ? warp / wpb : warp * bpw + i;
+            const long long cb = sb + (long long)b * (kTrStrip >> l);
+            if (cb >= n_nu) break;  // warp-uniform
+            const int4 u = l ? up[b >> 1] : make_int4(0, 0, 0, 0);
+            const int4 own = tree_inside(tree_ranges(ci, row, (float)cb, h, cut, m, reach), u);
+            jg_block<LM, NS>(g, off, tree_list(own, u), l < 3 ? warp % wpb : 0, wpb, (float)cb, h, icut2, lane,
+                             tiles[warp], tiles_lm + warp, part[l < 3 ? warp : b]);
+            if (lane == 0 && (l >= 3 || warp % wpb == 0)) {
+                if (l + 1 < kTrLevels) rg[(l & 1) * (kTrLeaves / 2) + b] = own;
+                else ranges[b] = own;
+            }
         }
         __syncthreads();
-        for (int si = 0; si < ns; ++si) {
-            const SegDev sg = segs[s0 + si];
-            const bool lm = ANY_LM && (sg.flags & SEG_LM);
-            const int jA = sj[si][0], jB = sj[si][1], jC = sj[si][2], jD = sj[si][3];
-            const int nL = jB - jA, n = nL + (jD - jC);
-            float2 v[7];  // this lane's node pair (np, np + 8), np = lane % 8, over lines lane / 8 + 4 i
+        double* Fo = F + (size_t)(l & 1) * (kTrLeaves / 2) * NC * kTrNodes;
+        const double* Fp = F + (size_t)((l + 1) & 1) * (kTrLeaves / 2) * NC * kTrNodes;
+        for (int i = threadIdx.x; i < nb * NC * kTrNodes; i += kJgWarps * 32) {
+            const int j = i % kTrNodes, c = (i / kTrNodes) % NC, b = i / (kTrNodes * NC);
+            if (!jg_used<LM, NS>(c) || sb + (long long)b * (kTrStrip >> l) >= n_nu) continue;
+            double v = 0.0;
+            for (int w = 0; w < wpb; ++w) v += (double)part[b * wpb + w][c][j];
+            if (l) {
+                const double* fp = Fp + ((b >> 1) * NC + c) * kTrNodes;
 #pragma unroll
-            for (int cc = 0; cc < 7; ++cc) v[cc] = make_float2(0.f, 0.f);
-            float QA[4] = {0.f, 0.f, 0.f, 0.f}, QB[4] = {0.f, 0.f, 0.f, 0.f}, QC[4] = {0.f, 0.f, 0.f, 0.f};
-            float QAc = 0.f, QBc = 0.f, QCc = 0.f;
-            for (int t0 = warp * 32; t0 < n; t0 += 32 * kJgWarps) {
-                const int t = t0 + lane, nt = min(32, n - t0);
-                float pA[4] = {0.f, 0.f, 0.f, 0.f}, pB[4] = {0.f, 0.f, 0.f, 0.f}, pC[4] = {0.f, 0.f, 0.f, 0.f};
-                if (t < n) {
-                    const long long q = sg.off + (t < nL ? jA + t : jC + (t - nL));
-                    const double u = g.U[q] - c;
-                    const float uh = (float)u, ul = (float)(u - (double)uh);
-                    const float4 a0 = g.q0[q], a1 = g.q1[q], a2 = g.q2[q], a3 = g.q3[q];
-                    const float4 a4 = lm ? g.q4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    float4 fu, fT, fp, fL0, fL1;
-                    float P[4];
-                    jg_wing_coeffs<ANY_LM>(a0, a1, a2, a3, a4, fu, fT, fp, fL0, fL1, P);
-                    sfu[warp][lane] = make_float4(uh, ul, fu.z, fu.w);
-                    sfT[warp][lane] = fT;
-                    sfp[warp][lane] = fp;
-                    if (ANY_LM) {
-                        sL0[warp][lane] = fL0;
-                        sL1[warp][lane] = fL1;
-                    }
-                    jg_pedestal_quadratics(P, a0, a2, a3, uh, icut2, pA, pB, pC);
+                for (int k = 0; k < kTrNodes; ++k) v = fma(fp[k], tab->M[b & 1][k][j], v);
+            }
+            if (l + 1 < kTrLevels) Fo[(b * NC + c) * kTrNodes + j] = v;
+            else far[(b * NC + c) * kTrNodes + j] = (float)v;
+        }
+        __syncthreads();
+    }
+}
+
+template <bool ANY_LM>
+__global__ void __launch_bounds__(kJgWarps * 32, 3) jg_tree_kernel(
+    const SegDev* __restrict__ segs, const unsigned* __restrict__ core_reach, CellIndex ci, JgOut g, float cut_g,
+    long long n_nu, int n_leaves, const TreeTables* __restrict__ tab, float* __restrict__ far,
+    int4* __restrict__ ranges, int seg0) {
+    extern __shared__ __align__(16) unsigned char jg_tree_sh[];
+    const int s = seg0 + (int)blockIdx.y;
+    const SegDev sg = segs[s];
+    const size_t cell = (size_t)blockIdx.y * n_leaves + (size_t)blockIdx.x * kTrLeaves;
+    float* fo = far + cell * jg_sums(ANY_LM) * kTrNodes;
+    int4* ro = ranges + cell;
+    const int* row = ci.idx + (size_t)sg.list * ci.n;
+    const float m = (float)sg.margin_g, reach = __uint_as_float(core_reach[s]);
+    const int mode = jg_mode(sg.flags);
+#define IRS_JT(LMX, NS) jg_tree_segment<ANY_LM, LMX, NS>(g, sg.off, ci, row, cut_g, m, reach, n_nu, tab, fo, ro, jg_tree_sh)
+    if (ANY_LM && mode == kJgLm2) IRS_JT(ANY_LM, 2);  // block-uniform
+    else if (ANY_LM && mode == kJgLm3) IRS_JT(ANY_LM, 3);
+    else if (mode == kJg4) IRS_JT(false, 4);
+    else if (mode == kJg3) IRS_JT(false, 3);
+    else IRS_JT(false, 2);
+#undef IRS_JT
+}
+
+// ------------------------------------------------------------------ near lines
+// Warp-private staging of one tile (32 lines), ordered by class: fast lines (wing at every
+// point, inside the cutoff: packed pairs of points, pedestals as quadratics), cutoff-edge
+// lines (wing, the cutoff falls among the points), core lines (inside the cutoff, the
+// Faddeeva core reaches some points: only the 32-point rows that it reaches take it; their
+// pedestals are quadratics too, so the cutoff has to be 8 times their reach, where the
+// pedestal is under 1/64 of the line's value at any point and cancels nothing), and general
+// ones (core and cutoff edge, or a narrow cutoff: H - pedestal per pair).  The inner points of core lines
+// (|x| + y < 15, the CF4 and Weideman branches) are evaluated lane-parallel per tile into
+// cw, as in the forward line sum.
+constexpr int kJgBuf = 128;
+template <bool LM>
+struct JgTile {
+    float4 f0[32], f1[32], f2[32];  // uh, ul, b2, a_s; wing coefficients
+    float4 q0[32], q1[32];          // core, general: primitives; edge: pedestals, their centre terms
+    float4 q2[32], q3[32];
+    float4 l0[LM ? 32 : 1], l1[LM ? 32 : 1], q4[LM ? 32 : 1];
+    int4 cr[32];                    // core lines: inner points [x, y], offset in cw, core rows (lo | hi << 8)
+    float df2[32];
+    float2 cw[kJgBuf];
+};
+
+template <bool LM, int NS>
+__device__ __forceinline__ void jg_segment(const SegDev& sg, const JgOut& g, long long wb, int4 own, int wlo, int whi,
+                                           float cut, int lane, JgTile<LM>& T, const float (*__restrict__ Lw)[kTrLeaf],
+                                           const float* __restrict__ gfar, const SegW& W,
+                                           const double* __restrict__ prow, long long pstride,
+                                           float* __restrict__ acc) {
+    constexpr float kCentre = 0.5f * (kJgWarpPts - 1);
+    constexpr float kHalf = 0.5f * kJgWarpPts + 0.5f;
+    const float cut2 = cut * cut, icut2 = 1.f / cut2;
+    const float pl0 = (float)lane;
+    const unsigned lt = (1u << lane) - 1u;
+    float2 S[2], C[2], SD[2], CD[2], V[2][7];  // value (compensated), dispersive value, the derivatives
+    float2 xn[2], xs[2];                       // the lane's points of rows (2h, 2h + 1), natural and swapped
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        S[h] = C[h] = SD[h] = CD[h] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 7; ++c) V[h][c] = make_float2(0.f, 0.f);
+        xn[h] = make_float2(pl0 + 64.f * h, pl0 + 64.f * h + 32.f);
+        xs[h] = make_float2(xn[h].y, xn[h].x);
+    }
+    float QA[NS], QB[NS], QC[NS], QAc = 0.f, QBc = 0.f, QCc = 0.f;
+#pragma unroll
+    for (int o = 0; o < NS; ++o) QA[o] = QB[o] = QC[o] = 0.f;
+    // the lines not taken by the far field: [wlo, own.x), [own.y, own.z), [own.w, whi)
+    const int n1 = max(own.x - wlo, 0), n2 = n1 + (own.z - own.y), n = n2 + max(whi - own.w, 0);
+    for (int t0 = 0; t0 < n; t0 += 32) {
+        const int nt = min(32, n - t0), t = t0 + lane;
+        int cls = 0;
+        float uh = 0.f, ul = 0.f, df = 0.f;
+        float4 a0, a1, a2, a3, a4;
+        if (lane < nt) {
+            const long long q = sg.off + (t < n1 ? wlo + t : t < n2 ? own.y + (t - n1) : own.w + (t - n2));
+            const float2 uf = g.U[q];
+            uh = uf.x - (float)wb;  // exact: see split_hi_lo
+            ul = uf.y;
+            df = g.df[q];
+            const float dist = fabsf(uh - kCentre);
+            const bool wing = dist > df + kHalf, in = dist + kHalf <= cut;
+            cls = dist > cut + kHalf ? 0 : wing ? (in ? 1 : 2) : (in && cut >= 8.f * (df + kHalf) ? 3 : 4);
+            if (cls) {
+                a0 = g.q0[q];
+                a1 = g.q1[q];
+                if (NS >= 3) { a2 = g.q2[q]; a3 = g.q3[q]; }
+                if (LM) a4 = g.q4[q];
+            }
+        }
+        const unsigned m1 = __ballot_sync(kFull, cls == 1), m2 = __ballot_sync(kFull, cls == 2);
+        const unsigned m3 = __ballot_sync(kFull, cls == 3), m4 = __ballot_sync(kFull, cls == 4);
+        const int e1 = __popc(m1), e2 = e1 + __popc(m2), e3 = e2 + __popc(m3), e4 = e3 + __popc(m4);
+        // inner points of the core lines and their offsets in cw (a warp scan)
+        int nin = 0, plo = 1, coff = 0, cfit = 0;
+        if (m3) {  // warp-uniform
+            if (cls == 3 && a0.z < 15.f) {
+                const float hw = (15.f - a0.z) / a0.y + 1.f, c = uh + ul;
+                const float lo = fmaxf(c - hw, 0.f), hi = fminf(c + hw, (float)(kJgWarpPts - 1));
+                if (lo <= hi) {
+                    plo = (int)ceilf(lo);
+                    nin = max((int)floorf(hi) - plo + 1, 0);
                 }
+            }
+            int inc = nin;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(kFull, inc, d);
+                if (lane >= d) inc += v;
+            }
+            coff = inc - nin;
+            const unsigned ov = __ballot_sync(kFull, inc > kJgBuf && nin > 0);
+            cfit = ov ? __shfl_sync(kFull, coff, __ffs(ov) - 1) : __shfl_sync(kFull, inc, 31);
+            if (inc > kJgBuf) nin = 0;  // beyond the buffer: per point
+        }
+        __syncwarp();
+        if (cls) {
+            const int pos = cls == 1 ? __popc(m1 & lt) : cls == 2 ? e1 + __popc(m2 & lt)
+                          : cls == 3 ? e2 + __popc(m3 & lt) : e3 + __popc(m4 & lt);
+            float4 f0, f1, f2, l0, l1;
+            float P[4];
+            jg_wing_coeffs<LM, NS>(a0, a1, a2, a3, a4, f0, f1, f2, l0, l1, P);
+            T.f0[pos] = make_float4(uh, ul, f0.z, f0.w);
+            T.f1[pos] = f1;
+            if (NS >= 3) T.f2[pos] = f2;
+            if (LM) {
+                T.l0[pos] = l0;
+                if (NS >= 3) T.l1[pos] = l1;
+            }
+            if (cls & 1) {  // inside the cutoff at every point
+                float pA[NS], pB[NS], pC[NS];
+                jg_pedestal_quadratics<NS>(P, a0, a2, a3, uh + ul, icut2, pA, pB, pC);
                 kahan_add(QA[0], QAc, pA[0]);
                 kahan_add(QB[0], QBc, pB[0]);
                 kahan_add(QC[0], QCc, pC[0]);
 #pragma unroll
-                for (int o = 1; o < 4; ++o) {
+                for (int o = 1; o < NS; ++o) {
                     QA[o] += pA[o];
                     QB[o] += pB[o];
                     QC[o] += pC[o];
                 }
-                __syncwarp();
-                for (int kk = lane >> 3; kk < nt; kk += 4) {  // packed: one reciprocal per node pair
-                    const float4 f0 = sfu[warp][kk], f1 = sfT[warp][kk], f2 = sfp[warp][kk];
-                    const float2 nu_ = make_float2(-f0.x, -f0.x), nl = make_float2(-f0.y, -f0.y);
-                    const float2 dn = __fadd2_rn(__fadd2_rn(xp, nu_), nl);     // (d_a, d_b)
-                    const float2 dsw = __fadd2_rn(__fadd2_rn(xps, nu_), nl);   // (d_b, d_a)
-                    const float2 es = __ffma2_rn(dsw, dsw, make_float2(f0.z, f0.z));  // (e_b, e_a)
-                    const float R = rcp_fast(es.x * es.y);
-                    const float2 rho = __fmul2_rn(es, make_float2(R, R));     // (1/e_a, 1/e_b)
-                    const float2 rho2 = __fmul2_rn(rho, rho), drho2 = __fmul2_rn(dn, rho2);
-                    v[0] = __ffma2_rn(make_float2(f0.w, f0.w), rho, v[0]);
-                    v[1] = __ffma2_rn(make_float2(f1.x, f1.x), rho, __ffma2_rn(make_float2(f1.y, f1.y), rho2, v[1]));
-                    v[2] = __ffma2_rn(make_float2(f1.z, f1.z), rho,
-                                      __ffma2_rn(make_float2(f1.w, f1.w), rho2,
-                                                 __ffma2_rn(make_float2(f2.x, f2.x), drho2, v[2])));
-                    v[3] = __ffma2_rn(make_float2(f2.y, f2.y), rho,
-                                      __ffma2_rn(make_float2(f2.z, f2.z), rho2,
-                                                 __ffma2_rn(make_float2(f2.w, f2.w), drho2, v[3])));
-                    if (ANY_LM) {
-                        const float4 l0 = sL0[warp][kk], l1 = sL1[warp][kk];
-                        const float2 drho = __fmul2_rn(dn, rho);
-                        v[4] = __ffma2_rn(make_float2(l0.x, l0.x), drho, v[4]);
-                        v[5] = __ffma2_rn(make_float2(l0.y, l0.y), drho, __ffma2_rn(make_float2(l0.z, l0.z), drho2, v[5]));
-                        v[6] = __ffma2_rn(make_float2(l0.w, l0.w), drho,
-                                          __ffma2_rn(make_float2(l1.x, l1.x), rho,
-                                                     __ffma2_rn(make_float2(l1.y, l1.y), rho2,
-                                                                __ffma2_rn(make_float2(l1.z, l1.z), drho2, v[6]))));
-                    }
-                }
-                __syncwarp();
             }
-            float* sl = slot[si][warp];
-#pragma unroll
-            for (int cc = 0; cc < NC; ++cc) {  // the four line groups, then node np and np + 8
-                float2 x = v[cc];
-                x.x += __shfl_xor_sync(kFull, x.x, 8);
-                x.y += __shfl_xor_sync(kFull, x.y, 8);
-                x.x += __shfl_xor_sync(kFull, x.x, 16);
-                x.y += __shfl_xor_sync(kFull, x.y, 16);
-                if (lane < 8) {
-                    sl[cc * kJgStripNodes + lane] = x.x;
-                    sl[cc * kJgStripNodes + lane + 8] = x.y;
+            if (cls == 2) {
+                T.q0[pos] = make_float4(P[0], P[1], NS >= 3 ? P[2] : 0.f, NS >= 4 ? P[3] : 0.f);
+                if (NS >= 3)
+                    T.q1[pos] = make_float4(2.f * a2.y * icut2 * P[0], 2.f * a3.y * icut2 * P[0], 0.f, 0.f);
+            } else if (cls >= 3) {
+                T.q0[pos] = a0;
+                T.q1[pos] = a1;
+                if (NS >= 3) {
+                    T.q2[pos] = a2;
+                    T.q3[pos] = a3;
                 }
-            }
-            float wA[4], wB[4], wC[4];
-            wA[0] = warp_sum(QA[0] - QAc);
-            wB[0] = warp_sum(QB[0] - QBc);
-            wC[0] = warp_sum(QC[0] - QCc);
-#pragma unroll
-            for (int o = 1; o < 4; ++o) {
-                wA[o] = warp_sum(QA[o]);
-                wB[o] = warp_sum(QB[o]);
-                wC[o] = warp_sum(QC[o]);
-            }
-            if (lane == 0) {
-#pragma unroll
-                for (int o = 0; o < 4; ++o) {
-                    sl[kJgStripOut * kJgStripNodes + 3 * o] = wA[o];
-                    sl[kJgStripOut * kJgStripNodes + 3 * o + 1] = wB[o];
-                    sl[kJgStripOut * kJgStripNodes + 3 * o + 2] = wC[o];
-                }
+                if (LM) T.q4[pos] = a4;
+                T.df2[pos] = df * df;
+                const float c = uh + ul;
+                const int rl = (int)fminf(fmaxf((c - df) * (1.f / 32.f) - 0.1f, 0.f), 4.f);  // rows the core reaches
+                const int rh = (int)fminf(fmaxf((c + df) * (1.f / 32.f) + 0.1f, -1.f), 3.f);
+                T.cr[pos] = make_int4(plo, plo + nin - 1, coff, rl | (rh << 8));
             }
         }
-        __syncthreads();
-        const float* Mw = M + ((size_t)warp * kJgFarNodes + (lane & (kJgFarNodes - 1))) * kJgStripNodes;
-        for (int si = 0; si < ns; ++si) {
-            const size_t cell = (size_t)(s0 + si) * n_strips + strip;
-            const bool lm = ANY_LM && (segs[s0 + si].flags & SEG_LM);
-#pragma unroll
-            for (int cc = 0; cc < NC; ++cc) {
-                if (cc >= 4 && !lm) break;
-                float fc = 0.f;  // lane k < 16: node k of sum cc, the warps in a fixed order
-                float A = 0.f, B = 0.f, C = 0.f;
-#pragma unroll
-                for (int w = 0; w < kJgWarps; ++w) {
-                    fc += slot[si][w][cc * kJgStripNodes + (lane & (kJgStripNodes - 1))];
-                    if (cc < 4) {
-                        A += slot[si][w][kJgStripOut * kJgStripNodes + 3 * cc];
-                        B += slot[si][w][kJgStripOut * kJgStripNodes + 3 * cc + 1];
-                        C += slot[si][w][kJgStripOut * kJgStripNodes + 3 * cc + 2];
-                    }
-                }
-                if (cc < 4) fc += fmaf(xk, fmaf(xk, C, B), A);
-                float gv = 0.f;
-#pragma unroll
-                for (int k = 0; k < kJgStripNodes; ++k) gv = fmaf(__ldg(Mw + k), __shfl_sync(kFull, fc, k), gv);
-                if (lane < kJgFarNodes) far[cell * kJgStripWords + (warp * kJgStripOut + cc) * kJgFarNodes + lane] = gv;
-            }
-            if (threadIdx.x == 0) ranges[cell] = make_int4(sj[si][0], sj[si][1], sj[si][2], sj[si][3]);
-        }
-        if (s0 + kJgStripSegs < rng.x + rng.y) __syncthreads();  // slots and ranges reused by the next batch
-    }
-}
-
-template <bool LM>
-__device__ void jg_segment(const SegDev& sg, long long cnt, const JgOut& g, long long wb, float cut, int lane,
-                           JgTile& T, const JgFarTable& FT, float xn, float sum[4][kJgQ], float dsum[3][kJgQ],
-                           int4 sx, const float* __restrict__ gfar) {
-    constexpr float kCentre = 0.5f * (kJgWarpPts - 1);
-    constexpr float kHalf = 0.5f * kJgWarpPts + 0.5f;
-    const float cut2 = cut * cut, icut2 = 1.f / cut2;
-    const long long jlo = warp_lower_bound(g.V + sg.off, (double)wb - cut - sg.margin_g, cnt, lane);
-    const long long jhi =
-        warp_lower_bound(g.V + sg.off, (double)(wb + kJgWarpPts - 1) + cut + sg.margin_g + 1e-9, cnt, lane);
-    const float pl0 = (float)lane;
-    const unsigned lt = (1u << lane) - 1u;
-    // packed accumulators over point pairs (q = 2h, 2h + 1)
-    float2 S[kJgQ / 2], C[kJgQ / 2], ST[kJgQ / 2], SP[kJgQ / 2], SV[kJgQ / 2];
-    float2 SD[kJgQ / 2], CD[kJgQ / 2], SDT[kJgQ / 2], SDP[kJgQ / 2];
-#pragma unroll
-    for (int h = 0; h < kJgQ / 2; ++h) {
-        S[h] = C[h] = ST[h] = SP[h] = SV[h] = make_float2(0.f, 0.f);
-        SD[h] = CD[h] = SDT[h] = SDP[h] = make_float2(0.f, 0.f);
-    }
-    float2 offn[kJgQ / 2], offs[kJgQ / 2];  // natural (32q, 32(q+1)) and swapped offsets
-#pragma unroll
-    for (int h = 0; h < kJgQ / 2; ++h) {
-        offn[h] = make_float2(64.f * h, 64.f * h + 32.f);
-        offs[h] = make_float2(64.f * h + 32.f, 64.f * h);
-    }
-    // far-field node sums: lane l accumulates node l % 8 over every fourth far line
-    float fS = 0.f, fC = 0.f, fT_ = 0.f, fP = 0.f, fV = 0.f, fD = 0.f, fDC = 0.f, fDT = 0.f, fDP = 0.f;
-    // pedestal quadratics of this lane's fast and far lines (the value sum compensated),
-    // reduced over the warp once per segment
-    float QA[4] = {0.f, 0.f, 0.f, 0.f}, QB[4] = {0.f, 0.f, 0.f, 0.f}, QC[4] = {0.f, 0.f, 0.f, 0.f};
-    float QAc = 0.f, QBc = 0.f, QCc = 0.f;
-    // the window without the strip far field's ranges [sx.x, sx.y) and [sx.z, sx.w):
-    // [ilo, ra), [rb, rc) and [rd, ihi), walked in turn (indices within a segment fit in int)
-    const int ilo = (int)jlo, ihi = (int)jhi;
-    const int ra = min(max(sx.x, ilo), ihi), rb = min(max(sx.y, ilo), ihi);
-    const int rc = min(max(sx.z, ilo), ihi), rd = min(max(sx.w, ilo), ihi);
-    int nt = 0;
-    for (int t0 = skip_ranges(ilo, ra, rb, rc, rd); t0 < ihi; t0 = skip_ranges(t0 + nt, ra, rb, rc, rd)) {
-        nt = min(32, (t0 < ra ? ra : t0 < rc ? rc : ihi) - t0);
-        int cls = 0;
-        float uh = 0.f, ul = 0.f;
-        float4 a0, a1, a2, a3, a4;
-        // pedestal quadratic of a fast line: value at point i is A + B i + Cq i^2
-        float pA[4] = {0.f, 0.f, 0.f, 0.f}, pB[4] = {0.f, 0.f, 0.f, 0.f}, pC[4] = {0.f, 0.f, 0.f, 0.f};
-        if (lane < nt) {
-            const long long q = sg.off + t0 + lane;
-            const double u = g.U[q] - (double)wb;
-            uh = (float)u;
-            ul = (float)(u - (double)uh);
-            a0 = g.q0[q];
-            a1 = g.q1[q];
-            a2 = g.q2[q];
-            a3 = g.q3[q];
-            if (LM) a4 = g.q4[q];
-            const float dist = fabsf(uh - kCentre);
-            if (dist > cut + kHalf) cls = 0;
-            else if (dist + kHalf <= cut && dist > a2.w + kHalf) cls = dist >= kJgFarDist ? 3 : 1;
-            else if (dist > a2.w + kHalf) cls = 4;  // far wing everywhere, the cutoff falls among the points
-            else cls = 2;
-        }
-        const unsigned fm = __ballot_sync(kFull, cls == 1), sm = __ballot_sync(kFull, cls == 2);
-        const unsigned xm = __ballot_sync(kFull, cls == 3), em = __ballot_sync(kFull, cls == 4);
         __syncwarp();
-        if (cls == 1 || cls == 3 || cls == 4) {  // fast lines first, far lines after them, edge lines from the top
-            const int pos = cls == 1 ? __popc(fm & lt) : (cls == 3 ? __popc(fm) + __popc(xm & lt) : 31 - __popc(em & lt));
-            float4 fu, fT, fp, fL0, fL1;
-            float P[4];
-            jg_wing_coeffs<LM>(a0, a1, a2, a3, a4, fu, fT, fp, fL0, fL1, P);
-            T.fu[pos] = make_float4(uh, ul, fu.z, fu.w);
-            T.fT[pos] = fT;
-            T.fp[pos] = fp;
-            if (LM) {
-                T.fL0[pos] = fL0;
-                T.fL1[pos] = fL1;
+        if (e4 == 0) continue;
+        if (cfit > 0) {
+            for (int e = lane; e < cfit; e += 32) {  // the line owning element e: the last with offset <= e
+                int lo = e2, hi = e3 - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (T.cr[mid].z <= e) lo = mid; else hi = mid - 1;
+                }
+                const int4 r = T.cr[lo];
+                const float4 u = T.f0[lo], p = T.q0[lo];
+                const float d = ((float)(r.x + (e - r.z)) - u.x) - u.y;
+                T.cw[e] = faddeeva32_inline(d * p.y, p.z);
             }
-            if (cls == 4) {  // edge lines: pedestals per point (masked by the cutoff), in the slow arrays' top
-                T.q0[pos] = make_float4(P[0], P[1], P[2], P[3]);
-                T.q1[pos] = make_float4(2.f * a2.y * icut2 * P[0], 2.f * a3.y * icut2 * P[0], 0.f, 0.f);
+            __syncwarp();
+        }
+        float2 v[2][7];  // this tile's sums of the value terms; the derivatives go to V directly
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            v[h][0] = v[h][4] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < 7; ++c)
+                if (c != 0 && c != 4) v[h][c] = V[h][c];
+        }
+        for (int k = 0; k < e1; ++k) {
+            const float4 f0 = T.f0[k], f1 = T.f1[k];
+            float4 f2, l0, l1;
+            if (NS >= 3) f2 = T.f2[k];
+            if (LM) {
+                l0 = T.l0[k];
+                if (NS >= 3) l1 = T.l1[k];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float2 dn, rho;
+                jg_offsets(xn[h], xs[h], f0.x, f0.y, f0.z, dn, rho);
+                jg_wing_add<LM, NS>(dn, rho, f0, f1, f2, l0, l1, v[h]);
+            }
+        }
+        // cutoff-edge lines: the wing and the pedestals of every point, masked by the cutoff
+        for (int k = e1; k < e2; ++k) {
+            const float4 f0 = T.f0[k], f1 = T.f1[k], P = T.q0[k];
+            float4 f2, l0, l1, pc;
+            if (NS >= 3) { f2 = T.f2[k]; pc = T.q1[k]; }
+            if (LM) {
+                l0 = T.l0[k];
+                if (NS >= 3) l1 = T.l1[k];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float2 dn, rho, e[7];
+                jg_offsets(xn[h], xs[h], f0.x, f0.y, f0.z, dn, rho);
+                const float2 d2 = __fmul2_rn(dn, dn);
+                const float2 pf = __ffma2_rn(d2, make_float2(icut2, icut2), make_float2(-2.f, -2.f));  // -(2 - d^2/c^2)
+                e[0] = __fmul2_rn(make_float2(P.x, P.x), pf);
+                e[1] = __fmul2_rn(make_float2(P.y, P.y), pf);
+                if (NS >= 3) e[2] = __ffma2_rn(make_float2(P.z, P.z), pf, __fmul2_rn(make_float2(-pc.x, -pc.x), dn));
+                if (NS >= 4) e[3] = __ffma2_rn(make_float2(P.w, P.w), pf, __fmul2_rn(make_float2(-pc.y, -pc.y), dn));
+                e[4] = e[5] = e[6] = make_float2(0.f, 0.f);
+                jg_wing_add<LM, NS>(dn, rho, f0, f1, f2, l0, l1, e);
+                const bool ix = d2.x <= cut2, iy = d2.y <= cut2;
+#pragma unroll
+                for (int c = 0; c < 7; ++c)
+                    if (jg_used<LM, NS>(c)) {
+                        v[h][c].x += ix ? e[c].x : 0.f;
+                        v[h][c].y += iy ? e[c].y : 0.f;
+                    }
+            }
+        }
+        // core lines
+        for (int k = e2; k < e3; ++k) {
+            const float4 f0 = T.f0[k], f1 = T.f1[k];
+            float4 f2, l0, l1;
+            if (NS >= 3) f2 = T.f2[k];
+            if (LM) {
+                l0 = T.l0[k];
+                if (NS >= 3) l1 = T.l1[k];
+            }
+            const int4 cr = T.cr[k];
+            const int rl = cr.w & 255, rh = cr.w >> 8;  // rh = -1: none (arithmetic shift)
+            const float df2 = T.df2[k];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float2 dn, rho;
+                jg_offsets(xn[h], xs[h], f0.x, f0.y, f0.z, dn, rho);
+                if (rh < 2 * h || rl > 2 * h + 1) {  // warp-uniform: no core point in these rows
+                    jg_wing_add<LM, NS>(dn, rho, f0, f1, f2, l0, l1, v[h]);
+                    continue;
+                }
+                float2 e[7];
+#pragma unroll
+                for (int c = 0; c < 7; ++c) e[c] = make_float2(0.f, 0.f);
+                jg_wing_add<LM, NS>(dn, rho, f0, f1, f2, l0, l1, e);
+                const float4 q0 = T.q0[k], q1 = T.q1[k];
+                float4 q2, q3, q4;
+                if (NS >= 3) { q2 = T.q2[k]; q3 = T.q3[k]; }
+                if (LM) q4 = T.q4[k];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const float d = r ? dn.y : dn.x;
+                    const bool core = d * d <= df2;
+                    if (!__any_sync(kFull, core)) continue;
+                    const float x = d * q0.y, y = q0.z;
+                    const int pt = lane + 32 * (2 * h + r);
+                    float2 gr;
+                    float2 w = faddeeva_cf2_grad(x, y, y * y, gr);
+                    if (core && fabsf(x) + y < 15.f) {
+                        w = pt >= cr.x && pt <= cr.y ? T.cw[cr.z + pt - cr.x] : faddeeva32(x, y);
+                        gr = wofz_grad32(x, y, w);
+                    }
+                    float t7[7];
+                    jg_core_terms<LM, NS>(d, w, gr, q0, q1, q2, q3, q4, t7);
+                    if (core) {
+#pragma unroll
+                        for (int c = 0; c < 7; ++c)
+                            if (jg_used<LM, NS>(c)) {
+                                if (r) e[c].y = t7[c];
+                                else e[c].x = t7[c];
+                            }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 7; ++c)
+                    if (jg_used<LM, NS>(c)) v[h][c] = __fadd2_rn(v[h][c], e[c]);
+            }
+        }
+        // general lines: the core and the cutoff edge among the points, H - pedestal per pair
+        for (int k = e3; k < e4; ++k) {
+            const float4 f0 = T.f0[k], q0 = T.q0[k], q1 = T.q1[k];
+            float4 q2 = make_float4(0.f, 0.f, 0.f, 0.f), q3 = q2, q4 = q2;
+            if (NS >= 3) { q2 = T.q2[k]; q3 = T.q3[k]; }
+            if (LM) q4 = T.q4[k];
+            const float df2 = T.df2[k];
+#pragma unroll
+            for (int q = 0; q < kJgQ; ++q) {
+                const float d = ((pl0 + 32.f * q) - f0.x) - f0.y, d2 = d * d;
+                if (d2 > cut2) continue;
+                float t7[7];
+                jg_pair<LM, NS>(d, d2 <= df2, q0, q1, q2, q3, q4, icut2, t7);
+                const int h = q >> 1;
+#pragma unroll
+                for (int c = 0; c < 7; ++c)
+                    if (jg_used<LM, NS>(c)) {
+                        if (q & 1) v[h][c].y += t7[c];
+                        else v[h][c].x += t7[c];
+                    }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // the compensated tile sums
+            kahan_add(S[h].x, C[h].x, v[h][0].x);
+            kahan_add(S[h].y, C[h].y, v[h][0].y);
+            if (LM) {
+                kahan_add(SD[h].x, CD[h].x, v[h][4].x);
+                kahan_add(SD[h].y, CD[h].y, v[h][4].y);
+            }
+#pragma unroll
+            for (int c = 0; c < 7; ++c)
+                if (c != 0 && c != 4) V[h][c] = v[h][c];
+        }
+    }
+    // pedestals, and the far field's interpolants, per sum
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+        if (!jg_used<LM, NS>(c)) continue;
+        float2 it[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        if (c < NS) {
+            const float A = warp_sum(c == 0 ? QA[0] - QAc : QA[c]), B = warp_sum(c == 0 ? QB[0] - QBc : QB[c]);
+            const float Cq = warp_sum(c == 0 ? QC[0] - QCc : QC[c]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                it[h].x = fmaf(xn[h].x, fmaf(xn[h].x, Cq, B), A);
+                it[h].y = fmaf(xn[h].y, fmaf(xn[h].y, Cq, B), A);
+            }
+        }
+        if (gfar) {
+            // about the value of a middle node, so that the weights' rounding acts on the
+            // field's variation over the leaf only
+            float nd = gfar[c * kTrNodes + (lane & (kTrNodes - 1))];
+            const float mid = __shfl_sync(kFull, nd, kTrNodes / 2);
+            nd -= mid;
+            float2 f[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+            for (int k = 0; k < kTrNodes; ++k) {
+                const float F = __shfl_sync(kFull, nd, k);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    f[h] = __ffma2_rn(make_float2(F, F), make_float2(Lw[k][64 * h + lane], Lw[k][64 * h + 32 + lane]), f[h]);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (c == 0) {
+                    kahan_add(S[h].x, C[h].x, mid);
+                    kahan_add(S[h].y, C[h].y, mid);
+                } else {
+                    f[h] = __fadd2_rn(f[h], make_float2(mid, mid));
+                }
+                it[h] = __fadd2_rn(it[h], f[h]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (c == 0) {
+                kahan_add(S[h].x, C[h].x, it[h].x);
+                kahan_add(S[h].y, C[h].y, it[h].y);
+                V[h][0] = S[h];
+            } else if (c == 4) {
+                kahan_add(SD[h].x, CD[h].x, it[h].x);
+                kahan_add(SD[h].y, CD[h].y, it[h].y);
+                V[h][4] = SD[h];
             } else {
-                jg_pedestal_quadratics(P, a0, a2, a3, uh, icut2, pA, pB, pC);
-            }
-        } else if (cls == 2) {
-            const int pos = __popc(sm & lt);
-            T.su[pos] = make_float4(uh, ul, 0.f, a2.w * a2.w);
-            T.q0[pos] = a0;
-            T.q1[pos] = a1;
-            T.q2[pos] = a2;
-            T.q3[pos] = a3;
-            if (LM) T.q4[pos] = a4;
-        }
-        kahan_add(QA[0], QAc, pA[0]);
-        kahan_add(QB[0], QBc, pB[0]);
-        kahan_add(QC[0], QCc, pC[0]);
-#pragma unroll
-        for (int o = 1; o < 4; ++o) {
-            QA[o] += pA[o];
-            QB[o] += pB[o];
-            QC[o] += pC[o];
-        }
-        __syncwarp();
-        const int nf = __popc(fm), ns = __popc(sm), nx = __popc(xm), ne = __popc(em);
-        {
-            float ts = 0.f, td = 0.f;
-            for (int kk = nf + (lane >> 3); kk < nf + nx; kk += 4) {
-                const float4 f0 = T.fu[kk], f1 = T.fT[kk], f2 = T.fp[kk];
-                const float d = (xn - f0.x) - f0.y;
-                const float rho = rcp_fast(fmaf(d, d, f0.z));
-                const float rho2 = rho * rho, drho2 = d * rho2;
-                ts = fmaf(f0.w, rho, ts);
-                fT_ = fmaf(f1.x, rho, fmaf(f1.y, rho2, fT_));
-                fP = fmaf(f1.z, rho, fmaf(f1.w, rho2, fmaf(f2.x, drho2, fP)));
-                fV = fmaf(f2.y, rho, fmaf(f2.z, rho2, fmaf(f2.w, drho2, fV)));
-                if (LM) {
-                    const float4 l0 = T.fL0[kk], l1 = T.fL1[kk];
-                    const float drho = d * rho;
-                    td = fmaf(l0.x, drho, td);
-                    fDT = fmaf(l0.y, drho, fmaf(l0.z, drho2, fDT));
-                    fDP = fmaf(l0.w, drho, fmaf(l1.x, rho, fmaf(l1.y, rho2, fmaf(l1.z, drho2, fDP))));
-                }
-            }
-            kahan_add(fS, fC, ts);
-            if (LM) kahan_add(fD, fDC, td);
-        }
-        if (nf + ns + ne == 0) continue;  // warp-uniform: nothing per point in this tile
-        float2 TS[kJgQ / 2], TD[kJgQ / 2];  // tile partials of the value sums (Kahan-added below)
-#pragma unroll
-        for (int h = 0; h < kJgQ / 2; ++h) TS[h] = TD[h] = make_float2(0.f, 0.f);
-        for (int kk = 0; kk < nf; ++kk) {
-            const float4 f0 = T.fu[kk], f1 = T.fT[kk], f2 = T.fp[kk];
-            const float d0 = (pl0 - f0.x) - f0.y;
-            const float2 d0s = make_float2(d0, d0), b2 = make_float2(f0.z, f0.z);
-            float4 l0, l1;
-            if (LM) {
-                l0 = T.fL0[kk];
-                l1 = T.fL1[kk];
-            }
-#pragma unroll
-            for (int h = 0; h < kJgQ / 2; ++h) {
-                const float2 dsw = __fadd2_rn(d0s, offs[h]);      // (d[q+1], d[q])
-                const float2 dn = __fadd2_rn(d0s, offn[h]);       // (d[q], d[q+1])
-                const float2 es = __ffma2_rn(dsw, dsw, b2);       // (e[q+1], e[q])
-                const float R = rcp_fast(es.x * es.y);
-                const float2 rho = __fmul2_rn(es, make_float2(R, R));  // (1/e[q], 1/e[q+1])
-                const float2 rho2 = __fmul2_rn(rho, rho);
-                const float2 drho2 = __fmul2_rn(dn, rho2);
-                TS[h] = __ffma2_rn(make_float2(f0.w, f0.w), rho, TS[h]);
-                ST[h] = __ffma2_rn(make_float2(f1.x, f1.x), rho, ST[h]);
-                ST[h] = __ffma2_rn(make_float2(f1.y, f1.y), rho2, ST[h]);
-                SP[h] = __ffma2_rn(make_float2(f1.z, f1.z), rho, SP[h]);
-                SP[h] = __ffma2_rn(make_float2(f1.w, f1.w), rho2, SP[h]);
-                SP[h] = __ffma2_rn(make_float2(f2.x, f2.x), drho2, SP[h]);
-                SV[h] = __ffma2_rn(make_float2(f2.y, f2.y), rho, SV[h]);
-                SV[h] = __ffma2_rn(make_float2(f2.z, f2.z), rho2, SV[h]);
-                SV[h] = __ffma2_rn(make_float2(f2.w, f2.w), drho2, SV[h]);
-                if (LM) {
-                    const float2 drho = __fmul2_rn(dn, rho);
-                    TD[h] = __ffma2_rn(make_float2(l0.x, l0.x), drho, TD[h]);
-                    SDT[h] = __ffma2_rn(make_float2(l0.y, l0.y), drho, SDT[h]);
-                    SDT[h] = __ffma2_rn(make_float2(l0.z, l0.z), drho2, SDT[h]);
-                    SDP[h] = __ffma2_rn(make_float2(l0.w, l0.w), drho, SDP[h]);
-                    SDP[h] = __ffma2_rn(make_float2(l1.x, l1.x), rho, SDP[h]);
-                    SDP[h] = __ffma2_rn(make_float2(l1.y, l1.y), rho2, SDP[h]);
-                    SDP[h] = __ffma2_rn(make_float2(l1.z, l1.z), drho2, SDP[h]);
-                }
-            }
-        }
-        // cutoff-edge lines: the far-wing coefficients and the per-point pedestals,
-        // masked to the points inside the cutoff
-        for (int e = 0; e < ne; ++e) {
-            const int kk = 31 - e;
-            const float4 f0 = T.fu[kk], f1 = T.fT[kk], f2 = T.fp[kk], P = T.q0[kk], c = T.q1[kk];
-            float4 l0, l1;
-            if (LM) {
-                l0 = T.fL0[kk];
-                l1 = T.fL1[kk];
-            }
-            const float d0 = (pl0 - f0.x) - f0.y;
-#pragma unroll
-            for (int q = 0; q < kJgQ; ++q) {
-                const float d = d0 + 32.f * q, d2 = d * d;
-                if (d2 > cut2) continue;
-                const float rho = rcp_fast(d2 + f0.z), rho2 = rho * rho, drho2 = d * rho2;
-                const float pf = fmaf(-d2, icut2, 2.f);
-                const float vs = fmaf(f0.w, rho, -P.x * pf);
-                const float vT = fmaf(f1.x, rho, fmaf(f1.y, rho2, -P.y * pf));
-                const float vp = fmaf(f1.z, rho, fmaf(f1.w, rho2, fmaf(f2.x, drho2, -fmaf(c.x, d, P.z * pf))));
-                const float vv = fmaf(f2.y, rho, fmaf(f2.z, rho2, fmaf(f2.w, drho2, -fmaf(c.y, d, P.w * pf))));
-                const int h = q >> 1;
-                float vD = 0.f, vDT = 0.f, vDP = 0.f;
-                if (LM) {
-                    const float drho = d * rho;
-                    vD = l0.x * drho;
-                    vDT = fmaf(l0.y, drho, l0.z * drho2);
-                    vDP = fmaf(l0.w, drho, fmaf(l1.x, rho, fmaf(l1.y, rho2, l1.z * drho2)));
-                }
-                if (q & 1) {
-                    TS[h].y += vs; ST[h].y += vT; SP[h].y += vp; SV[h].y += vv;
-                    if (LM) { TD[h].y += vD; SDT[h].y += vDT; SDP[h].y += vDP; }
-                } else {
-                    TS[h].x += vs; ST[h].x += vT; SP[h].x += vp; SV[h].x += vv;
-                    if (LM) { TD[h].x += vD; SDT[h].x += vDT; SDP[h].x += vDP; }
-                }
-            }
-        }
-        for (int kk = 0; kk < ns; ++kk) {
-            const float4 u = T.su[kk];
-            const float4 q0 = T.q0[kk], q1 = T.q1[kk], q2 = T.q2[kk], q3 = T.q3[kk];
-            const float4 q4 = LM ? T.q4[kk] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int q = 0; q < kJgQ; ++q) {
-                const float d = ((pl0 + 32.f * q) - u.x) - u.y;
-                const float d2 = d * d;
-                if (d2 > cut2) continue;
-                float s = 0.f, sT = 0.f, sp = 0.f, sv = 0.f, D = 0.f, DT = 0.f, Dp = 0.f;
-                jg_pair<LM>(d, d2 <= u.w, q0, q1, q2, q3, q4, icut2, s, sT, sp, sv, D, DT, Dp);
-                const int h = q >> 1;
-                if (q & 1) {
-                    TS[h].y += s; ST[h].y += sT; SP[h].y += sp; SV[h].y += sv;
-                    if (LM) { TD[h].y += D; SDT[h].y += DT; SDP[h].y += Dp; }
-                } else {
-                    TS[h].x += s; ST[h].x += sT; SP[h].x += sp; SV[h].x += sv;
-                    if (LM) { TD[h].x += D; SDT[h].x += DT; SDP[h].x += Dp; }
-                }
-            }
-        }
-        // the compensated tile sums
-#pragma unroll
-        for (int h = 0; h < kJgQ / 2; ++h) {
-            kahan_add(S[h].x, C[h].x, TS[h].x);
-            kahan_add(S[h].y, C[h].y, TS[h].y);
-            if (LM) {
-                kahan_add(SD[h].x, CD[h].x, TD[h].x);
-                kahan_add(SD[h].y, CD[h].y, TD[h].y);
+                V[h][c] = __fadd2_rn(V[h][c], it[h]);
             }
         }
     }
-    {  // pedestals of the fast and far lines
-        float wA[4], wB[4], wC[4];
-        wA[0] = warp_sum(QA[0] - QAc);
-        wB[0] = warp_sum(QB[0] - QBc);
-        wC[0] = warp_sum(QC[0] - QCc);
+    // clamps (voigt.jl:276, line_mixing.jl:1368, cross_section_jacobian.jl:107-113, :312-319)
+    // and the segment's weights onto the layer channels
 #pragma unroll
-        for (int o = 1; o < 4; ++o) {
-            wA[o] = warp_sum(QA[o]);
-            wB[o] = warp_sum(QB[o]);
-            wC[o] = warp_sum(QC[o]);
+    for (int q = 0; q < kJgQ; ++q) {
+        float s[7];
+#pragma unroll
+        for (int c = 0; c < 7; ++c) s[c] = jg_used<LM, NS>(c) ? ((q & 1) ? V[q >> 1][c].y : V[q >> 1][c].x) : 0.f;
+        float v = s[0], vT = s[1], vp = s[2], vv = s[3];
+        if (!(v > 0.f)) v = vT = vp = vv = 0.f;
+        if (LM) {
+            v += s[4];
+            vT += s[5];
+            vp += s[6];
+            if (!(v > 0.f)) v = vT = vp = 0.f;
         }
-#pragma unroll
-        for (int h = 0; h < kJgQ / 2; ++h) {
-            const float i0 = pl0 + 64.f * h, i1 = i0 + 32.f;
-            kahan_add(S[h].x, C[h].x, fmaf(i0, fmaf(i0, wC[0], wB[0]), wA[0]));
-            kahan_add(S[h].y, C[h].y, fmaf(i1, fmaf(i1, wC[0], wB[0]), wA[0]));
-            ST[h].x += fmaf(i0, fmaf(i0, wC[1], wB[1]), wA[1]);
-            ST[h].y += fmaf(i1, fmaf(i1, wC[1], wB[1]), wA[1]);
-            SP[h].x += fmaf(i0, fmaf(i0, wC[2], wB[2]), wA[2]);
-            SP[h].y += fmaf(i1, fmaf(i1, wC[2], wB[2]), wA[2]);
-            SV[h].x += fmaf(i0, fmaf(i0, wC[3], wB[3]), wA[3]);
-            SV[h].y += fmaf(i1, fmaf(i1, wC[3], wB[3]), wA[3]);
+        if (prow) {  // relaxation-matrix line mixing: rows (perturbation, d/dT, d/dp) x column amount
+            v += (float)prow[32 * q];
+            vT += (float)prow[pstride + 32 * q];
+            if (NS >= 3) vp += (float)prow[2 * pstride + 32 * q];
+            if (!(v > 0.f)) v = vT = vp = 0.f;
         }
-    }
-    {  // node totals (4 lanes per node), then the interpolants at this lane's points
-        float v[7] = {fS, fT_, fP, fV, fD, fDT, fDP};
-#pragma unroll
-        for (int c = 0; c < 7; ++c) {
-            if (!LM && c >= 4) continue;
-            v[c] += __shfl_xor_sync(kFull, v[c], 8);
-            v[c] += __shfl_xor_sync(kFull, v[c], 16);
-            if (gfar) v[c] += gfar[c * kJgFarNodes + (lane & (kJgFarNodes - 1))];  // the strip far field
-        }
-        float it[7][kJgQ];
-#pragma unroll
-        for (int c = 0; c < 7; ++c)
-#pragma unroll
-            for (int q = 0; q < kJgQ; ++q) it[c][q] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < kJgFarNodes; ++kk) {
-            float w[kJgQ];
-#pragma unroll
-            for (int q = 0; q < kJgQ; ++q) w[q] = FT.L[kk][32 * q + lane];
-#pragma unroll
-            for (int c = 0; c < 7; ++c) {
-                if (!LM && c >= 4) continue;
-                const float n = __shfl_sync(kFull, v[c], kk);
-#pragma unroll
-                for (int q = 0; q < kJgQ; ++q) it[c][q] = fmaf(n, w[q], it[c][q]);
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < kJgQ / 2; ++h) {
-            kahan_add(S[h].x, C[h].x, it[0][2 * h]);
-            kahan_add(S[h].y, C[h].y, it[0][2 * h + 1]);
-            ST[h].x += it[1][2 * h]; ST[h].y += it[1][2 * h + 1];
-            SP[h].x += it[2][2 * h]; SP[h].y += it[2][2 * h + 1];
-            SV[h].x += it[3][2 * h]; SV[h].y += it[3][2 * h + 1];
-            if (LM) {
-                kahan_add(SD[h].x, CD[h].x, it[4][2 * h]);
-                kahan_add(SD[h].y, CD[h].y, it[4][2 * h + 1]);
-                SDT[h].x += it[5][2 * h]; SDT[h].y += it[5][2 * h + 1];
-                SDP[h].x += it[6][2 * h]; SDP[h].y += it[6][2 * h + 1];
-            }
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < kJgQ / 2; ++h) {
-        sum[0][2 * h] = S[h].x; sum[0][2 * h + 1] = S[h].y;
-        sum[1][2 * h] = ST[h].x; sum[1][2 * h + 1] = ST[h].y;
-        sum[2][2 * h] = SP[h].x; sum[2][2 * h + 1] = SP[h].y;
-        sum[3][2 * h] = SV[h].x; sum[3][2 * h + 1] = SV[h].y;
-        dsum[0][2 * h] = SD[h].x; dsum[0][2 * h + 1] = SD[h].y;
-        dsum[1][2 * h] = SDT[h].x; dsum[1][2 * h + 1] = SDT[h].y;
-        dsum[2][2 * h] = SDP[h].x; dsum[2][2 * h + 1] = SDP[h].y;
+        auto add = [&](const float w[4], int o) {
+            float a = w[0] * v + w[1] * vT;
+            if (NS >= 3) a += w[2] * vp;
+            if (NS >= 4) a += w[3] * vv;
+            acc[o * kJgWarpPts + 32 * q + lane] += a;
+        };
+        for (int o = 0; o < 3; ++o) add(W.base[o], o);
+        for (unsigned r = W.retr; r; r &= r - 1)  // warp-uniform
+            for (int o = 0; o < 2; ++o) add(W.pair[o], 3 + 2 * (__ffs(r) - 1) + o);
     }
 }
 
-// Segment weights: out[o] += W[o][0] s + W[o][1] s_T + W[o][2] s_p + W[o][3] s_v
-struct SegW {
-    float w[kJgMaxOut][4];
-};
-
-// dynamic shared memory of jg_linesum_kernel<*, NOUT>: the warps' tiles and their
-// per-point output accumulators
-constexpr size_t jg_smem_bytes(int nout) {
-    return sizeof(JgTile) * kJgWarps + sizeof(float) * kJgWarps * nout * kJgWarpPts + sizeof(JgFarTable);
+// dynamic shared memory of jg_linesum_kernel<LM, NS>: the warps' tiles, the leaf weights and
+// the warps' per-point output accumulators
+constexpr size_t jg_smem_bytes(bool lm, int n_out) {
+    return (lm ? sizeof(JgTile<true>) : sizeof(JgTile<false>)) * kJgWarps + sizeof(float) * kTrNodes * kTrLeaf +
+           sizeof(float) * kJgWarps * n_out * kJgWarpPts;
 }
 
-template <bool ANY_LM, int NOUT>
-__global__ void __launch_bounds__(kJgWarps * 32, 2) jg_linesum_kernel(
-    const SegDev* __restrict__ segs, const int* __restrict__ seg_n, const SegW* __restrict__ wts,
-    const int2* __restrict__ pl_segs, JgOut g, long long n_nu, float cut_g, float* __restrict__ out,
-    const double* __restrict__ pert, long long pstride, const float* __restrict__ sfar,
-    const int4* __restrict__ sranges, int n_strips) {
-    extern __shared__ float4 jg_sh[];
-    JgTile* tiles = (JgTile*)jg_sh;
-    JgFarTable& ftab = *(JgFarTable*)((float*)(tiles + kJgWarps) + (size_t)kJgWarps * NOUT * kJgWarpPts);
-    jg_far_table_init(ftab);
+// One warp per leaf, the segments of one kind (MODE); one launch per kind, the first stores
+// the layer channels and the others add to theirs.  A kernel holding every kind ran out of
+// instruction cache (warps in different kinds at a time: 6.5 of 9 stall cycles per
+// instruction were for instructions).
+// Bound by issue.  Measured on a B200, against two-level far fields (1024-point strips, then
+// each warp's 8 nodes from 320 points), four sums (seven) for every segment and the cores per
+// pair: 16 scenes of the 5,000-line list 1.53 + 7.50 -> 1.10 + 2.89 ms (far + near lines), one
+// IASI spectrum with VP_Y 9.78 + 91.9 -> 7.7 + 35.3 ms, two 645-1000 cm^-1 profiles of six
+// species 2.74 + 12.9 -> 2.5 + 8.5 ms.  K of three species against the FP64 oracle: 1.2e-6 ->
+// 1.6e-7 of its norm at 700 cm^-1, 9.3e-7 -> 8.2e-7 at 2200; single monochromatic entries
+// 1.7e-4 -> 2.7e-7 of the largest (the gradient of w in closed form).
+template <int MODE>
+__global__ void __launch_bounds__(kJgWarps * 32, MODE == kJg2 ? 3 : 2) jg_linesum_kernel(
+    const SegDev* __restrict__ segs, const SegW* __restrict__ wts, const int2* __restrict__ pl_segs, CellIndex ci,
+    JgOut g, long long n_nu, float cut_g, int n_out, int store, int far_sums, float* __restrict__ out,
+    const double* __restrict__ pert, long long pstride, const TreeTables* __restrict__ tab,
+    const float* __restrict__ far, const int4* __restrict__ ranges, int n_leaves, int pl0, int seg0) {
+    constexpr bool LM = MODE == kJgLm2 || MODE == kJgLm3;
+    constexpr int NS = MODE == kJg2 || MODE == kJgLm2 ? 2 : MODE == kJg4 ? 4 : 3;
+    extern __shared__ __align__(16) unsigned char jg_sh[];
+    JgTile<LM>* tiles = (JgTile<LM>*)jg_sh;
+    float(*Lw)[kTrLeaf] = (float(*)[kTrLeaf])(tiles + kJgWarps);
+    for (int i = threadIdx.x; i < kTrNodes * kTrLeaf; i += kJgWarps * 32) ((float*)Lw)[i] = ((const float*)tab->L)[i];
     __syncthreads();  // the only block-wide barrier: before any warp leaves
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* acc = (float*)(tiles + kJgWarps) + (size_t)warp * NOUT * kJgWarpPts;  // [NOUT][128], warp-private
-    const int pl = blockIdx.y;
-    const long long wb = (long long)blockIdx.x * kJgStrip + (long long)warp * kJgWarpPts;
+    float* acc = (float*)(Lw + kTrNodes) + (size_t)warp * n_out * kJgWarpPts;  // [n_out][128], warp-private
+    const int pl = pl0 + (int)blockIdx.y, leaf = (int)blockIdx.x * kJgWarps + warp;
+    const long long wb = (long long)leaf * kJgWarpPts;
     if (wb >= n_nu) return;
-    const float xn = (float)jg_far_node(lane & (kJgFarNodes - 1));
-    for (int o = 0; o < NOUT; ++o)
-#pragma unroll
-        for (int q = 0; q < kJgQ; ++q) acc[o * kJgWarpPts + 32 * q + lane] = 0.f;
+    for (int i = lane; i < n_out * kJgWarpPts; i += 32) acc[i] = 0.f;
+    unsigned touched = 0;  // layer channels with a contribution (warp-uniform)
     const int2 rng = pl_segs[pl];
     for (int si = rng.x; si < rng.x + rng.y; ++si) {
         const SegDev sg = segs[si];
-        float s[4][kJgQ], ds[3][kJgQ];
-        const long long nl = seg_n[si];
-        const bool lm = ANY_LM && (sg.flags & SEG_LM);
-        int4 sx = make_int4(0, 0, 0, 0);  // no strip far field: the whole window
+        if (jg_mode(sg.flags) != MODE) continue;
+        const int* row = ci.idx + (size_t)sg.list * ci.n;
+        const float m = (float)sg.margin_g;
+        const int wlo = cell_floor(ci, row, (float)wb - cut_g - m);
+        const int whi = cell_ceil(ci, row, (float)(wb + kJgWarpPts) + cut_g + m);
+        int4 own = make_int4(wlo, wlo, whi, whi);  // no far field: every line direct
         const float* gf = nullptr;
-        if (sfar) {
-            const size_t cell = (size_t)si * n_strips + blockIdx.x;
-            sx = sranges[cell];
-            gf = sfar + cell * kJgStripWords + (size_t)warp * kJgStripOut * kJgFarNodes;
+        if (far) {
+            const size_t cell = (size_t)(si - seg0) * n_leaves + leaf;
+            own = ranges[cell];
+            gf = far + cell * far_sums * kTrNodes;
         }
-        if (lm)
-            jg_segment<true>(sg, nl, g, wb, cut_g, lane, tiles[warp], ftab, xn, s, ds, sx, gf);
-        else
-            jg_segment<false>(sg, nl, g, wb, cut_g, lane, tiles[warp], ftab, xn, s, ds, sx, gf);
-        // clamps (voigt.jl:276, line_mixing.jl:1368, cross_section_jacobian.jl:107-113, :312-319)
-        const SegW& W = wts[si];
-        // relaxation-matrix line mixing: rows (perturbation, d/dT, d/dp) x column amount
         const double* prow = pert && (sg.flags & SEG_RELMAT) ? pert + (size_t)pl * 3 * pstride + wb + lane : nullptr;
-#pragma unroll
-        for (int q = 0; q < kJgQ; ++q) {
-            float v = s[0][q], vT = s[1][q], vp = s[2][q], vv = s[3][q];
-            if (!(v > 0.f)) v = vT = vp = vv = 0.f;
-            if (lm) {
-                v += ds[0][q];
-                vT += ds[1][q];
-                vp += ds[2][q];
-                if (!(v > 0.f)) v = vT = vp = 0.f;
-            }
-            if (prow) {
-                v += (float)prow[32 * q];
-                vT += (float)prow[pstride + 32 * q];
-                vp += (float)prow[2 * pstride + 32 * q];
-                if (!(v > 0.f)) v = vT = vp = 0.f;
-            }
-            for (int o = 0; o < NOUT; ++o)
-                acc[o * kJgWarpPts + 32 * q + lane] += W.w[o][0] * v + W.w[o][1] * vT + W.w[o][2] * vp + W.w[o][3] * vv;
-        }
+        const SegW& W = wts[si];
+        touched |= 7u;
+        for (unsigned r = W.retr; r; r &= r - 1) touched |= 3u << (3 + 2 * (__ffs(r) - 1));
+        jg_segment<LM, NS>(sg, g, wb, own, wlo, whi, cut_g, lane, tiles[warp], Lw, gf, W, prow, pstride, acc);
     }
-    float* base = out + (size_t)pl * NOUT * n_nu;
-    for (int o = 0; o < NOUT; ++o)
+    float* base = out + (size_t)pl * n_out * n_nu;
+    for (int o = 0; o < n_out; ++o) {
+        if (!store && !(touched >> o & 1u)) continue;
 #pragma unroll
         for (int q = 0; q < kJgQ; ++q) {
             const long long i = wb + 32 * q + lane;
-            if (i < n_nu) base[(size_t)o * n_nu + i] = acc[o * kJgWarpPts + 32 * q + lane];
+            const float v = acc[o * kJgWarpPts + 32 * q + lane];
+            if (i < n_nu) base[(size_t)o * n_nu + i] = store ? v : base[(size_t)o * n_nu + i] + v;
         }
+    }
 }
 
 // ------------------------------------------------------------------ RTE Jacobian
