@@ -16,6 +16,7 @@
 #include "lineparams.cuh"
 #include "linesum.cuh"
 #include "linesum_tree32.cuh"
+#include "linesum_tree64.cuh"
 #include "rte_ils.cuh"
 
 namespace irs {
@@ -974,45 +975,92 @@ struct JgProfile {     // per profile
     int n_state;
 };
 
-__device__ __forceinline__ double dB_dT64(double nu, double T) {  // planck.jl:67-71
-    const double x = 1.4387769 * nu / T, ex = exp(x);
-    return 1.191042953e-5 * 1.4387769 * (nu * nu * nu * nu) * ex / ((T * T) * (ex - 1.0) * (ex - 1.0));
+// 1/x: MUFU's 20-bit estimate and one third-order step (rcp64_fast), IEEE division outside
+// the range where it holds
+__device__ __forceinline__ double rcp64(double x) {
+    const double a = fabs(x);
+    return a > 1e-290 && a < 1e290 ? rcp64_fast(x) : 1.0 / x;
 }
-__device__ __forceinline__ double cim_corr_d(double s) {
-    if (s < 0.06) return 1.0 / 6.0;
-    const double w = exp(-s);
-    return 2.0 / (s * s) - 2.0 * w / ((w - 1.0) * (w - 1.0));
-}
-__device__ __forceinline__ double lit_corr_d(double s) {
-    if (s < 1e-4) return 0.5 - s * (2.0 / 3.0 - s * 0.375);
-    const double e = exp(-s);
-    return (e * (s + 1.0) - 1.0) / (s * s) + e;
+// exp(a) for the small arguments of the temperature differences (a^7/5040 < 1e-17)
+__device__ __forceinline__ double exp_small(double a) {
+    if (fabs(a) > 0.01) return exp(a);
+    return fma(a, fma(a, fma(a, fma(a, fma(a, fma(a, 1.0 / 720.0, 1.0 / 120.0), 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0), 1.0);
 }
 
-// continuum optical depth of one layer at (vh, vc, Tm), continuum.jl:183-250 and
-// the dz(Tm) of optical_depth.jl:123-130 (vmr_jacobian.jl:300-311)
-template <bool CIA>
-__device__ __forceinline__ double cont_tau(double nu, const LayerRT& r, double dp, const ContDev& c, double Cs,
-                                          double Cf, double te, double Se, double td, double vh, double vc,
-                                          double Tm, const CiaPoint& cp) {
-    const double p = r.p_mid;
-    const double dz = 8.314462 * Tm / (0.028964 * 9.80665) * dp / p * 100.0;
-    const double rho = (p / 1013.0) * (296.0 / Tm);
-    const double rad = radfn(nu, Tm);
-    double t = 0.0;
-    if (c.mask & 1) {
-        const double n = vh * p * 100.0 / (1.380649e-23 * Tm) * 1e-6;
-        const double ks = Cs * pow(296.0 / Tm, te) * vh * rho * rad * n;
-        const double kf = Cf * (1.0 - vh) * rho * rad * n;
-        t += (ks + kf) * dz;
+// Constants of one layer for jg_rte_kernel, formed once per (profile, layer): the MT-CKD
+// continua's column factor and exponents at T_mid and, as ratios, at T_mid +- 0.05 K (the
+// reference's central difference, vmr_jacobian.jl:322-344); c2/T and 1/T of the Planck terms.
+// Per (point, layer) the continua then take three exponentials for their value and all their
+// derivatives; evaluated from scratch at every perturbed argument (two pow, one exp and
+// several divisions each, eight times) they were most of the kernel.
+struct JgRteLayer {
+    double c2m, l296, l246, G, vh, vc;  // c2/T_mid, ln(296/T_mid), ln(T_mid/246), column factor, VMRs
+    double rp, rm, dp, dm;              // T/(T + h), T/(T - h) and their logs
+    double c2a, ia, c2t, it, c2b, ib;   // c2/T and 1/T at T_ave, T_top, T_bot
+    double frac, wM;
+};
+constexpr double kJgRteDT = 0.05;
+__global__ void __launch_bounds__(128) jg_rte_layers_kernel(const LayerRT* __restrict__ lrt, const JgLayer* __restrict__ jl,
+                                                            int n, JgRteLayer* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const LayerRT r = lrt[i];
+    const JgLayer y = jl[i];
+    JgRteLayer o;
+    const double T = r.T_mid, p = r.p_mid;
+    o.c2m = 1.4387769 / T;
+    o.l296 = log(296.0 / T);
+    o.l246 = log(T / 246.0);
+    const double rho = (p / 1013.0) * (296.0 / T), n1 = p * 100.0 / (1.380649e-23 * T) * 1e-6;
+    o.G = rho * n1 * (8.314462 * T / (0.028964 * 9.80665) * y.dp / p * 100.0);
+    o.vh = r.vmr_h2o;
+    o.vc = r.vmr_co2;
+    o.rp = T / (T + kJgRteDT);
+    o.rm = T / (T - kJgRteDT);
+    o.dp = -log1p(kJgRteDT / T);
+    o.dm = -log1p(-kJgRteDT / T);
+    o.c2a = 1.4387769 / r.T_ave;
+    o.ia = 1.0 / r.T_ave;
+    o.c2t = 1.4387769 / r.T_top;
+    o.it = 1.0 / r.T_top;
+    o.c2b = 1.4387769 / r.T_bot;
+    o.ib = 1.0 / r.T_bot;
+    o.frac = y.frac;
+    o.wM = y.wM;
+    out[i] = o;
+}
+
+// planck_radiance and dB/dT (planck.jl:22-24, :67-71) from one expm1 and one reciprocal:
+// B = c1 nu^3 / (e^x - 1), dB/dT = B (x/T) e^x / (e^x - 1), x = c2 nu / T
+__device__ __forceinline__ void planck_grad64(double c1nu3, double nu, double c2T, double iT, double& B, double& dB) {
+    const double x = nu * c2T, r = rcp64(expm1(x));
+    B = c1nu3 * r;
+    dB = B * (x * iT) * (1.0 + r);
+}
+// radfn (continuum.jl:169-174) with e = exp(-x)
+__device__ __forceinline__ double radfn_e(double nu, double x, double e) {
+    return x <= 0.01 ? 0.5 * x * nu : x <= 10.0 ? nu * (1.0 - e) * rcp64(1.0 + e) : nu;
+}
+// _cim_correction and its derivative (schwarzschild.jl:59-63, schwarzschild_jacobian.jl) with
+// w = exp(-s)
+__device__ __forceinline__ void cim_both(double s, double w, double& f, double& fp) {
+    f = s / 6.0;
+    fp = 1.0 / 6.0;
+    if (!(s < 0.06)) {
+        const double a = w - 1.0, r = rcp64(s * a), is = a * r, iw = s * r;  // 1/s, 1/(w - 1)
+        f = 1.0 - 2.0 * fma(w, iw, is);
+        fp = 2.0 * (is * is) - 2.0 * w * (iw * iw);
     }
-    if (c.mask & 2) {
-        const double n = vc * p * 100.0 / (1.380649e-23 * Tm) * 1e-6;
-        const double tc = td == 0.0 ? 1.0 : pow(Tm / 246.0, td);
-        t += Se * tc * (1e-20 * n * rho) * rad * dz;
+}
+// _lit_correction and its derivative
+__device__ __forceinline__ void lit_both(double s, double w, double& f, double& fp) {
+    f = s * (0.5 - s * (1.0 / 3.0 - s * 0.125));
+    fp = 0.5 - s * (2.0 / 3.0 - s * 0.375);
+    if (!(s < 1e-4)) {
+        const double is = rcp64(s);
+        f = (1.0 - w) * is - w;
+        fp = (w * (s + 1.0) - 1.0) * (is * is) + w;
     }
-    if (CIA) t += cia_tau(c, cp, nu, vh, vc, p, Tm, dz);
-    return t;
 }
 
 // One thread per (profile, grid point): the monochromatic Jacobian columns
@@ -1030,9 +1078,16 @@ __device__ __forceinline__ double cont_tau(double nu, const LayerRT& r, double d
 //      (warp shuffles, then FP64 shared-memory and global atomics) into xbar[profile][x]
 //      = sum_nu Ibar D[x] = (K^T dy)[x].  D is never stored.  Dynamic shared memory:
 //      n_state doubles.
+//
+// Bound by FP64 issue and latency (about 420 FP64 instructions a point and layer; the bytes,
+// 0.9 GB for 16 scenes, take 0.14 ms).  Six CTAs per SM (80 registers, a few spills) against
+// the four that 112 registers allow: 1.59 / 1.92 ms (16 scenes), 1.24 / 1.37 (adjoint);
+// five 1.71 / 1.45.  With JgRteLayer and one exponential per term, 16 scenes of the
+// 5,000-line list 3.69 -> 1.59 ms, one IASI profile 7.11 -> 2.42, the adjoint of two
+// 645-1000 cm^-1 profiles 1.13 + 4.38 -> 0.53 + 1.24.
 template <bool CIA = false, int MODE = 0>
-__global__ void __launch_bounds__(128) jg_rte_kernel(
-    const float* __restrict__ jl, int n_out, const LayerRT* __restrict__ lrt, const JgLayer* __restrict__ jlay,
+__global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
+    const float* __restrict__ jl, int n_out, const LayerRT* __restrict__ lrt, const JgRteLayer* __restrict__ jlay,
     const ProfileRT* __restrict__ prt, const JgProfile* __restrict__ jprof, const double* __restrict__ vlev,
     int L, const double* __restrict__ grid, long long n_nu, int src, ContDev cont, double* __restrict__ I,
     float* __restrict__ D, const double* __restrict__ Ibar = nullptr, double* __restrict__ xbar = nullptr) {
@@ -1048,11 +1103,11 @@ __global__ void __launch_bounds__(128) jg_rte_kernel(
         __syncthreads();
     }
     const double ib = MODE == 2 && valid ? Ibar[(size_t)p * n_nu + i] : 0.0;
-    const double nu = grid[i];
+    const double nu = grid[i], c1nu3 = 1.191042953e-5 * (nu * nu * nu);
     const ProfileRT pr = prt[p];
     const JgProfile jp = jprof[p];
     const LayerRT* lr = lrt + (size_t)p * L;
-    const JgLayer* jy = jlay + (size_t)p * L;
+    const JgRteLayer* jy = jlay + (size_t)p * L;
     const float* out = jl + (size_t)p * L * n_out * n_nu;
     const double* vl = vlev + (size_t)p * 4 * (L + 1);  // level VMR of the retrieved species
     double Cs = 0, Cf = 0, te = 0, Se = 0, td = 0;
@@ -1064,48 +1119,70 @@ __global__ void __launch_bounds__(128) jg_rte_kernel(
     }
     if (cont.mask & 2) {
         const Lerp l = lerp_at(cont.co2, cont.n_co2, nu);
-        Se = lerp_val(cont.co2 + cont.n_co2, l);
+        Se = 1e-20 * lerp_val(cont.co2 + cont.n_co2, l);
         td = lerp_val(cont.co2 + 2 * cont.n_co2, l);
     }
     CiaPoint cp;
     if (CIA) cia_prepare(cont.cia, cont.mask, nu, cp);
     const double invmu = 1.0 / pr.mu, eps = pr.eps;
-    auto layer_s = [&](int k) {
-        double t = (double)out[((size_t)k * n_out) * n_nu + i];
-        if (cont.mask) t += cont_tau<CIA>(nu, lr[k], jy[k].dp, cont, Cs, Cf, te, Se, td, lr[k].vmr_h2o, lr[k].vmr_co2, lr[k].T_mid, cp);
-        return t * invmu;
+    // MT-CKD continua of layer k, continuum.jl:183-250 (with the dz(T) of
+    // optical_depth.jl:123-130 inside G): tau = G rad [vh (Cs E vh + Cf (1 - vh)) + Se Q vc]
+    struct Cont {
+        double x, e, E, Q;  // c2 nu / T, exp(-x), (296/T)^te, (T/246)^td
     };
-    auto emission_down = [&](int k, double s, double& em, double& dem) {  // schwarzschild_jacobian.jl:221-243
-        const double w = exp(-s), u = 1.0 - w;
-        if (src == 0) {
-            const double Ba = planck64(nu, lr[k].T_ave), Bb = planck64(nu, lr[k].T_bot);
-            const double f = cim_corr(s), fp = cim_corr_d(s), core = Ba + (Bb - Ba) * f;
-            em = u * core;
-            dem = w * core + u * (Bb - Ba) * fp;
-        } else {
-            const double Bb = planck64(nu, lr[k].T_bot), Bt = planck64(nu, lr[k].T_top);
-            const double fl = lit_corr(s), flp = lit_corr_d(s);
-            em = Bb * u + (Bt - Bb) * fl;
-            dem = Bb * w + (Bt - Bb) * flp;
-        }
+    const bool mt = (cont.mask & 3) != 0;
+    auto cont_at = [&](const JgRteLayer& r) {
+        Cont c{0.0, 0.0, 0.0, 1.0};
+        c.x = nu * r.c2m;
+        c.e = exp(-c.x);
+        if (cont.mask & 1) c.E = exp(te * r.l296);
+        if ((cont.mask & 2) && td != 0.0) c.Q = exp(td * r.l246);
+        return c;
+    };
+    auto cont_sum = [&](const JgRteLayer& r, double E, double Q) {
+        return fma(r.vh, fma(Cs * E, r.vh, Cf * (1.0 - r.vh)), Se * Q * r.vc);
+    };
+    auto cia_at = [&](const LayerRT& r, const JgRteLayer& y, double vh, double vc, double T) {
+        // y.G = rho n1 dz(T_mid): dz(T) = dz(T_mid) T / T_mid
+        const double rho = (r.p_mid / 1013.0) * (296.0 / r.T_mid), n1 = r.p_mid * 100.0 / (1.380649e-23 * r.T_mid) * 1e-6;
+        return cia_tau(cont, cp, nu, vh, vc, r.p_mid, T, y.G / (rho * n1) * (T / r.T_mid));
+    };
+    auto layer_s = [&](int k, const JgRteLayer& r, const Cont& c) {
+        double t = (double)out[((size_t)k * n_out) * n_nu + i];
+        if (mt) t = fma(r.G * radfn_e(nu, c.x, c.e), cont_sum(r, c.E, c.Q), t);
+        if (CIA) t += cia_at(lr[k], r, r.vh, r.vc, lr[k].T_mid);
+        return t * invmu;
     };
     // pass 1: total optical depth and the downwelling radiance at the surface
     double OD = 0.0, Id = 0.0, gk = 1.0;
     for (int k = 0; k < L; ++k) {
-        const double s = layer_s(k);
+        const JgRteLayer& r = jy[k];
+        Cont c{};
+        if (mt) c = cont_at(r);
+        const double s = layer_s(k, r, c);
         OD += s;
-        if (eps < 1.0) {
-            double em, dem;
-            emission_down(k, s, em, dem);
-            Id += gk * em;
-            gk *= exp(-s);
+        if (eps < 1.0) {  // schwarzschild_jacobian.jl:221-243
+            const double w = exp(-s), u = 1.0 - w;
+            double Ba, Bb, f, fp, d;
+            planck_grad64(c1nu3, nu, r.c2b, r.ib, Bb, d);
+            if (src == 0) {
+                planck_grad64(c1nu3, nu, r.c2a, r.ia, Ba, d);
+                cim_both(s, w, f, fp);
+                Id += gk * (u * fma(Bb - Ba, f, Ba));
+            } else {
+                planck_grad64(c1nu3, nu, r.c2t, r.it, Ba, d);
+                lit_both(s, w, f, fp);
+                Id += gk * fma(Ba - Bb, f, Bb * u);
+            }
+            gk *= w;
         }
     }
     const double Tr0 = exp(-OD), refl = 1.0 - eps;
-    const double Bs = planck64(nu, pr.T_sfc);
+    double Bs, dBs;
+    planck_grad64(c1nu3, nu, 1.4387769 / pr.T_sfc, 1.0 / pr.T_sfc, Bs, dBs);
     double Iv = eps * Bs * Tr0, Ib = eps * Bs * Tr0;
     const double dIde = Bs * Tr0 - (eps < 1.0 ? Id * Tr0 : 0.0);
-    const double dIdTs = eps * dB_dT64(nu, pr.T_sfc) * Tr0;
+    const double dIdTs = eps * dBs * Tr0;
     // pass 2, surface to top
     const int nT = jp.include_T ? L + 1 : 0;
     double cum = 0.0, gdn = 1.0, Id_below = 0.0;
@@ -1123,80 +1200,110 @@ __global__ void __launch_bounds__(128) jg_rte_kernel(
         }
     };
     constexpr bool DERIV = MODE != 1;
+    double Bb, dBb;  // at the layer's bottom level: the top of the layer below
+    planck_grad64(c1nu3, nu, jy[0].c2b, jy[0].ib, Bb, dBb);
     for (int m = 0; m < L; ++m) {
-        const LayerRT r = lr[m];
-        const JgLayer jm = jy[m];
-        const double s = layer_s(m);
+        const JgRteLayer& r = jy[m];
+        Cont c{};
+        if (mt) c = cont_at(r);
+        const double s = layer_s(m, r, c);
         cum += s;
         const double Tt = exp(-(OD - cum));  // transmittance from the top of layer m to space
         const double w = exp(-s), u = 1.0 - w;
-        double e, dea, dTl_lo, dTl_hi;
+        double e, dea, dTl_lo, dTl_hi, Ba = 0.0, dBa = 0.0, Bt, dBt, f, fp;
+        planck_grad64(c1nu3, nu, r.c2t, r.it, Bt, dBt);
         if (src == 0) {
-            const double Ba = planck64(nu, r.T_ave), Bt = planck64(nu, r.T_top);
-            const double f = cim_corr(s), fp = cim_corr_d(s), core = Ba + (Bt - Ba) * f;
+            planck_grad64(c1nu3, nu, r.c2a, r.ia, Ba, dBa);
+            cim_both(s, w, f, fp);
+            const double core = Ba + (Bt - Ba) * f;
             e = u * core;
             dea = w * core + u * (Bt - Ba) * fp;
-            const double cavg = Tt * u * (1.0 - f) * dB_dT64(nu, r.T_ave);
-            dTl_lo = cavg * (1.0 - jm.frac);
-            dTl_hi = cavg * jm.frac + Tt * u * f * dB_dT64(nu, r.T_top);
+            const double cavg = Tt * u * (1.0 - f) * dBa;
+            dTl_lo = cavg * (1.0 - r.frac);
+            dTl_hi = cavg * r.frac + Tt * u * f * dBt;
         } else {
-            const double Bb = planck64(nu, r.T_bot), Bt = planck64(nu, r.T_top);
-            const double fl = lit_corr(s), flp = lit_corr_d(s);
-            e = Bt * u + (Bb - Bt) * fl;
-            dea = Bt * w + (Bb - Bt) * flp;
-            dTl_lo = Tt * fl * dB_dT64(nu, r.T_bot);
-            dTl_hi = Tt * (u - fl) * dB_dT64(nu, r.T_top);
+            lit_both(s, w, f, fp);
+            e = Bt * u + (Bb - Bt) * f;
+            dea = Bt * w + (Bb - Bt) * fp;
+            dTl_lo = Tt * f * dBb;
+            dTl_hi = Tt * (u - f) * dBt;
         }
         double dIdtau = invmu * (-Ib + Tt * dea);
         if (eps < 1.0) {  // reflected downwelling, schwarzschild_jacobian.jl:210-264
             double em, dem;
-            emission_down(m, s, em, dem);
+            if (src == 0) {
+                const double core = Ba + (Bb - Ba) * f;
+                em = u * core;
+                dem = w * core + u * (Bb - Ba) * fp;
+            } else {
+                em = Bb * u + (Bt - Bb) * f;
+                dem = Bb * w + (Bt - Bb) * fp;
+            }
             const double above = Id - Id_below - gdn * em;  // emitted above layer m
             dIdtau += refl * invmu * Tr0 * (-above + gdn * dem - Id);
+            const double rg = refl * Tr0 * gdn;
             if (src == 0) {
-                const double f = cim_corr(s);
-                const double cavg = refl * Tr0 * gdn * u * (1.0 - f) * dB_dT64(nu, r.T_ave);
-                dTl_lo += cavg * (1.0 - jm.frac) + refl * Tr0 * gdn * u * f * dB_dT64(nu, r.T_bot);
-                dTl_hi += cavg * jm.frac;
+                const double cavg = rg * u * (1.0 - f) * dBa;
+                dTl_lo += cavg * (1.0 - r.frac) + rg * u * f * dBb;
+                dTl_hi += cavg * r.frac;
             } else {
-                const double fl = lit_corr(s);
-                dTl_lo += refl * Tr0 * gdn * (u - fl) * dB_dT64(nu, r.T_bot);
-                dTl_hi += refl * Tr0 * gdn * fl * dB_dT64(nu, r.T_top);
+                dTl_lo += rg * (u - f) * dBb;
+                dTl_hi += rg * f * dBt;
             }
             Id_below += gdn * em;
             gdn *= w;
         }
         Iv += Tt * e;
         Ib += Tt * e;
-        // continuum derivatives by central differences (vmr_jacobian.jl:322-344)
+        Bb = Bt;
+        dBb = dBt;
+        // continuum derivatives: d/dT by the reference's central difference
+        // (vmr_jacobian.jl:322-344), the VMR ones of the quadratic in closed form, which its
+        // central differences give
         const float* om = out + (size_t)m * n_out * nn;
         double cT = 0.0, cvh = 0.0, cvc = 0.0;
-        if (DERIV && cont.mask) {
-            const double vh = r.vmr_h2o, vc = r.vmr_co2, Tm = r.T_mid;
+        if (DERIV && mt) {
+            const double Gr = r.G * radfn_e(nu, c.x, c.e);
+            if (jp.include_T) {
+                const double xp = c.x * r.rp, xm = c.x * r.rm;  // -x(T +- h) = -x + x - x r
+                const double ep = c.e * exp_small(c.x - xp), em = c.e * exp_small(c.x - xm);
+                const double Ep = (cont.mask & 1) ? c.E * exp_small(te * r.dp) : 0.0;
+                const double Em = (cont.mask & 1) ? c.E * exp_small(te * r.dm) : 0.0;
+                double Qp = c.Q, Qm = c.Q;
+                if ((cont.mask & 2) && td != 0.0) {
+                    Qp *= exp_small(-td * r.dp);
+                    Qm *= exp_small(-td * r.dm);
+                }
+                cT = (r.G * r.rp * radfn_e(nu, xp, ep) * cont_sum(r, Ep, Qp) -
+                      r.G * r.rm * radfn_e(nu, xm, em) * cont_sum(r, Em, Qm)) * (1.0 / (2 * kJgRteDT));
+            }
+            cvh = Gr * (2.0 * r.vh * (Cs * c.E) + Cf * (1.0 - 2.0 * r.vh));
+            cvc = Gr * (Se * c.Q);
+        }
+        if (DERIV && CIA) {
+            const LayerRT lm = lr[m];
+            const double vh = r.vh, vc = r.vc, Tm = lm.T_mid;
             if (jp.include_T)
-                cT = (cont_tau<CIA>(nu, r, jm.dp, cont, Cs, Cf, te, Se, td, vh, vc, Tm + 0.05, cp) -
-                      cont_tau<CIA>(nu, r, jm.dp, cont, Cs, Cf, te, Se, td, vh, vc, Tm - 0.05, cp)) / 0.1;
+                cT += (cia_at(lm, r, vh, vc, Tm + kJgRteDT) - cia_at(lm, r, vh, vc, Tm - kJgRteDT)) / (2 * kJgRteDT);
             if (jp.retr_h2o >= 0) {
                 const double h = fmax(fabs(vh), 1e-30) * 1e-6;
-                cvh = (cont_tau<CIA>(nu, r, jm.dp, cont, Cs, Cf, te, Se, td, vh + h, vc, Tm, cp) -
-                       cont_tau<CIA>(nu, r, jm.dp, cont, Cs, Cf, te, Se, td, vh - h, vc, Tm, cp)) / (2 * h);
+                cvh += (cia_at(lm, r, vh + h, vc, Tm) - cia_at(lm, r, vh - h, vc, Tm)) / (2 * h);
             }
             if (jp.retr_co2 >= 0) {
                 const double h = fmax(fabs(vc), 1e-30) * 1e-6;
-                cvc = (cont_tau<CIA>(nu, r, jm.dp, cont, Cs, Cf, te, Se, td, vh, vc + h, Tm, cp) -
-                       cont_tau<CIA>(nu, r, jm.dp, cont, Cs, Cf, te, Se, td, vh, vc - h, Tm, cp)) / (2 * h);
+                cvc += (cia_at(lm, r, vh, vc + h, Tm) - cia_at(lm, r, vh, vc - h, Tm)) / (2 * h);
             }
         }
         if (DERIV && jp.include_T) {
-            const double tlo = (double)om[1 * nn + i] + cT * (1.0 - jm.wM);
-            const double thi = (double)om[2 * nn + i] + cT * jm.wM;
+            const double tlo = (double)om[1 * nn + i] + cT * (1.0 - r.wM);
+            const double thi = (double)om[2 * nn + i] + cT * r.wM;
             emit((size_t)m, carryT + dTl_lo + dIdtau * tlo);
             carryT = dTl_hi + dIdtau * thi;
         }
         for (int rr = 0; DERIV && rr < jp.n_retr; ++rr) {
             const double cv = rr == jp.retr_h2o ? cvh : (rr == jp.retr_co2 ? cvc : 0.0);
-            const double vlo = (double)om[(size_t)(3 + 2 * rr) * nn + i] + cv * (1.0 - jm.wM);
-            const double vhi = (double)om[(size_t)(4 + 2 * rr) * nn + i] + cv * jm.wM;
+            const double vlo = (double)om[(size_t)(3 + 2 * rr) * nn + i] + cv * (1.0 - r.wM);
+            const double vhi = (double)om[(size_t)(4 + 2 * rr) * nn + i] + cv * r.wM;
             const double sc = jp.log_vmr ? vl[rr * (L + 1) + m] : 1.0;
             emit((size_t)(nT + rr * (L + 1) + m), sc * (carryV[rr] + dIdtau * vlo));
             carryV[rr] = dIdtau * vhi;
@@ -1205,7 +1312,7 @@ __global__ void __launch_bounds__(128) jg_rte_kernel(
     if (DERIV && jp.include_T) emit((size_t)L, carryT);
     for (int rr = 0; DERIV && rr < jp.n_retr; ++rr) {
         const double sc = jp.log_vmr ? vl[rr * (L + 1) + L] : 1.0;
-        if (DERIV) emit((size_t)(nT + rr * (L + 1) + L), sc * carryV[rr]);
+        emit((size_t)(nT + rr * (L + 1) + L), sc * carryV[rr]);
     }
     int col = nT + jp.n_retr * (L + 1);
     if (DERIV && jp.include_tsfc) emit((size_t)(col++), dIdTs);

@@ -87,3 +87,16 @@ def test_node_buffer_groups(pkg, monkeypatch):
         c.close()
     assert np.array_equal(K[0], K[1])
     assert np.all(np.abs(K[2] - K[0]) <= 1e-5 * np.max(np.abs(K[0]), axis=0))
+
+
+@pytest.mark.parametrize("lo", [20.0, 700.0, 2300.0])  # radfn's three branches (c2 nu/T below 0.01 .. above 10)
+@pytest.mark.parametrize("source_function,eps", [("cim", 1.0), ("cim", 0.9), ("toon", 1.0), ("toon", 0.9)])
+def test_radiative_transfer_terms(pkg, ctx, oracle, orc_mod, lo, source_function, eps):
+    """The continua's and the source functions' derivatives (both sources, reflecting surface)
+    with thin and thick layers, at wavenumbers where each branch of the terms is taken."""
+    prof = atm(pkg, 7)
+    ll = {s: pkg.synthetic.synthetic_linelist(30, s, 80 + s, max(lo - 8.0, 1.0), lo + 16.0).lines for s in (1, 2)}
+    spec = pkg.StateVectorSpec(len(prof.pressure), [1, 2])
+    check_vs_oracle(pkg, ctx, oracle, orc_mod, prof, ll, spec, snd(300, lo, 0.02),
+                    dict(apply_continuum=True, continua=("h2o", "co2"), with_ils=False, high_res_factor=1,
+                         source_function=source_function), eps=eps)
