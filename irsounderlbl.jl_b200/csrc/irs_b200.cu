@@ -13,6 +13,7 @@
 #include "lineparams.cuh"
 #include "linesum.cuh"
 #include "linesum_tree64.cuh"
+#include "linesum_mixed_tree.cuh"
 #include "rte_ils.cuh"
 #include "jacobian.cuh"
 #include "oe.cuh"
@@ -183,19 +184,28 @@ static double u_granularity(int64_t n_nu, double cut_g) {
     return g;
 }
 
-// Cell index (linesum_tree32.cuh) of rows of sorted keys V[off[r] .. + n[r]) over the grid
-// and `reach` (cutoff and margin) beyond each end: cells of 32 points, wider where the grid
-// and its margins would take more than a million.
-static CellIndex cell_index(irs_ctx* ctx, const double* d_V, const std::vector<long long>& off, const std::vector<int>& n,
-                            int64_t n_nu, double reach) {
-    const double span = (double)((n_nu + kTrStrip - 1) / kTrStrip * kTrStrip) + 2.0 * reach;
-    double cell = 32.0;
+static int64_t tree_leaves(int64_t n_nu) { return (n_nu + kTrStrip - 1) / kTrStrip * kTrLeaves; }
+
+// Layout of a cell index (linesum_tree32.cuh) over the grid and `reach` (cutoff and margin)
+// beyond each end: cells of 32 points, wider where the grid and its margins would take more
+// than a million.
+static CellIndex cell_layout(int64_t n_nu, double reach, double& cell, double& off) {
+    const double span = (double)tree_leaves(n_nu) * kTrLeaf + 2.0 * reach;
+    cell = 32.0;
     while (span / cell > 1048576.0) cell *= 2.0;
     CellIndex ci;
-    const double o = std::ceil(reach / cell + 1.0) * cell;
-    ci.n = (int)((span + 2.0 * (o - reach)) / cell) + 3;
+    off = std::ceil(reach / cell + 1.0) * cell;
+    ci.n = (int)((span + 2.0 * (off - reach)) / cell) + 3;
     ci.inv_cell = (float)(1.0 / cell);
-    ci.off = (float)o;
+    ci.off = (float)off;
+    ci.idx = nullptr;
+    return ci;
+}
+// The index of rows of sorted keys V[off[r] .. + n[r])
+static CellIndex cell_index(irs_ctx* ctx, const double* d_V, const std::vector<long long>& off, const std::vector<int>& n,
+                            int64_t n_nu, double reach) {
+    double cell, o;
+    CellIndex ci = cell_layout(n_nu, reach, cell, o);
     int* d_idx = (int*)workspace(ctx, "cell_idx", off.size() * (size_t)ci.n * sizeof(int));
     const long long* d_off = upload(ctx, "cell_off", off);
     const int* d_n = upload(ctx, "cell_n", n);
@@ -288,6 +298,84 @@ static void tree64_launch(irs_ctx* ctx, const Plan& pl, const std::vector<int>& 
     }
 }
 
+// bytes of one (segment, leaf) cell of the FP32 forward far field
+static size_t fw_cell_bytes(bool lm) { return fw_sums(lm) * kTrNodes * sizeof(float) + sizeof(int4); }
+
+// The FP32 line sum of IRS_MIXED (linesum_mixed_tree.cuh): the cell index of the kept lines,
+// the far field's node values and the leaf kernels, in groups of profile-layers (their
+// segments are contiguous) whose node values fit ctx->strip_buf_max (one profile-layer beyond
+// it runs without the far field, every line direct).
+static void mixed_tree_launch(irs_ctx* ctx, const Plan& pl, const std::vector<int>& first, const SegDev* d_segs,
+                              const int* d_count, const unsigned* d_reach, const int2* d_pl, const LpOutMixed& om,
+                              int64_t n_nu, float cut_g, const irs_fm_options& o, float* d_tau, double* d_pert,
+                              long long pstride, unsigned long long* d_eval) {
+    cudaStream_t st = ctx->stream;
+    const int npl = pl.n_prof * pl.L, nseg = first[npl];
+    double margin = 0.0;
+    int any[2] = {0, 0};  // segments without and with per-line mixing
+    for (auto& g : pl.segs) {
+        margin = std::max(margin, g.margin_g);
+        any[(g.flags & SEG_LM) ? 1 : 0] = 1;
+    }
+    const bool lm = any[1] != 0;
+    double off, cell;
+    CellIndex ci = cell_layout(n_nu, cut_g + margin, cell, off);
+    int* d_idx = (int*)workspace(ctx, "fw_cell_idx", (size_t)nseg * ci.n * sizeof(int));
+    ci.idx = d_idx;
+    cell_fill_kernel<<<dim3((unsigned)(pl.max_list / 256 + 1), nseg), 256, 0, st>>>(d_segs, d_count, om.V, ci.n, 1.0 / cell,
+                                                                                   off, d_idx);
+    check_launch(ctx);
+    const TreeTables* d_tab = tree_tables(ctx);
+    const int n_leaves = (int)tree_leaves(n_nu);
+    const size_t cell_bytes = fw_cell_bytes(lm);
+    const size_t max_cells = std::min((size_t)nseg * n_leaves, ctx->strip_buf_max / cell_bytes);
+    char* buf = (char*)workspace(ctx, "fw_far", max_cells * cell_bytes);
+    // one warp or eight per (strip, segment): by the strips of one profile's segments (not the
+    // batch's, so that a profile's result does not depend on it).  From 16 warps per SM on, one
+    // warp is the cheaper; 9 strips x 49 segments would leave it three warps per SM, where
+    // eight take 67 us
+    int n_lists = 0;
+    for (auto& l : ctx->lists) n_lists += l.n > 0 ? 1 : 0;
+    const bool warp_tree = (int64_t)(n_leaves / kTrLeaves) * pl.L * n_lists >= 148 * 16;
+    for (int pa = 0; pa < npl;) {
+        int pb = pa;
+        const int s_a = first[pa];
+        while (pb < npl && (size_t)(first[pb + 1] - s_a) * n_leaves <= max_cells) ++pb;
+        if (pb == pa) pb = pa + 1;
+        const int ns = first[pb] - s_a;
+        const size_t cells = (size_t)ns * n_leaves;
+        float* far = nullptr;
+        int4* rng = nullptr;
+        if (cells <= max_cells && ns > 0) {
+            rng = (int4*)buf;
+            far = (float*)(buf + cells * sizeof(int4));
+            const dim3 gt(n_leaves / kTrLeaves, ns), gw((gt.x + kFwTreeWarps - 1) / kFwTreeWarps, ns);
+            if (warp_tree) {
+                if (lm) fw_tree_warp_kernel<true><<<gw, 32 * kFwTreeWarps, 0, st>>>(d_segs, d_reach, ci, om, cut_g, n_nu, n_leaves, d_tab, far, rng, s_a, d_eval);
+                else fw_tree_warp_kernel<false><<<gw, 32 * kFwTreeWarps, 0, st>>>(d_segs, d_reach, ci, om, cut_g, n_nu, n_leaves, d_tab, far, rng, s_a, d_eval);
+            } else if (lm) fw_tree_kernel<true><<<gt, 32 * kFwWarps, 0, st>>>(d_segs, d_reach, ci, om, cut_g, n_nu, n_leaves, d_tab, far, rng, s_a, d_eval);
+            else fw_tree_kernel<false><<<gt, 32 * kFwWarps, 0, st>>>(d_segs, d_reach, ci, om, cut_g, n_nu, n_leaves, d_tab, far, rng, s_a, d_eval);
+            check_launch(ctx);
+        }
+        const dim3 gl((unsigned)((n_nu + kFwWarps * kTrLeaf - 1) / (kFwWarps * kTrLeaf)), pb - pa);
+        int store = 1;
+#define IRS_FW(M, LMX)                                                                                                 \
+    do {                                                                                                               \
+        fw_leaf_kernel<M, LMX><<<gl, 32 * kFwWarps, 0, st>>>(d_segs, d_pl, ci, om, n_nu, cut_g, (float)o.x_far, store, \
+                                                             fw_sums(lm), d_tau, d_pert, pstride, d_tab, far, rng, n_leaves, pa, s_a, d_eval); \
+        check_launch(ctx);                                                                                             \
+        store = 0;                                                                                                     \
+    } while (0)
+        if (any[0] || !lm) {
+            if (o.method == IRS_WEIDEMAN) IRS_FW(1, false);
+            else IRS_FW(3, false);
+        }
+        if (lm) IRS_FW(3, true);
+#undef IRS_FW
+        pa = pb;
+    }
+}
+
 // Runs the line-parameter passes and the line sum for the plan; returns the
 // device tau buffer ([n_prof * L][n_nu], FP32 for mixed or FP64 for plain).
 static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n_nu, double grid0,
@@ -351,12 +439,13 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
         lp_write_kernel<0><<<g1, kLpThreads, 0, st>>>(d_segs, d_lists, tp, cfg, d_keep, d_chunk, n_chunks,
                                                       d_count, o64, om, d_pairs, d_reach);
     if (mixed) {
-        char* base = (char*)workspace(ctx, "lpmx", S * (8 + 8 + 16 + 16 + 16));
-        om.V = (double*)base;
-        om.U = (float2*)(base + S * 8);
-        om.p0 = (float4*)(base + S * 16);
-        om.p1 = (float4*)(base + S * 32);
-        om.p2 = (float4*)(base + S * 48);
+        char* base = (char*)workspace(ctx, "lpmx", S * kLpMixedBytes);
+        om.p0 = (float4*)base;
+        om.p1 = om.p0 + S;
+        om.V = (double*)(base + S * 32);
+        om.U = (float2*)(base + S * 40);
+        om.p2 = (float2*)(base + S * 48);
+        om.df = (float*)(base + S * 56);
         lp_write_kernel<1><<<g1, kLpThreads, 0, st>>>(d_segs, d_lists, tp, cfg, d_keep, d_chunk, n_chunks,
                                                       d_count, o64, om, d_pairs, d_reach);
     }
@@ -380,62 +469,25 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
                 linesum_f64_kernel<3><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride, du);
         }
     } else {
-        dim3 g2((unsigned)((n_nu + kMxStrip - 1) / kMxStrip), npl);
         const float cut_g = (float)(o.cutoff / dnu_g);
         unsigned long long* d_eval = d_pairs + 2;
-        const bool far = o.precision == IRS_MIXED;
-        const bool anylm = o.line_mixing == IRS_LM_PER_LINE_Y;
-        // strip far field (pre-pass): 528 bytes per (segment, strip) in a buffer of at most
-        // ctx->strip_buf_max; larger batches run in groups of profile-layers (their segments
-        // are contiguous) whose cells fit it
-        const int n_strips = (int)g2.x;
-        const size_t cell_bytes = kStripWords * sizeof(float) + sizeof(int4);
-        const bool strip = far && o.method == 3;
-        float* d_M = nullptr;
-        char* d_sbuf = nullptr;
-        size_t max_cells = 0;
-        if (strip) {
-            max_cells = std::min((size_t)nseg * n_strips, ctx->strip_buf_max / cell_bytes);
-            d_sbuf = (char*)workspace(ctx, "strip_far", max_cells * cell_bytes);
-            constexpr int nM = kMxWarps * kFarNodes * kCtaNodes;
-            d_M = (float*)workspace(ctx, "strip_M", nM * sizeof(float));
-            strip_table_kernel<<<(nM + 255) / 256, 256, 0, st>>>(d_M);
-            check_launch(ctx);
-        }
-        for (int pa = 0; pa < npl;) {
-            // this launch: profile-layers [pa, pb) and their segments [s_a, first[pb])
-            int pb = npl;
-            const int s_a = first[pa];
-            float* d_sfar = nullptr;
-            int4* d_srng = nullptr;
-            if (strip) {
-                pb = pa;
-                while (pb < npl && (size_t)(first[pb + 1] - s_a) * n_strips <= max_cells) ++pb;
-                if (pb == pa) pb = pa + 1;  // one profile-layer beyond the buffer: no strip far field
-                const size_t cells = (size_t)(first[pb] - s_a) * n_strips;
-                if (cells <= max_cells) {
-                    d_sfar = (float*)d_sbuf;
-                    d_srng = (int4*)(d_sbuf + cells * kStripWords * sizeof(float));
-                    dim3 g3(n_strips, pb - pa);
-                    if (anylm) strip_far_kernel<true><<<g3, kStripThreads, 0, st>>>(d_segs, d_count, d_reach, d_pl, om, cut_g, n_strips, d_M, d_sfar, d_srng, d_eval, pa, s_a);
-                    else strip_far_kernel<false><<<g3, kStripThreads, 0, st>>>(d_segs, d_count, d_reach, d_pl, om, cut_g, n_strips, d_M, d_sfar, d_srng, d_eval, pa, s_a);
-                    check_launch(ctx);
-                }
-            }
-            const dim3 g2c(g2.x, pb - pa);
-#define IRS_MX(M, LMX, F, P) do { \
-        IRS_CUDA(cudaFuncSetAttribute(linesum_mixed_kernel<M, LMX, F, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMxSmem)); \
-        linesum_mixed_kernel<M, LMX, F, P><<<g2c, kMxThreads, kMxSmem, st>>>(d_segs, d_count, d_pl, om, n_nu, cut_g, (float*)d_tau, d_eval, d_pert, pstride, d_sfar, d_srng, n_strips, pa, s_a); \
+        const bool lm = o.line_mixing == IRS_LM_PER_LINE_Y;
+        if (o.precision == IRS_MIXED && o.method != IRS_PSEUDOVOIGT) {
+            mixed_tree_launch(ctx, pl, first, d_segs, d_count, d_reach, d_pl, om, n_nu, cut_g, o, (float*)d_tau, d_pert,
+                              pstride, d_eval);
+        } else {
+            dim3 g2((unsigned)((n_nu + kMxStrip - 1) / kMxStrip), npl);
+#define IRS_MX(M, LMX, P) do { \
+        IRS_CUDA(cudaFuncSetAttribute(linesum_mixed_kernel<M, LMX, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMxSmem)); \
+        linesum_mixed_kernel<M, LMX, P><<<g2, kMxThreads, kMxSmem, st>>>(d_segs, d_count, d_pl, om, n_nu, cut_g, (float*)d_tau, d_eval, d_pert, pstride); \
     } while (0)
-            if (o.method == 1) { if (far) IRS_MX(1, false, true, false); else IRS_MX(1, false, false, false); }
-            else if (o.method == 2) IRS_MX(2, false, false, false);
-            else if (o.line_mixing == IRS_LM_PER_LINE_Y) { if (far) IRS_MX(3, true, true, false); else IRS_MX(3, true, false, false); }
-            else if (d_pert) { if (far) IRS_MX(3, false, true, true); else IRS_MX(3, false, false, true); }
-            else { if (far) IRS_MX(3, false, true, false); else IRS_MX(3, false, false, false); }
-            check_launch(ctx);
-            pa = pb;
-        }
+            if (o.method == 1) IRS_MX(1, false, false);
+            else if (o.method == 2) IRS_MX(2, false, false);
+            else if (lm) IRS_MX(3, true, false);
+            else if (d_pert) IRS_MX(3, false, true);
+            else IRS_MX(3, false, false);
 #undef IRS_MX
+        }
     }
     check_launch(ctx);
     return d_tau;
@@ -655,16 +707,17 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
         workspace(ctx, "I", (size_t)n_prof * n_nu * sizeof(double));
         workspace(ctx, "grid", n_nu * sizeof(double));
         if (slots > 0) {
-            workspace(ctx, mixed ? "lpmx" : "lp64", (size_t)slots * (mixed ? 64 : kLpF64 * sizeof(double)));
+            workspace(ctx, mixed ? "lpmx" : "lp64", (size_t)slots * (mixed ? kLpMixedBytes : kLpF64 * sizeof(double)));
             workspace(ctx, "keep", (size_t)slots);
             workspace(ctx, "chunk_count", sizeof(int) * (size_t)nseg * ((max_list + kLpChunk - 1) / kLpChunk));
         }
         workspace(ctx, "seg_count", sizeof(int) * nseg);
-        if (o.precision == IRS_MIXED && o.method == 3) {  // the strip far field's buffers
-            const size_t n_strips = (size_t)((n_nu + kMxStrip - 1) / kMxStrip);
-            const size_t cb = kStripWords * sizeof(float) + sizeof(int4);
-            workspace(ctx, "strip_far", std::min((size_t)nseg * n_strips, ctx->strip_buf_max / cb) * cb);
-            workspace(ctx, "strip_M", sizeof(float) * kMxWarps * kFarNodes * kCtaNodes);
+        if (o.precision == IRS_MIXED && o.method != IRS_PSEUDOVOIGT) {  // the far field's buffers
+            const size_t cb = fw_cell_bytes(o.line_mixing == IRS_LM_PER_LINE_Y);
+            workspace(ctx, "fw_far", std::min((size_t)nseg * tree_leaves(n_nu), ctx->strip_buf_max / cb) * cb);
+            double margin = 0.0, cell, off;
+            for (auto& g : pl.segs) margin = std::max(margin, g.margin_g);
+            workspace(ctx, "fw_cell_idx", (size_t)nseg * cell_layout(n_nu, o.cutoff / ig.dnu_hi + margin, cell, off).n * sizeof(int));
         }
         if (!mixed && o.method != IRS_PSEUDOVOIGT) {
             const size_t cb = t64_cell_bytes(o.line_mixing == IRS_LM_PER_LINE_Y);
@@ -1123,7 +1176,7 @@ static void forward_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, c
     int64_t total_lines = 0;
     for (auto& l : ctx->lists) total_lines += l.n;
     const bool mixed = o.precision != IRS_FP64;
-    const size_t per_prof = (size_t)L * total_lines * (mixed ? 65 : 1 + kLpF64 * sizeof(double)) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
+    const size_t per_prof = (size_t)L * total_lines * (mixed ? 1 + kLpMixedBytes : 1 + kLpF64 * sizeof(double)) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
                             (size_t)ig.g.n * 8;
     const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {

@@ -116,18 +116,6 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
-// Per-line parameter arrays for the line sum (one slot per (segment, line)).
-struct LineParamsF64 {  // FP64 kernels; PseudoVoigt reuses f=gV, y=eta, Sn=S, Hc=base
-    double *nu0, *f, *y, *Sn, *Hc, *YSn, *b, *k0, *g;
-};
-struct LineParamsMixed {  // FP32 kernel, grid units relative to the grid start
-    double* V;            // unshifted centre (sorted key)
-    double* U;            // shifted centre
-    float4* p0;           // b2, a, c1, c0        (PV: gV2, aPV, c1, c0)
-    float4* p1;           // dfar2, An, fx, y     (PV: kPV, gPV, -, -)
-    float4* p2;           // g, Yw, dfar, - (dispersive line mixing, core reach)
-};
-
 struct Tables {
     std::map<std::pair<int, int>, std::pair<int, std::vector<double>>> tips;  // (tmin, q)
     double q_value(int mol, int iso, double T) const;  // partition.jl:8-24

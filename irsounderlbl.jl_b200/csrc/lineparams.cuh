@@ -197,8 +197,10 @@ struct LpOutMixed {
     double* V;   // unshifted centre, grid units (the sorted key of the window searches)
     float2* U;   // shifted centre, grid units, as hi + lo: hi = (float)U, lo = (float)(U - hi)
     float4 *p0, *p1;
-    float4* p2;
+    float2* p2;  // segments with line mixing only
+    float* df;   // core half-width, grid units
 };
+constexpr size_t kLpMixedBytes = 8 + 8 + 16 + 16 + 8 + 4;
 // U as hi + lo with hi a multiple of the power of two g (LpConfig::u_gran, chosen so
 // that |U| < 2^24 g over the grid and its cutoff margin): for an integer grid index w,
 // hi - w is then a multiple of g below 2^24 g in magnitude, exact in FP32, so the
@@ -315,7 +317,6 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
                                               (float)(P * (dg / c) * (dg / c)), (float)(-2.0 * P));
                     om.p1[slot] = make_float4((float)(1.0 / (gVg * gVg)),
                                               (float)(ph.S * co * (1.0 - eta) * cG / gV), 0.f, 0.f);
-                    om.p2[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             } else {
                 const double xc = c * f;
@@ -346,7 +347,8 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
                     const double c1 = P * (dg / c) * (dg / c);
                     om.p0[slot] = make_float4((float)b2, (float)(An * b * isp * ifx), (float)c1, (float)(-2.0 * P));
                     om.p1[slot] = make_float4((float)fmin(dfar * dfar, 3.0e38), (float)An, (float)fx, (float)y);
-                    om.p2[slot] = make_float4((float)(Yw * isp * ifx), (float)Yw, (float)fmin(dfar, 1.0e30), 0.f);
+                    om.df[slot] = (float)fmin(dfar, 1.0e30);
+                    if (sg.flags & 2) om.p2[slot] = make_float2((float)(Yw * isp * ifx), (float)Yw);
                 }
             }
         }
