@@ -412,12 +412,14 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
         IRS_CUDA(cudaEventRecord(ctx->ev[ev_mid], st));
         return d_tau;
     }
-    const int n_chunks = (int)((pl.max_list + kLpChunk - 1) / kLpChunk);
+    const int rounds = lp_rounds(pl.max_list, nseg);
+    const int n_chunks = (int)((pl.max_list + kLpThreads * rounds - 1) / (kLpThreads * rounds));
     unsigned char* d_keep = (unsigned char*)workspace(ctx, "keep", (size_t)pl.slots);
     int* d_chunk = (int*)workspace(ctx, "chunk_count", sizeof(int) * (size_t)nseg * n_chunks);
     LpConfig cfg;
     cfg.cutoff = o.cutoff; cfg.x_far = o.x_far; cfg.dptmn = o.dptmn;
     cfg.grid0 = grid0; cfg.dnu_g = dnu_g; cfg.method = o.method; cfg.n_nu = n_nu;
+    cfg.rounds = rounds;
     cfg.u_gran = u_granularity(n_nu, o.cutoff / dnu_g);
     const TipsDev tp = tips_dev(ctx);
     dim3 g1(n_chunks, nseg);
@@ -666,6 +668,25 @@ static const double* relmat_launch(irs_ctx* ctx, const RelmatPlan& rp, const dou
     return d_out;
 }
 
+// the FP64 radiative transfer of np profiles
+static void launch_rte64(irs_ctx* ctx, const double* d_tau, const LayerRT* d_lrt, const ProfileRT* d_prt, int L, int np,
+                         const double* d_grid, int64_t n_nu, int src, const ContDev& cd, double* d_I) {
+    const int n = np * L;
+    RteLayer64* d_ly = (RteLayer64*)workspace(ctx, "rte_layers", (size_t)n * sizeof(RteLayer64));
+    rte_layers_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>(d_lrt, n, cd.mask, d_ly);
+    check_launch(ctx);
+#define IRS_RTE(G, CIA)                                                                                                \
+    rte_kernel<double, G, CIA><<<dim3((unsigned)((n_nu + RteShape<G>::points - 1) / RteShape<G>::points), np), kRteThreads, 0, \
+                                 ctx->stream>>>(d_tau, d_lrt, d_ly, d_prt, L, d_grid, n_nu, src, cd, d_I)
+    if (cd.mask & kCiaMask) {
+        if (n_nu < kRteWide) IRS_RTE(4, true); else IRS_RTE(1, true);
+    } else {
+        if (n_nu < kRteWide) IRS_RTE(4, false); else IRS_RTE(1, false);
+    }
+#undef IRS_RTE
+    check_launch(ctx);
+}
+
 static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, const irs_sounder& s,
                          const irs_fm_options& o, double* d_R, double* d_BT) {
     upload_tables(ctx);
@@ -709,7 +730,8 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
         if (slots > 0) {
             workspace(ctx, mixed ? "lpmx" : "lp64", (size_t)slots * (mixed ? kLpMixedBytes : kLpF64 * sizeof(double)));
             workspace(ctx, "keep", (size_t)slots);
-            workspace(ctx, "chunk_count", sizeof(int) * (size_t)nseg * ((max_list + kLpChunk - 1) / kLpChunk));
+            const int lc = kLpThreads * lp_rounds(max_list, (int)pl.segs.size());
+            workspace(ctx, "chunk_count", sizeof(int) * (size_t)nseg * ((max_list + lc - 1) / lc));
         }
         workspace(ctx, "seg_count", sizeof(int) * nseg);
         if (o.precision == IRS_MIXED && o.method != IRS_PSEUDOVOIGT) {  // the far field's buffers
@@ -778,25 +800,26 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
         if ((o.continua & 1) && ctx->n_h2o > 1) cd.mask |= 1;
         if ((o.continua & 2) && ctx->n_co2 > 1) cd.mask |= 2;
     }
-    dim3 g3((unsigned)((n_nu + 255) / 256), n_prof);
     if (o.precision != IRS_FP64) {
         const size_t sm = (size_t)L * sizeof(RteLayerF);
         IRS_REQUIRE(sm <= 200 * 1024, "too many layers for the RTE kernel (at most 4266)");
+#define IRS_RTE(G, CIA)                                                                                                \
+    do {                                                                                                               \
+        if (sm > 32 * 1024) /* beside the kernel's own 16 KB */                                                        \
+            IRS_CUDA(cudaFuncSetAttribute(rte_mixed_kernel<G, CIA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+        rte_mixed_kernel<G, CIA><<<dim3((unsigned)((n_nu + RteShape<G>::points - 1) / RteShape<G>::points), n_prof), kRteThreads, sm, st>>>( \
+            (const float*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);                           \
+    } while (0)
         if (cd.mask & kCiaMask) {
-            if (sm > 48 * 1024)
-                IRS_CUDA(cudaFuncSetAttribute(rte_mixed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            rte_mixed_kernel<true><<<g3, 256, sm, st>>>((const float*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);
+            if (n_nu < kRteWide) IRS_RTE(4, true); else IRS_RTE(1, true);
         } else {
-            if (sm > 48 * 1024)
-                IRS_CUDA(cudaFuncSetAttribute(rte_mixed_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            rte_mixed_kernel<false><<<g3, 256, sm, st>>>((const float*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);
+            if (n_nu < kRteWide) IRS_RTE(4, false); else IRS_RTE(1, false);
         }
-    } else
-        if (cd.mask & kCiaMask)
-            rte_kernel<double, true><<<g3, 256, 0, st>>>((const double*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);
-        else
-            rte_kernel<double><<<g3, 256, 0, st>>>((const double*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);
-    check_launch(ctx);
+#undef IRS_RTE
+        check_launch(ctx);
+    } else {
+        launch_rte64(ctx, (const double*)d_tau, d_lrt, d_prt, L, n_prof, d_grid, n_nu, o.source_function, cd, d_I);
+    }
     IRS_CUDA(cudaEventRecord(ctx->ev[3], st));
     launch_ils(ctx, d_I, n_nu, n_prof, ig, ch, o.with_ils, d_R, d_BT);
     IRS_CUDA(cudaEventRecord(ctx->ev[4], st));
@@ -2039,9 +2062,7 @@ int irs_schwarzschild_rte(irs_ctx* ctx, const double* grid, int64_t n_nu, int n_
     double* d_I = (double*)workspace(ctx, "op_out", (size_t)n_nu * sizeof(double));
     ContDev cd{};
     cd.mask = 0;
-    rte_kernel<double><<<dim3((unsigned)((n_nu + 255) / 256), 1), 256, 0, ctx->stream>>>(
-        d_tau, d_lrt, d_prt, n_layers, d_grid, n_nu, source_function, cd, d_I);
-    check_launch(ctx);
+    launch_rte64(ctx, d_tau, d_lrt, d_prt, n_layers, 1, d_grid, n_nu, source_function, cd, d_I);
     to_host(ctx, I, d_I, n_nu);
     IRS_API_END
 }

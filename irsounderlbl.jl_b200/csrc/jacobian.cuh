@@ -975,12 +975,6 @@ struct JgProfile {     // per profile
     int n_state;
 };
 
-// 1/x: MUFU's 20-bit estimate and one third-order step (rcp64_fast), IEEE division outside
-// the range where it holds
-__device__ __forceinline__ double rcp64(double x) {
-    const double a = fabs(x);
-    return a > 1e-290 && a < 1e290 ? rcp64_fast(x) : 1.0 / x;
-}
 // exp(a) for the small arguments of the temperature differences (a^7/5040 < 1e-17)
 __device__ __forceinline__ double exp_small(double a) {
     if (fabs(a) > 0.01) return exp(a);
@@ -1036,10 +1030,6 @@ __device__ __forceinline__ void planck_grad64(double c1nu3, double nu, double c2
     const double x = nu * c2T, r = rcp64(expm1(x));
     B = c1nu3 * r;
     dB = B * (x * iT) * (1.0 + r);
-}
-// radfn (continuum.jl:169-174) with e = exp(-x)
-__device__ __forceinline__ double radfn_e(double nu, double x, double e) {
-    return x <= 0.01 ? 0.5 * x * nu : x <= 10.0 ? nu * (1.0 - e) * rcp64(1.0 + e) : nu;
 }
 // _cim_correction and its derivative (schwarzschild.jl:59-63, schwarzschild_jacobian.jl) with
 // w = exp(-s)

@@ -9,7 +9,7 @@
 //   DPTMIN peak test               voigt.jl:333-355
 //   VP_Y dispersive weight         line_mixing.jl:1193-1220 with Y(T) = y0 (296/T)^0.75
 //
-// Two passes over (segment, chunk of kLpChunk lines): pass A decides keep/reject
+// Two passes over (segment, chunk of kLpThreads x rounds lines): pass A decides keep/reject
 // and counts per chunk; pass B recomputes the parameters of the kept lines and
 // writes them compacted (order preserved), so the line sums only see kept lines.
 #pragma once
@@ -18,12 +18,20 @@
 namespace irs {
 
 constexpr int kLpThreads = 256;
-constexpr int kLpPerThread = 8;
+constexpr int kLpPerThread = 8;  // rounds of a thread at most (LpConfig::rounds)
 // Both passes are latency-bound (FP64 line physics, scattered line loads): three
 // 256-thread CTAs per SM (80 registers, a few spills) measured 13 % faster than the
 // two that 96-128 registers allow, four (64 registers) slower again.
 constexpr int kLpMinBlocks = 3;
-constexpr int kLpChunk = kLpThreads * kLpPerThread;  // lines per CTA
+// Rounds per CTA: eight share a CTA's set-up, but a short list then leaves most SMs without
+// one (5,000 lines x 49 layers: 147 CTAs in a serial chain of eight lines, keep + write 13.5 +
+// 20.2 us, at two rounds 10.2 + 17.8; the same list in one segment 3.6 + 24.4, at one round 2.9
+// + 6.3).  Fewer rounds until the launch has three CTAs per SM.
+inline int lp_rounds(long long max_list, int nseg) {
+    int r = kLpPerThread;
+    while (r > 1 && (max_list + kLpThreads * r - 1) / (kLpThreads * r) * nseg < 148 * kLpMinBlocks) r /= 2;
+    return r;
+}
 
 struct ListDev {
     const double *nu, *S296, *E, *gair, *gself, *nair, *delta, *y0;
@@ -49,6 +57,7 @@ struct LpConfig {
     long long n_nu;       // grid points (for the pair counts)
     double u_gran;        // granularity of the FP32 high part of the shifted centres (mixed)
     int method;           // 1 Weideman, 2 PseudoVoigt, 3 FullFaddeeva
+    int rounds;           // kLpThreads * rounds lines per CTA (a chunk)
 };
 
 __device__ __forceinline__ double tips_lookup(const TipsDev& t, int idx, double T) {
@@ -165,7 +174,8 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_keep_kernel(
     unsigned char* __restrict__ keep, int* __restrict__ chunk_count, int n_chunks_max) {
     const SegDev sg = segs[blockIdx.y];
     const ListDev L = lists[sg.list];
-    const long long base = (long long)blockIdx.x * kLpChunk;
+    const int chunk = kLpThreads * cfg.rounds;
+    const long long base = (long long)blockIdx.x * chunk;
     __shared__ int s_cnt;
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
@@ -175,7 +185,7 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_keep_kernel(
     }
     int cnt = 0;
     const SegPhys g = seg_phys(L.mol, sg.T, sg.p_atm, sg.vs);
-    for (int r = 0; r < kLpPerThread; ++r) {
+    for (int r = 0; r < cfg.rounds; ++r) {
         const long long j = base + r * kLpThreads + threadIdx.x;
         if (j >= L.n) break;
         bool k = true;
@@ -219,7 +229,8 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
     unsigned* __restrict__ seg_core_reach) {
     const SegDev sg = segs[blockIdx.y];
     const ListDev L = lists[sg.list];
-    const long long base = (long long)blockIdx.x * kLpChunk;
+    const int chunk = kLpThreads * cfg.rounds;
+    const long long base = (long long)blockIdx.x * chunk;
     if (base >= L.n) return;
     __shared__ int s_warp[kLpPerThread][kLpThreads / 32];  // kept lines per (round, warp)
     __shared__ long long s_off;
@@ -234,9 +245,9 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
             s_off = s;
             s_pairs[0] = s_pairs[1] = 0;
             s_reach = 0u;
-            if (blockIdx.x == gridDim.x - 1 || base + kLpChunk >= L.n) {
+            if (blockIdx.x == gridDim.x - 1 || base + chunk >= L.n) {
                 // last chunk of the segment publishes the segment's kept count
-                const long long last = (L.n - 1) / kLpChunk;
+                const long long last = (L.n - 1) / chunk;
                 if ((long long)blockIdx.x == last)
                     seg_count[blockIdx.y] = (int)(s + chunk_count[(size_t)blockIdx.y * n_chunks_max + blockIdx.x]);
             }
@@ -246,6 +257,7 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
     unsigned bals[kLpPerThread];
 #pragma unroll
     for (int r = 0; r < kLpPerThread; ++r) {
+        if (r >= cfg.rounds) break;
         const long long j = base + r * kLpThreads + threadIdx.x;
         bals[r] = __ballot_sync(0xffffffffu, j < L.n && keep[sg.off + j]);
         if (lane == 0) s_warp[r][warp] = __popc(bals[r]);
@@ -258,7 +270,7 @@ __global__ void __launch_bounds__(kLpThreads, kLpMinBlocks) lp_write_kernel(
     const SegPhys g = seg_phys(L.mol, sg.T, sg.p_atm, sg.vs);
     const double inv_dg = 1.0 / cfg.dnu_g, inv_gran = 1.0 / cfg.u_gran;  // u_gran: a power of two
 #pragma unroll 1
-    for (int r = 0; r < kLpPerThread; ++r) {
+    for (int r = 0; r < cfg.rounds; ++r) {
         const long long j = base + r * kLpThreads + threadIdx.x;
         const unsigned bal = bals[r];
         const bool k = (bal >> lane) & 1u;

@@ -29,6 +29,7 @@
 // the spectrum's norm before, 6.2e-16 / 5.7e-16 after.
 #pragma once
 #include "linesum.cuh"
+#include "rte_ils.cuh"  // rcp64_fast
 
 namespace irs {
 
@@ -45,14 +46,6 @@ struct T64Tables {
     double L4[kT64Nodes][128], L1[kT64Nodes][32];  // [k][i]: L_k at point i of a 128- / 32-point leaf
 };
 
-// 1/x for positive normal x: MUFU's 20-bit estimate and one third-order step
-// y (1 + e + e^2), e = 1 - x y (error e^3 = 2^-60 before rounding)
-__device__ __forceinline__ double rcp64_fast(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
 // four reciprocals from one (Montgomery's trick); products of the far-wing denominators
 // (between about 1e-4 and 1e3 cm^-2 squared) stay normal
 __device__ __forceinline__ void rcp64_quad(const double e[4], double r[4]) {

@@ -148,24 +148,34 @@ __global__ void grid_values_kernel(GridDev g, double* out) {
     if (i < g.n) out[i] = g.at(i);
 }
 
-__device__ __forceinline__ double planck64(double nu, double T) {
-    return 1.191042953e-5 * (nu * nu * nu) / expm1(1.4387769 * nu / T);
+// 1/x for positive normal x: MUFU's 20-bit estimate and one third-order step
+// y (1 + e + e^2), e = 1 - x y (error e^3 = 2^-60 before rounding)
+__device__ __forceinline__ double rcp64_fast(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
-__device__ __forceinline__ double cim_corr(double s) {  // schwarzschild.jl:59-63
+// the same for any x: IEEE division outside the range where it holds
+__device__ __forceinline__ double rcp64(double x) {
+    const double a = fabs(x);
+    return a > 1e-290 && a < 1e290 ? rcp64_fast(x) : 1.0 / x;
+}
+// planck_radiance (planck.jl:22-24) with c1 nu^3 and c2/T given
+__device__ __forceinline__ double planck64(double c1nu3, double nu, double c2T) { return c1nu3 * rcp64(expm1(nu * c2T)); }
+// _cim_correction (schwarzschild.jl:59-63) and _lit_correction (:43-47) with w = exp(-s)
+__device__ __forceinline__ double cim_w(double s, double w) {
     if (s < 0.06) return s / 6.0;
-    const double e = exp(-s);
-    return 1.0 - 2.0 * (e / (e - 1.0) + 1.0 / s);
+    const double a = w - 1.0, r = rcp64(s * a);  // 1/s = a r, 1/(w - 1) = s r
+    return 1.0 - 2.0 * fma(w, s * r, a * r);
 }
-__device__ __forceinline__ double lit_corr(double s) {  // schwarzschild.jl:43-47
+__device__ __forceinline__ double lit_w(double s, double w) {
     if (s < 1e-4) return s * (0.5 - s * (1.0 / 3.0 - s * 0.125));
-    const double e = exp(-s);
-    return (1.0 - e) / s - e;
+    return (1.0 - w) * rcp64(s) - w;
 }
-__device__ __forceinline__ double radfn(double nu, double T) {  // continuum.jl:169-174
-    const double x = 1.4387769 * nu / T;
-    if (x <= 0.01) return 0.5 * x * nu;
-    if (x <= 10.0) return nu * (1.0 - exp(-x)) / (1.0 + exp(-x));
-    return nu;
+// radfn (continuum.jl:169-174) with x = c2 nu / T and e = exp(-x)
+__device__ __forceinline__ double radfn_e(double nu, double x, double e) {
+    return x <= 0.01 ? 0.5 * x * nu : x <= 10.0 ? nu * (1.0 - e) * rcp64(1.0 + e) : nu;
 }
 // Interpolations.jl linear interpolation, Flat() extrapolation
 struct Lerp {
@@ -188,97 +198,156 @@ __device__ __forceinline__ double lerp_val(const double* v, const Lerp& l) {
     return v[l.i] * (1.0 - l.w) + v[l.i + 1] * l.w;
 }
 
-template <bool CIA, typename TT>
-__device__ __forceinline__ double layer_tau(const TT* tau_l, long long i, double nu, const LayerRT& r,
-                                            const ContDev& c, double Cs, double Cf, double te, double Se,
-                                            double td, const CiaPoint& cp) {
-    double t = (double)tau_l[i];
-    if (CIA) t += cia_tau(c, cp, nu, r.vmr_h2o, r.vmr_co2, r.p_mid, r.T_mid, r.dz_cm);
-    if (c.mask) {
+// Constants of one layer for rte_kernel: c2/T at its temperatures and the MT-CKD continua's
+// column factors and exponents, formed once per (profile, layer).
+struct RteLayer64 {
+    double c2a, c2t, c2b;               // c2/T at T_ave, T_top, T_bot
+    double c2m, l296, l246, G, vh, vc;  // c2/T_mid, ln(296/T_mid), ln(T_mid/246), rho n1 dz, VMRs
+};
+__global__ void __launch_bounds__(128) rte_layers_kernel(const LayerRT* __restrict__ lrt, int n, int cont,
+                                                         RteLayer64* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const LayerRT r = lrt[i];
+    RteLayer64 o{};
+    o.c2a = 1.4387769 / r.T_ave;
+    o.c2t = 1.4387769 / r.T_top;
+    o.c2b = 1.4387769 / r.T_bot;
+    if (cont) {
         const double T = r.T_mid, p = r.p_mid;
-        const double rho = (p / 1013.0) * (296.0 / T);
-        const double rad = radfn(nu, T);
-        if (c.mask & 1) {
-            const double n = r.vmr_h2o * p * 100.0 / (1.380649e-23 * T) * 1e-6;
-            const double ks = Cs * pow(296.0 / T, te) * r.vmr_h2o * rho * rad * n;
-            const double kf = Cf * (1.0 - r.vmr_h2o) * rho * rad * n;
-            t += (ks + kf) * r.dz_cm;
-        }
-        if (c.mask & 2) {
-            const double n = r.vmr_co2 * p * 100.0 / (1.380649e-23 * T) * 1e-6;
-            const double pref = 1e-20 * n * rho;
-            const double tc = td == 0.0 ? 1.0 : pow(T / 246.0, td);
-            t += Se * tc * pref * rad * r.dz_cm;
-        }
+        o.c2m = 1.4387769 / T;
+        o.l296 = log(296.0 / T);
+        o.l246 = log(T / 246.0);
+        o.G = (p / 1013.0) * (296.0 / T) * (p * 100.0 / (1.380649e-23 * T) * 1e-6) * r.dz_cm;
+        o.vh = r.vmr_h2o;
+        o.vc = r.vmr_co2;
     }
-    return t;
+    out[i] = o;
+}
+
+// A point's layers are cut into G runs, one thread each: within a run the recursion from its
+// top (transmittance 1), and the runs are joined by the products of their transmittances,
+//   I = sum_g T_above(g) I_g,      D <- D T_g + D_g   (downwelling at the run's bottom),
+// so that the serial chain of a point is a G-th as long and G times the warps hide it: one
+// scene's 34,801 points were 136 CTAs, one wave of one CTA per SM, each thread 49 layers in a
+// row.  G = 4 for grids under kRteWide points (FP32, 34,801 points: 52 us at G = 1, 26 at 4),
+// else 1, where the points alone fill the chip and a point's set-up and join are made once
+// (4.2 M points: 2.07 ms at G = 1, 2.9 at 4).  The rule reads the grid only, so that a batch
+// equals its profiles one by one.  Threads of one run hold consecutive points.
+constexpr int kRteThreads = 256;
+constexpr long long kRteWide = 148LL * 1024;
+template <int G>
+struct RteShape {
+    static constexpr int points = kRteThreads / G;
+};
+
+// MT-CKD coefficients at a point, by the threads of the first two runs for all of its runs
+template <int G>
+struct RteCont {
+    double v[5][RteShape<G>::points];  // h2o self, foreign, exponent; co2 strength, exponent
+};
+template <int G>
+__device__ __forceinline__ void rte_cont_load(const ContDev& cont, double nu, int pt, int g, RteCont<G>& c) {
+    if ((cont.mask & 1) && g == 0) {
+        const Lerp l = lerp_at(cont.h2o, cont.n_h2o, nu);
+        c.v[0][pt] = lerp_val(cont.h2o + cont.n_h2o, l);
+        c.v[1][pt] = lerp_val(cont.h2o + 2 * cont.n_h2o, l);
+        c.v[2][pt] = lerp_val(cont.h2o + 3 * cont.n_h2o, l);
+    }
+    if ((cont.mask & 2) && g == (G > 1 ? 1 : 0)) {
+        const Lerp l = lerp_at(cont.co2, cont.n_co2, nu);
+        c.v[3][pt] = lerp_val(cont.co2 + cont.n_co2, l);
+        c.v[4][pt] = lerp_val(cont.co2 + 2 * cont.n_co2, l);
+    }
+    if (G > 1) __syncthreads();
 }
 
 // CIA: a CIA table is in use (a separate instantiation keeps the per-point CIA cache
-// out of the common kernel)
-template <typename TT, bool CIA = false>
-__global__ void __launch_bounds__(256) rte_kernel(const TT* __restrict__ tau, const LayerRT* __restrict__ lrt,
-                                                  const ProfileRT* __restrict__ prt, int L,
-                                                  const double* __restrict__ grid, long long n_nu, int src,
+// out of the common kernel).  Bound by FP64 issue and latency.  One exponential per continuum
+// term and per transmittance, one expm1 per Planck radiance (the level between two layers
+// once), reciprocals in place of divisions.  One scene (34,801 points x 49 layers) 116 -> 44
+// us; with a reflecting surface, Toon source and 44,801 points 246 -> 38 us.
+template <typename TT, int G, bool CIA = false>
+__global__ void __launch_bounds__(kRteThreads) rte_kernel(const TT* __restrict__ tau, const LayerRT* __restrict__ lrt,
+                                                  const RteLayer64* __restrict__ lay, const ProfileRT* __restrict__ prt,
+                                                  int L, const double* __restrict__ grid, long long n_nu, int src,
                                                   ContDev cont, double* __restrict__ I) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int P = RteShape<G>::points;
+    __shared__ double sT[G][P], sI[G][P], sD[G][P];
+    __shared__ RteCont<G> sC;
+    const int pt = threadIdx.x % P, g = threadIdx.x / P;
+    const long long i_raw = (long long)blockIdx.x * P + pt;
     const int p = blockIdx.y;
-    if (i >= n_nu) return;
-    const double nu = grid[i];
+    const long long i = min(i_raw, n_nu - 1);
+    const double nu = grid[i], c1nu3 = 1.191042953e-5 * (nu * nu * nu);
+    rte_cont_load<G>(cont, nu, pt, g, sC);
     double Cs = 0, Cf = 0, te = 0, Se = 0, td = 0;
     if (cont.mask & 1) {
-        const Lerp l = lerp_at(cont.h2o, cont.n_h2o, nu);
-        Cs = lerp_val(cont.h2o + cont.n_h2o, l);
-        Cf = lerp_val(cont.h2o + 2 * cont.n_h2o, l);
-        te = lerp_val(cont.h2o + 3 * cont.n_h2o, l);
+        Cs = sC.v[0][pt];
+        Cf = sC.v[1][pt];
+        te = sC.v[2][pt];
     }
     if (cont.mask & 2) {
-        const Lerp l = lerp_at(cont.co2, cont.n_co2, nu);
-        Se = lerp_val(cont.co2 + cont.n_co2, l);
-        td = lerp_val(cont.co2 + 2 * cont.n_co2, l);
+        Se = 1e-20 * sC.v[3][pt];
+        td = sC.v[4][pt];
     }
     CiaPoint cp;
     if (CIA) cia_prepare(cont.cia, cont.mask, nu, cp);
     const ProfileRT pr = prt[p];
+    const double invmu = 1.0 / pr.mu;
+    const bool refl = pr.eps < 1.0, mt = (cont.mask & 3) != 0;
     const LayerRT* lr = lrt + (size_t)p * L;
-    const TT* tp = tau + (size_t)p * L * n_nu;
-    double Tr_up = 1.0;   // transmittance of the level above (TOA = 1)
-    double I_atm = 0.0;
-    for (int k = L - 1; k >= 0; --k) {
-        const LayerRT r = lr[k];
-        const double s = layer_tau<CIA>(tp + (size_t)k * n_nu, i, nu, r, cont, Cs, Cf, te, Se, td, cp) / pr.mu;
-        const double Tr_k = Tr_up * exp(-s);
-        const double dT = Tr_up - Tr_k;
+    const RteLayer64* ly = lay + (size_t)p * L;
+    const TT* tp = tau + (size_t)p * L * n_nu + i;
+    // this run: layers k1 - 1 down to k0 (group 0 at the top)
+    const int k1 = (int)((long long)L * (G - g) / G), k0 = (int)((long long)L * (G - 1 - g) / G);
+    double T = 1.0, Iv = 0.0, D = 0.0;
+    double Bt = k1 > k0 ? planck64(c1nu3, nu, ly[k1 - 1].c2t) : 0.0;  // at the top of the current layer
+    for (int k = k1 - 1; k >= k0; --k) {
+        const RteLayer64& r = ly[k];
+        double t = (double)tp[(size_t)k * n_nu];
+        if (mt) {  // continuum.jl:169-250
+            const double x = nu * r.c2m;
+            double E = 0.0, Q = 1.0;
+            if (cont.mask & 1) E = exp(te * r.l296);
+            if ((cont.mask & 2) && td != 0.0) Q = exp(td * r.l246);
+            t = fma(r.G * radfn_e(nu, x, exp(-x)), fma(r.vh, fma(Cs * E, r.vh, Cf * (1.0 - r.vh)), Se * Q * r.vc), t);
+        }
+        if (CIA) t += cia_tau(cont, cp, nu, lr[k].vmr_h2o, lr[k].vmr_co2, lr[k].p_mid, lr[k].T_mid, lr[k].dz_cm);
+        const double s = t * invmu, w = exp(-s), u = 1.0 - w;
+        const double Tk = T * w, dT = T - Tk;
+        const double Bb = src != 0 || refl ? planck64(c1nu3, nu, r.c2b) : 0.0;
+        double f;
         if (src == 0) {
-            const double Ba = planck64(nu, r.T_ave), Bt = planck64(nu, r.T_top);
-            I_atm += Ba * dT + (Bt - Ba) * (dT * cim_corr(s));
+            const double Ba = planck64(c1nu3, nu, r.c2a);
+            f = cim_w(s, w);
+            Iv += Ba * dT + (Bt - Ba) * (dT * f);
+            if (refl) D = fma(D, w, u * (Ba + (Bb - Ba) * f));  // add_reflected_downwelling!, schwarzschild.jl:228-274
+            Bt = refl ? Bb : k > k0 ? planck64(c1nu3, nu, ly[k - 1].c2t) : 0.0;
         } else {
-            const double Bb = planck64(nu, r.T_bot), Bt = planck64(nu, r.T_top);
-            I_atm += Bt * dT + (Bb - Bt) * (Tr_up * lit_corr(s));
+            f = lit_w(s, w);
+            Iv += Bt * dT + (Bb - Bt) * (T * f);
+            if (refl) D = fma(D, w, Bb * u + (Bt - Bb) * f);
+            Bt = Bb;
         }
-        Tr_up = Tr_k;
+        T = Tk;
     }
-    const double Tr0 = Tr_up;
-    double Iv = pr.eps * planck64(nu, pr.T_sfc) * Tr0 + I_atm;
-    if (pr.eps < 1.0) {
-        double Id = 0.0, g = 1.0;
-        for (int k = 0; k < L; ++k) {
-            const LayerRT r = lr[k];
-            const double s = layer_tau<CIA>(tp + (size_t)k * n_nu, i, nu, r, cont, Cs, Cf, te, Se, td, cp) / pr.mu;
-            double em;
-            if (src == 0) {
-                const double Ba = planck64(nu, r.T_ave), Bb = planck64(nu, r.T_bot);
-                em = (1.0 - exp(-s)) * (Ba + (Bb - Ba) * cim_corr(s));
-            } else {
-                const double Bb = planck64(nu, r.T_bot), Bt = planck64(nu, r.T_top);
-                em = Bb * (1.0 - exp(-s)) + (Bt - Bb) * lit_corr(s);
-            }
-            Id += g * em;
-            g *= exp(-s);
+    sT[g][pt] = T;
+    sI[g][pt] = Iv;
+    sD[g][pt] = D;
+    __syncthreads();
+    if (g == 0 && i_raw < n_nu) {
+        double Tt = 1.0, It = 0.0, Dt = 0.0;
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            It = fma(Tt, sI[q][pt], It);
+            Dt = fma(Dt, sT[q][pt], sD[q][pt]);
+            Tt *= sT[q][pt];
         }
-        Iv += (1.0 - pr.eps) * Id * Tr0;
+        It += pr.eps * planck64(c1nu3, nu, 1.4387769 / pr.T_sfc) * Tt;
+        if (refl) It += (1.0 - pr.eps) * Dt * Tt;
+        I[(size_t)p * n_nu + i] = It;
     }
-    I[(size_t)p * n_nu + i] = Iv;
 }
 
 // ------------------------------------------------------- RTE, mixed precision
@@ -291,17 +360,24 @@ __global__ void __launch_bounds__(256) rte_kernel(const TT* __restrict__ tau, co
 //
 // Per-layer FP32 constants, computed once per CTA from LayerRT into shared memory:
 struct RteLayerF {
-    float c2_ave, c2_top, c2_bot, c2_mid;  // c2 / T
+    float2 c2_ave, c2_top, c2_bot;         // c2 / T as hi + lo
+    float c2_mid;
     float h2o_self, h2o_for, l2_296, co2;  // continuum column factors, log2(296/T_mid)
-    float l2_246, pad0, pad1, pad2;        // log2(T_mid / 246)
+    float l2_246;                          // log2(T_mid / 246)
 };
-constexpr float kC1 = 1.191042953e-5f, kC2 = 1.4387769f;
-
-// planck_radiance (planck.jl:22-24) with c1 nu^3 and c2/T given: c1 nu^3 / expm1(c2 nu / T);
-// above x = 0.5 exp(x) - 1 loses under one bit, so the cheaper expf serves there
-__device__ __forceinline__ float planck32(float c1nu3, float nu, float c2T) {
-    const float x = nu * c2T;
-    return c1nu3 * __frcp_rn(x > 0.5f ? expf(x) - 1.0f : expm1f(x));
+__device__ __forceinline__ float2 split_f(double x) {
+    const float h = (float)x;
+    return make_float2(h, (float)(x - (double)h));
+}
+// planck_radiance (planck.jl:22-24) with c1 nu^3, nu and c2/T given: c1 nu^3 / expm1(c2 nu / T);
+// above x = 0.5 exp(x) - 1 loses under one bit, so the cheaper expf serves there.  x carries
+// its rounding error xl (an FP32 x alone is 1e-7 x of B off, the largest error of the mixed
+// spectra): e^(x + xl) - 1 = E + xl (E + 1).
+__device__ __forceinline__ float planck32(float c1nu3, float2 nu, float2 c2T) {
+    const float x = nu.x * c2T.x;
+    const float xl = fmaf(nu.x, c2T.x, -x) + fmaf(nu.x, c2T.y, nu.y * c2T.x);
+    const float E = x > 0.5f ? expf(x) - 1.0f : expm1f(x);
+    return c1nu3 * __frcp_rn(fmaf(xl, E + 1.0f, E));
 }
 // _cim_correction (schwarzschild.jl:59-63): s/6 below 0.06 as the reference, then the
 // series 1 - 2 (1/s - 1/(e^s - 1)) = s/6 - s^3/360 + s^5/15120 - ... (next term below
@@ -335,21 +411,29 @@ __device__ __forceinline__ float radfn32(float nu, float c2T) {
     return nu;
 }
 
-template <bool CIA>
-__global__ void __launch_bounds__(256) rte_mixed_kernel(const float* __restrict__ tau, const LayerRT* __restrict__ lrt,
+// Runs of layers as in rte_kernel (G threads per point).  Within a run the
+// transmittance is exp(-od) of the run's FP64 cumulative optical depth.  One scene's 34,801
+// points 51 -> 26 us, 160,001 points with a reflecting surface 325 -> 232 us; 4.2 M points
+// 1.91 -> 2.07 ms (of 84), the price of the compensated Planck argument: BT of the 5,000-line
+// scenes against FP64 3.5e-6 -> 1.7e-6 K RMS.
+template <int G, bool CIA>
+__global__ void __launch_bounds__(kRteThreads) rte_mixed_kernel(const float* __restrict__ tau, const LayerRT* __restrict__ lrt,
                                                         const ProfileRT* __restrict__ prt, int L,
                                                         const double* __restrict__ grid, long long n_nu, int src,
                                                         ContDev cont, double* __restrict__ I) {
     extern __shared__ __align__(16) unsigned char rte_smem[];
     RteLayerF* lc = reinterpret_cast<RteLayerF*>(rte_smem);
+    constexpr int P = RteShape<G>::points;
+    __shared__ double sO[G][P], sI[G][P], sD[G][P];
+    __shared__ RteCont<G> sC;
     const int p = blockIdx.y;
     const LayerRT* lr = lrt + (size_t)p * L;
     for (int k = threadIdx.x; k < L; k += blockDim.x) {  // layer constants (FP64 -> FP32)
         const LayerRT r = lr[k];
         RteLayerF c;
-        c.c2_ave = (float)(1.4387769 / r.T_ave);
-        c.c2_top = (float)(1.4387769 / r.T_top);
-        c.c2_bot = (float)(1.4387769 / r.T_bot);
+        c.c2_ave = split_f(1.4387769 / r.T_ave);
+        c.c2_top = split_f(1.4387769 / r.T_top);
+        c.c2_bot = split_f(1.4387769 / r.T_bot);
         c.c2_mid = (float)(1.4387769 / r.T_mid);
         const double rho = (r.p_mid / 1013.0) * (296.0 / r.T_mid);
         const double nh = r.vmr_h2o * r.p_mid * 100.0 / (1.380649e-23 * r.T_mid) * 1e-6;
@@ -359,31 +443,32 @@ __global__ void __launch_bounds__(256) rte_mixed_kernel(const float* __restrict_
         c.l2_296 = (float)log2(296.0 / r.T_mid);
         c.co2 = (float)(1e-20 * nc * rho * r.dz_cm);
         c.l2_246 = (float)log2(r.T_mid / 246.0);
-        c.pad0 = c.pad1 = c.pad2 = 0.f;
         lc[k] = c;
     }
     __syncthreads();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_nu) return;
+    const int pt = threadIdx.x % P, g = threadIdx.x / P;
+    const ProfileRT pr = prt[p];
+    const float imu = (float)(1.0 / pr.mu);
+    const bool refl = pr.eps < 1.0;
+    const long long i_raw = (long long)blockIdx.x * P + pt;
+    const long long i = min(i_raw, n_nu - 1);
     const double nud = grid[i];
-    const float nu = (float)nud;
-    const float c1nu3 = kC1 * nu * nu * nu;
+    const float2 nu2 = split_f(nud);
+    const float nu = nu2.x;
+    const float c1nu3 = (float)(1.191042953e-5 * (nud * nud * nud));
+    rte_cont_load<G>(cont, nud, pt, g, sC);
     float Cs = 0.f, Cf = 0.f, te = 0.f, Se = 0.f, td = 0.f;
     if (cont.mask & 1) {
-        const Lerp l = lerp_at(cont.h2o, cont.n_h2o, nud);
-        Cs = (float)lerp_val(cont.h2o + cont.n_h2o, l);
-        Cf = (float)lerp_val(cont.h2o + 2 * cont.n_h2o, l);
-        te = (float)lerp_val(cont.h2o + 3 * cont.n_h2o, l);
+        Cs = (float)sC.v[0][pt];
+        Cf = (float)sC.v[1][pt];
+        te = (float)sC.v[2][pt];
     }
     if (cont.mask & 2) {
-        const Lerp l = lerp_at(cont.co2, cont.n_co2, nud);
-        Se = (float)lerp_val(cont.co2 + cont.n_co2, l);
-        td = (float)lerp_val(cont.co2 + 2 * cont.n_co2, l);
+        Se = (float)sC.v[3][pt];
+        td = (float)sC.v[4][pt];
     }
     CiaPoint cp;
     if (CIA) cia_prepare(cont.cia, cont.mask, nud, cp);
-    const ProfileRT pr = prt[p];
-    const float imu = (float)(1.0 / pr.mu);
     const float* tp = tau + (size_t)p * L * n_nu + i;
     // the layer's optical depth along the path (FP32)
     auto slant = [&](int k) -> float {
@@ -402,51 +487,51 @@ __global__ void __launch_bounds__(256) rte_mixed_kernel(const float* __restrict_
         }
         return t * imu;
     };
-    double od = 0.0;        // cumulative optical depth from the top of the atmosphere
+    const int k1 = (int)((long long)L * (G - g) / G), k0 = (int)((long long)L * (G - 1 - g) / G);
+    double od = 0.0;        // cumulative optical depth from the top of the run
     double Tr_up = 1.0;     // transmittance of the level above
+    double D = 0.0;         // downwelling radiance at the current bottom (reflecting surface)
     float Is = 0.f, Ic = 0.f;  // radiance, Kahan-compensated
-    float B_up = planck32(c1nu3, nu, lc[L - 1].c2_top);  // B at the top level of the current layer
-    for (int k = L - 1; k >= 0; --k) {
+    float B_up = k1 > k0 ? planck32(c1nu3, nu2, lc[k1 - 1].c2_top) : 0.f;  // B at the top level of the current layer
+    for (int k = k1 - 1; k >= k0; --k) {
         const RteLayerF& c = lc[k];
         const float s = slant(k);
         od += (double)s;
         const double Tr_k = exp(-od);
         const float dT = (float)(Tr_up - Tr_k);
-        const float B_bot = planck32(c1nu3, nu, c.c2_bot);
-        float v;
+        const float B_bot = planck32(c1nu3, nu2, c.c2_bot);
+        float v, em = 0.f;
         if (src == 0) {
-            const float Ba = planck32(c1nu3, nu, c.c2_ave);
-            v = fmaf(Ba, dT, (B_up - Ba) * (dT * cim_corr32(s)));
+            const float Ba = planck32(c1nu3, nu2, c.c2_ave), f = cim_corr32(s);
+            v = fmaf(Ba, dT, (B_up - Ba) * (dT * f));
+            if (refl) em = -expm1f(-s) * fmaf(B_bot - Ba, f, Ba);
         } else {
-            v = fmaf(B_up, dT, (B_bot - B_up) * ((float)Tr_up * lit_corr32(s)));
+            const float f = lit_corr32(s);
+            v = fmaf(B_up, dT, (B_bot - B_up) * ((float)Tr_up * f));
+            if (refl) em = fmaf(B_bot, -expm1f(-s), (B_up - B_bot) * f);
         }
+        if (refl) D = fma(D, exp(-(double)s), (double)em);  // add_reflected_downwelling!
         kahan_add32(Is, Ic, v);
         B_up = B_bot;
         Tr_up = Tr_k;
     }
-    const double Tr0 = Tr_up;
-    double Iv = (double)(Is - Ic) + pr.eps * (double)planck32(c1nu3, nu, kC2 / (float)pr.T_sfc) * Tr0;
-    if (pr.eps < 1.0) {  // add_reflected_downwelling!: layers from the surface up
-        float Ds = 0.f, Dc = 0.f;
-        double od_s = 0.0;  // optical depth from the surface to the bottom of layer k
-        for (int k = 0; k < L; ++k) {
-            const RteLayerF& c = lc[k];
-            const float s = slant(k);
-            const float one_m = -expm1f(-s);
-            float em;
-            if (src == 0) {
-                const float Ba = planck32(c1nu3, nu, c.c2_ave), Bb = planck32(c1nu3, nu, c.c2_bot);
-                em = one_m * fmaf(Bb - Ba, cim_corr32(s), Ba);
-            } else {
-                const float Bb = planck32(c1nu3, nu, c.c2_bot), Bt = planck32(c1nu3, nu, c.c2_top);
-                em = fmaf(Bb, one_m, (Bt - Bb) * lit_corr32(s));
-            }
-            kahan_add32(Ds, Dc, (float)exp(-od_s) * em);
-            od_s += (double)s;
+    sO[g][pt] = od;
+    sI[g][pt] = (double)Is - (double)Ic;
+    sD[g][pt] = D;
+    __syncthreads();
+    if (g == 0 && i_raw < n_nu) {
+        double ot = 0.0, Tt = 1.0, It = 0.0, Dt = 0.0;
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            It = fma(Tt, sI[q][pt], It);
+            if (refl) Dt = fma(Dt, exp(-sO[q][pt]), sD[q][pt]);
+            ot += sO[q][pt];
+            Tt = exp(-ot);
         }
-        Iv += (1.0 - pr.eps) * (double)(Ds - Dc) * Tr0;
+        It += pr.eps * (double)planck32(c1nu3, nu2, split_f(1.4387769 / pr.T_sfc)) * Tt;
+        if (refl) It += (1.0 - pr.eps) * Dt * Tt;
+        I[(size_t)p * n_nu + i] = It;
     }
-    I[(size_t)p * n_nu + i] = Iv;
 }
 
 // ---------------------------------------------------------------- ILS
