@@ -496,8 +496,8 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
 }
 
 __global__ void ils_float_kernel(const double* __restrict__ k, long long n, float* __restrict__ kf) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) kf[i] = (float)k[i];
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, q = i - kJgcPad;
+    if (q < n + kJgcBack) kf[i] = q >= 0 && q < n ? (float)k[q] : 0.f;
 }
 
 static void ensure_ils(irs_ctx* ctx, double dnu, double opd, double fwhm, int apod) {
@@ -511,8 +511,9 @@ static void ensure_ils(irs_ctx* ctx, double dnu, double opd, double fwhm, int ap
     ils_normalise_kernel<<<1, 1024, 0, ctx->stream>>>(k, n, dnu);
     check_launch(ctx);
     // the same taps rounded to FP32 for the Jacobian's channel contraction (FP32 sums)
-    float* kf = (float*)workspace(ctx, "ils_f", n * sizeof(float));
-    ils_float_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(k, n, kf);
+    const int64_t nf = kJgcPad + n + kJgcBack;  // zeros around them
+    float* kf = (float*)workspace(ctx, "ils_f", nf * sizeof(float));
+    ils_float_kernel<<<(unsigned)((nf + 255) / 256), 256, 0, ctx->stream>>>(k, n, kf);
     check_launch(ctx);
     std::memcpy(ctx->ils_key, key, sizeof key);
     ctx->ils_n = n;
@@ -1116,11 +1117,12 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
         const float* d_kernf = o.with_ils ? (const float*)ctx->work["ils_f"].p : nullptr;
         const ChanNodes cn = o.with_ils ? chan_nodes(ig.g, ch) : ChanNodes{0, 0};
         if (cn.step)
-            jg_channel_nodes_kernel<<<dim3((unsigned)((n_ch + kJgChan - 1) / kJgChan), (unsigned)n_state, np), kChanThreads, 0, st>>>(
+            jg_channel_nodes_kernel<<<dim3((unsigned)((n_ch + kJgChan - 1) / kJgChan), (unsigned)((n_state + 1) / 2), np), kChanThreads,
+                                      kJgChanSmem, st>>>(
                 d_D, (int)n_nu, (int)n_state, d_kernf, (int)n_taps, ig.dnu_hi, to_dev(ch), cn, d_RB, sp.observable, d_K);
         else
             jg_channel_kernel<<<dim3((unsigned)((n_ch * 32 + 255) / 256), (unsigned)n_state, np), 256, 0, st>>>(
-                d_D, n_nu, (int)n_state, d_kernf, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), o.with_ils, d_RB,
+                d_D, n_nu, (int)n_state, d_kernf ? d_kernf + kJgcPad : nullptr, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), o.with_ils, d_RB,
                 sp.observable, d_K);
         check_launch(ctx);
         if (!K_dev) {

@@ -591,8 +591,7 @@ constexpr int kChanThreads = 256;
 // point meets in the C channels are C rows of the same phase, so a ring of C registers holds
 // them and each point costs two coalesced loads for C products.  One warp per channel and
 // two loads per product, as apod_at does it, left 221 channels of one scene waiting on 400
-// dependent loads (94 us, now 13) and the Jacobian's states on L2: a 151-element IASI
-// Jacobian's contraction took 4.76 ms, now 2.10 (16 scenes x 101 x 221: 1.51, now 0.61).
+// dependent loads (94 us, now 13).  jg_channel_nodes_kernel does the same for the Jacobian.
 // Returns the sum of channel threadIdx.x to the first C threads.
 template <typename T, int C>
 __device__ __forceinline__ T chan_sums(const T* __restrict__ X, int n_nu, const T* __restrict__ kern, int n_taps,
