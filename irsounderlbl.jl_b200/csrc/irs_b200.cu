@@ -1062,22 +1062,22 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             if ((o.continua & 2) && ctx->n_co2 > 1) cd.mask |= 2;
         }
         JgRteLayer* d_jrl = (JgRteLayer*)workspace(ctx, "jg_rte_layers", (size_t)np * L * sizeof(JgRteLayer));
-        jg_rte_layers_kernel<<<(np * L + 127) / 128, 128, 0, st>>>(d_lrt, d_jl, np * L, d_jrl);
+        jg_rte_layers_kernel<<<(np * L * kJgRteFine + 127) / 128, 128, 0, st>>>(d_lrt, d_jl, np * L, ig.dnu_hi, d_jrl);
         check_launch(ctx);
-        const dim3 gr((unsigned)((n_nu + 127) / 128), np);
+        const dim3 gr((unsigned)((n_nu + kJgRteThreads - 1) / kJgRteThreads), np);
         const bool cia = (cd.mask & kCiaMask) != 0;
         if (!adjoint) {
             if (cia)
-                jg_rte_kernel<true><<<gr, 128, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid, n_nu,
+                jg_rte_kernel<true><<<gr, kJgRteThreads, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid, n_nu,
                                                         o.source_function, cd, d_I, d_D);
             else
-                jg_rte_kernel<<<gr, 128, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid, n_nu,
+                jg_rte_kernel<<<gr, kJgRteThreads, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid, n_nu,
                                                   o.source_function, cd, d_I, d_D);
         } else if (cia) {
-            jg_rte_kernel<true, 1><<<gr, 128, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid, n_nu,
+            jg_rte_kernel<true, 1><<<gr, kJgRteThreads, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid, n_nu,
                                                        o.source_function, cd, d_I, nullptr);
         } else {
-            jg_rte_kernel<false, 1><<<gr, 128, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
+            jg_rte_kernel<false, 1><<<gr, kJgRteThreads, 0, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
                                                         n_nu, o.source_function, cd, d_I, nullptr);
         }
         check_launch(ctx);
@@ -1101,10 +1101,10 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             IRS_CUDA(cudaMemsetAsync(d_xb, 0, (size_t)np * n_state * sizeof(double), st));
             const size_t xsm = (size_t)n_state * sizeof(double);
             if (cia)
-                jg_rte_kernel<true, 2><<<gr, 128, xsm, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
+                jg_rte_kernel<true, 2><<<gr, kJgRteThreads, xsm, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
                                                              n_nu, o.source_function, cd, d_I, nullptr, d_ib, d_xb);
             else
-                jg_rte_kernel<false, 2><<<gr, 128, xsm, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
+                jg_rte_kernel<false, 2><<<gr, kJgRteThreads, xsm, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
                                                               n_nu, o.source_function, cd, d_I, nullptr, d_ib, d_xb);
             check_launch(ctx);
             IRS_CUDA(cudaMemcpyAsync(dx_h + (size_t)p0 * n_state, d_xb, (size_t)np * n_state * sizeof(double),

@@ -977,12 +977,21 @@ struct JgProfile {     // per profile
     int n_state;
 };
 
-// exp(a) for the small arguments of the temperature differences (a^7/5040 < 1e-17)
+// exp(a) for small arguments (a^7/5040 < 1e-17)
 __device__ __forceinline__ double exp_small(double a) {
     if (fabs(a) > 0.01) return exp(a);
     return fma(a, fma(a, fma(a, fma(a, fma(a, fma(a, 1.0 / 720.0, 1.0 / 120.0), 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0), 1.0);
 }
 
+// exp(a) - 1 for the steps of a central difference: below 2^-8 the series' next term is
+// a^5/120 of a, under 1e-11 of the difference it goes into
+__device__ __forceinline__ double expm1_tiny(double a) {
+    if (fabs(a) > 0.00390625) return expm1(a);
+    return a * fma(a, fma(a, fma(a, fma(a, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0);
+}
+
+constexpr int kJgRteThreads = 128, kJgRteFine = 16;
+constexpr int kJgRteChunk = 64;  // layers of JgRteBase in shared memory at a time
 // Constants of one layer for jg_rte_kernel, formed once per (profile, layer): the MT-CKD
 // continua's column factor and exponents at T_mid and, as ratios, at T_mid +- 0.05 K (the
 // reference's central difference, vmr_jacobian.jl:322-344); c2/T and 1/T of the Planck terms.
@@ -994,17 +1003,31 @@ struct JgRteLayer {
     double rp, rm, dp, dm;              // T/(T + h), T/(T - h) and their logs
     double c2a, ia, c2t, it, c2b, ib;   // c2/T and 1/T at T_ave, T_top, T_bot
     double frac, wM;
+    // exp(-c2/T j d), d the grid step, at T_mid, T_ave, T_top: the factors of exp(-c2 nu/T)
+    // within 16 grid points (JgRteBase has the other factor)
+    double step[3][kJgRteFine];
+};
+// Per CTA and layer: exp(-c2 nu/T) at T_mid, T_ave, T_top on every 16th of its points, and
+// the self continuum's (296/T)^te at the first.
+struct JgRteBase {
+    double q[3][kJgRteThreads / kJgRteFine];
+    double E;
 };
 constexpr double kJgRteDT = 0.05;
 __global__ void __launch_bounds__(128) jg_rte_layers_kernel(const LayerRT* __restrict__ lrt, const JgLayer* __restrict__ jl,
-                                                            int n, JgRteLayer* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                            int n, double dnu, JgRteLayer* __restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kJgRteFine, j = t % kJgRteFine;
     if (i >= n) return;
     const LayerRT r = lrt[i];
-    const JgLayer y = jl[i];
-    JgRteLayer o;
+    JgRteLayer& o = out[i];
     const double T = r.T_mid, p = r.p_mid;
-    o.c2m = 1.4387769 / T;
+    const double c2m = 1.4387769 / T, c2a = 1.4387769 / r.T_ave, c2t = 1.4387769 / r.T_top;
+    o.step[0][j] = exp(-c2m * (j * dnu));
+    o.step[1][j] = exp(-c2a * (j * dnu));
+    o.step[2][j] = exp(-c2t * (j * dnu));
+    if (j) return;
+    const JgLayer y = jl[i];
+    o.c2m = c2m;
     o.l296 = log(296.0 / T);
     o.l246 = log(T / 246.0);
     const double rho = (p / 1013.0) * (296.0 / T), n1 = p * 100.0 / (1.380649e-23 * T) * 1e-6;
@@ -1015,15 +1038,14 @@ __global__ void __launch_bounds__(128) jg_rte_layers_kernel(const LayerRT* __res
     o.rm = T / (T - kJgRteDT);
     o.dp = -log1p(kJgRteDT / T);
     o.dm = -log1p(-kJgRteDT / T);
-    o.c2a = 1.4387769 / r.T_ave;
+    o.c2a = c2a;
     o.ia = 1.0 / r.T_ave;
-    o.c2t = 1.4387769 / r.T_top;
+    o.c2t = c2t;
     o.it = 1.0 / r.T_top;
     o.c2b = 1.4387769 / r.T_bot;
     o.ib = 1.0 / r.T_bot;
     o.frac = y.frac;
     o.wM = y.wM;
-    out[i] = o;
 }
 
 // planck_radiance and dB/dT (planck.jl:22-24, :67-71) from one expm1 and one reciprocal:
@@ -1032,6 +1054,14 @@ __device__ __forceinline__ void planck_grad64(double c1nu3, double nu, double c2
     const double x = nu * c2T, r = rcp64(expm1(x));
     B = c1nu3 * r;
     dB = B * (x * iT) * (1.0 + r);
+}
+// the same with q = exp(-x) given: 1/(e^x - 1) = q/(1 - q); where 1 - q would lose more than
+// two bits, from x
+__device__ __forceinline__ void planck_grad64_q(double c1nu3, double nu, double c2T, double iT, double q, double& B, double& dB) {
+    if (q > 0.75) return planck_grad64(c1nu3, nu, c2T, iT, B, dB);
+    const double r = q * rcp64_fast(1.0 - q);
+    B = c1nu3 * r;
+    dB = B * (nu * c2T * iT) * (1.0 + r);
 }
 // _cim_correction and its derivative (schwarzschild.jl:59-63, schwarzschild_jacobian.jl) with
 // w = exp(-s)
@@ -1071,24 +1101,26 @@ __device__ __forceinline__ void lit_both(double s, double w, double& f, double& 
 //      = sum_nu Ibar D[x] = (K^T dy)[x].  D is never stored.  Dynamic shared memory:
 //      n_state doubles.
 //
-// Bound by FP64 issue and latency (about 420 FP64 instructions a point and layer; the bytes,
-// 0.9 GB for 16 scenes, take 0.14 ms).  Six CTAs per SM (80 registers, a few spills) against
-// the four that 112 registers allow: 1.59 / 1.92 ms (16 scenes), 1.24 / 1.37 (adjoint);
-// five 1.71 / 1.45.  With JgRteLayer and one exponential per term, 16 scenes of the
-// 5,000-line list 3.69 -> 1.59 ms, one IASI profile 7.11 -> 2.42, the adjoint of two
-// 645-1000 cm^-1 profiles 1.13 + 4.38 -> 0.53 + 1.24.
+// Bound by latency and issue (some 970 instructions a point and layer, 290 of them FP64; the
+// bytes, 0.9 GB for 16 scenes, take 0.14 ms), so registers are given up for warps: eight CTAs
+// per SM in forward mode (64 registers, some spills; 1.28 ms, seven 1.39, six 1.44), six in
+// the adjoint (1.04 ms, eight 1.19).  exp(-c2 nu/T) is the product of a factor per 16th point
+// and one per step, both from tables, and the continuum exponent's change across a CTA a short
+// series; the next layer's sums are prefetched.  16 scenes of the 5,000-line list 1.59 -> 1.28
+// ms (3.69 with every continuum evaluated from scratch), one IASI profile 2.42 -> 2.15, the
+// adjoint of two 645-1000 cm^-1 profiles 0.55 + 1.25 -> 0.47 + 1.04.
 template <bool CIA = false, int MODE = 0>
-__global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
+__global__ void __launch_bounds__(kJgRteThreads, CIA ? 1 : MODE == 0 ? 8 : 6) jg_rte_kernel(
     const float* __restrict__ jl, int n_out, const LayerRT* __restrict__ lrt, const JgRteLayer* __restrict__ jlay,
     const ProfileRT* __restrict__ prt, const JgProfile* __restrict__ jprof, const double* __restrict__ vlev,
     int L, const double* __restrict__ grid, long long n_nu, int src, ContDev cont, double* __restrict__ I,
     float* __restrict__ D, const double* __restrict__ Ibar = nullptr, double* __restrict__ xbar = nullptr) {
     extern __shared__ double jg_xsh[];
-    const long long i_raw = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ JgRteBase base[kJgRteChunk];
+    const long long i0 = (long long)blockIdx.x * kJgRteThreads, i_raw = i0 + threadIdx.x;
     const int p = blockIdx.y;
     const bool valid = i_raw < n_nu;
-    if (MODE != 2 && !valid) return;
-    // the adjoint keeps every lane to the end (warp reductions); others are clamped
+    // every lane stays to the end (the layers' base, the adjoint's reductions), clamped
     const long long i = valid ? i_raw : n_nu - 1;
     if (MODE == 2) {
         for (int x = threadIdx.x; x < jprof[p].n_state; x += blockDim.x) jg_xsh[x] = 0.0;
@@ -1114,6 +1146,25 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
         Se = 1e-20 * lerp_val(cont.co2 + cont.n_co2, l);
         td = lerp_val(cont.co2 + 2 * cont.n_co2, l);
     }
+    __shared__ double te_first;
+    if (threadIdx.x == 0) te_first = te;
+    auto fill = [&](int k0) {  // the base of the layers k0 ..
+        __syncthreads();
+        constexpr int Q = kJgRteThreads / kJgRteFine;
+        const int nl = min(kJgRteChunk, L - k0);
+        for (int e = threadIdx.x; e < nl * 3 * Q; e += kJgRteThreads) {
+            const int k = e / (3 * Q), x = e / Q % 3, a = e % Q;
+            const JgRteLayer& r = jy[k0 + k];
+            base[k].q[x][a] = exp(-grid[min(i0 + a * kJgRteFine, n_nu - 1)] * (x == 0 ? r.c2m : x == 1 ? r.c2a : r.c2t));
+        }
+        if (cont.mask & 1)
+            for (int k = threadIdx.x; k < nl; k += kJgRteThreads) base[k].E = exp(te_first * jy[k0 + k].l296);
+        __syncthreads();
+    };
+    // exp(-c2 nu/T) of layer k, x as in JgRteBase
+    auto q_at = [&](int k, const JgRteLayer& r, int x) {
+        return base[k % kJgRteChunk].q[x][threadIdx.x / kJgRteFine] * __ldg(&r.step[x][threadIdx.x % kJgRteFine]);
+    };
     CiaPoint cp;
     if (CIA) cia_prepare(cont.cia, cont.mask, nu, cp);
     const double invmu = 1.0 / pr.mu, eps = pr.eps;
@@ -1123,11 +1174,11 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
         double x, e, E, Q;  // c2 nu / T, exp(-x), (296/T)^te, (T/246)^td
     };
     const bool mt = (cont.mask & 3) != 0;
-    auto cont_at = [&](const JgRteLayer& r) {
+    auto cont_at = [&](int k, const JgRteLayer& r) {
         Cont c{0.0, 0.0, 0.0, 1.0};
         c.x = nu * r.c2m;
-        c.e = exp(-c.x);
-        if (cont.mask & 1) c.E = exp(te * r.l296);
+        c.e = q_at(k, r, 0);
+        if (cont.mask & 1) c.E = base[k % kJgRteChunk].E * exp_small((te - te_first) * r.l296);
         if ((cont.mask & 2) && td != 0.0) c.Q = exp(td * r.l246);
         return c;
     };
@@ -1147,26 +1198,31 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
     };
     // pass 1: total optical depth and the downwelling radiance at the surface
     double OD = 0.0, Id = 0.0, gk = 1.0;
+    double Bb, dBb;  // at the layer's bottom level: the top of the layer below
+    planck_grad64(c1nu3, nu, jy[0].c2b, jy[0].ib, Bb, dBb);
+    const double B0 = Bb, dB0 = dBb;
     for (int k = 0; k < L; ++k) {
+        if (k % kJgRteChunk == 0) fill(k);
+        if (k + 2 < L) asm volatile("prefetch.global.L1 [%0];" ::"l"(out + (size_t)(k + 2) * n_out * n_nu + i));
         const JgRteLayer& r = jy[k];
         Cont c{};
-        if (mt) c = cont_at(r);
+        if (mt) c = cont_at(k, r);
         const double s = layer_s(k, r, c);
         OD += s;
         if (eps < 1.0) {  // schwarzschild_jacobian.jl:221-243
             const double w = exp(-s), u = 1.0 - w;
-            double Ba, Bb, f, fp, d;
-            planck_grad64(c1nu3, nu, r.c2b, r.ib, Bb, d);
+            double Ba, Bt, f, fp, d;
+            planck_grad64_q(c1nu3, nu, r.c2t, r.it, q_at(k, r, 2), Bt, d);
             if (src == 0) {
-                planck_grad64(c1nu3, nu, r.c2a, r.ia, Ba, d);
+                planck_grad64_q(c1nu3, nu, r.c2a, r.ia, q_at(k, r, 1), Ba, d);
                 cim_both(s, w, f, fp);
                 Id += gk * (u * fma(Bb - Ba, f, Ba));
             } else {
-                planck_grad64(c1nu3, nu, r.c2t, r.it, Ba, d);
                 lit_both(s, w, f, fp);
-                Id += gk * fma(Ba - Bb, f, Bb * u);
+                Id += gk * fma(Bt - Bb, f, Bb * u);
             }
             gk *= w;
+            Bb = Bt;
         }
     }
     const double Tr0 = exp(-OD), refl = 1.0 - eps;
@@ -1183,7 +1239,7 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
     float* Dp = MODE == 0 ? D + (size_t)p * jp.n_state * nn : nullptr;
     auto emit = [&](size_t x, double val) {  // D[x][nu] = val
         if (MODE == 0) {
-            Dp[x * nn + i] = (float)val;
+            if (valid) Dp[x * nn + i] = (float)val;
         } else if (MODE == 2) {
             double v = valid ? val * ib : 0.0;
 #pragma unroll
@@ -1192,20 +1248,25 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
         }
     };
     constexpr bool DERIV = MODE != 1;
-    double Bb, dBb;  // at the layer's bottom level: the top of the layer below
-    planck_grad64(c1nu3, nu, jy[0].c2b, jy[0].ib, Bb, dBb);
+    Bb = B0;
+    dBb = dB0;
     for (int m = 0; m < L; ++m) {
+        if (L > kJgRteChunk && m % kJgRteChunk == 0) fill(m);
+        if (m + 1 < L) {  // the loads are a layer's longest wait
+            const float* nx = out + (size_t)(m + 1) * n_out * nn + i;
+            for (int q = 0; q < (DERIV ? n_out : 1); ++q) asm volatile("prefetch.global.L1 [%0];" ::"l"(nx + q * nn));
+        }
         const JgRteLayer& r = jy[m];
         Cont c{};
-        if (mt) c = cont_at(r);
+        if (mt) c = cont_at(m, r);
         const double s = layer_s(m, r, c);
         cum += s;
         const double Tt = exp(-(OD - cum));  // transmittance from the top of layer m to space
         const double w = exp(-s), u = 1.0 - w;
         double e, dea, dTl_lo, dTl_hi, Ba = 0.0, dBa = 0.0, Bt, dBt, f, fp;
-        planck_grad64(c1nu3, nu, r.c2t, r.it, Bt, dBt);
+        planck_grad64_q(c1nu3, nu, r.c2t, r.it, q_at(m, r, 2), Bt, dBt);
         if (src == 0) {
-            planck_grad64(c1nu3, nu, r.c2a, r.ia, Ba, dBa);
+            planck_grad64_q(c1nu3, nu, r.c2a, r.ia, q_at(m, r, 1), Ba, dBa);
             cim_both(s, w, f, fp);
             const double core = Ba + (Bt - Ba) * f;
             e = u * core;
@@ -1258,13 +1319,12 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
             const double Gr = r.G * radfn_e(nu, c.x, c.e);
             if (jp.include_T) {
                 const double xp = c.x * r.rp, xm = c.x * r.rm;  // -x(T +- h) = -x + x - x r
-                const double ep = c.e * exp_small(c.x - xp), em = c.e * exp_small(c.x - xm);
-                const double Ep = (cont.mask & 1) ? c.E * exp_small(te * r.dp) : 0.0;
-                const double Em = (cont.mask & 1) ? c.E * exp_small(te * r.dm) : 0.0;
+                const double ep = fma(c.e, expm1_tiny(c.x - xp), c.e), em = fma(c.e, expm1_tiny(c.x - xm), c.e);
+                const double Ep = fma(c.E, expm1_tiny(te * r.dp), c.E), Em = fma(c.E, expm1_tiny(te * r.dm), c.E);
                 double Qp = c.Q, Qm = c.Q;
                 if ((cont.mask & 2) && td != 0.0) {
-                    Qp *= exp_small(-td * r.dp);
-                    Qm *= exp_small(-td * r.dm);
+                    Qp = fma(Qp, expm1_tiny(-td * r.dp), Qp);
+                    Qm = fma(Qm, expm1_tiny(-td * r.dm), Qm);
                 }
                 cT = (r.G * r.rp * radfn_e(nu, xp, ep) * cont_sum(r, Ep, Qp) -
                       r.G * r.rm * radfn_e(nu, xm, em) * cont_sum(r, Em, Qm)) * (1.0 / (2 * kJgRteDT));
@@ -1292,7 +1352,9 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
             emit((size_t)m, carryT + dTl_lo + dIdtau * tlo);
             carryT = dTl_hi + dIdtau * thi;
         }
-        for (int rr = 0; DERIV && rr < jp.n_retr; ++rr) {
+#pragma unroll
+        for (int rr = 0; rr < (DERIV ? 4 : 0); ++rr) {
+            if (rr >= jp.n_retr) break;
             const double cv = rr == jp.retr_h2o ? cvh : (rr == jp.retr_co2 ? cvc : 0.0);
             const double vlo = (double)om[(size_t)(3 + 2 * rr) * nn + i] + cv * (1.0 - r.wM);
             const double vhi = (double)om[(size_t)(4 + 2 * rr) * nn + i] + cv * r.wM;
@@ -1302,7 +1364,9 @@ __global__ void __launch_bounds__(128, CIA || MODE == 1 ? 1 : 6) jg_rte_kernel(
         }
     }
     if (DERIV && jp.include_T) emit((size_t)L, carryT);
-    for (int rr = 0; DERIV && rr < jp.n_retr; ++rr) {
+#pragma unroll
+    for (int rr = 0; rr < (DERIV ? 4 : 0); ++rr) {
+        if (rr >= jp.n_retr) break;
         const double sc = jp.log_vmr ? vl[rr * (L + 1) + L] : 1.0;
         emit((size_t)(nT + rr * (L + 1) + L), sc * carryV[rr]);
     }

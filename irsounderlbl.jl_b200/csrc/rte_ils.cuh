@@ -175,7 +175,7 @@ __device__ __forceinline__ double lit_w(double s, double w) {
 }
 // radfn (continuum.jl:169-174) with x = c2 nu / T and e = exp(-x)
 __device__ __forceinline__ double radfn_e(double nu, double x, double e) {
-    return x <= 0.01 ? 0.5 * x * nu : x <= 10.0 ? nu * (1.0 - e) * rcp64(1.0 + e) : nu;
+    return x <= 0.01 ? 0.5 * x * nu : x <= 10.0 ? nu * (1.0 - e) * rcp64_fast(1.0 + e) : nu;
 }
 // Interpolations.jl linear interpolation, Flat() extrapolation
 struct Lerp {
