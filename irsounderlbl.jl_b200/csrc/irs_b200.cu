@@ -1100,6 +1100,9 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             double* d_xb = (double*)workspace(ctx, "vjp_xbar", (size_t)np * n_state * sizeof(double));
             IRS_CUDA(cudaMemsetAsync(d_xb, 0, (size_t)np * n_state * sizeof(double), st));
             const size_t xsm = (size_t)n_state * sizeof(double);
+            if (xsm > 32 * 1024)  // beside the kernel's own 13 KB
+                for (const void* f : {(const void*)jg_rte_kernel<true, 2>, (const void*)jg_rte_kernel<false, 2>})
+                    IRS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsm));
             if (cia)
                 jg_rte_kernel<true, 2><<<gr, kJgRteThreads, xsm, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
                                                              n_nu, o.source_function, cd, d_I, nullptr, d_ib, d_xb);

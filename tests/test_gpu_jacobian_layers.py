@@ -39,3 +39,19 @@ def test_layers_and_ranges(pkg, ctx, oracle, orc_mod, src, nlev, nu0, dnu):
                     dict(nu_min=nu0, nu_max=nu0 + 6.0, dnu=0.5, opd_max=2.0, fwhm_gauss=0.5),
                     dict(apply_continuum=True, continua=("h2o",), with_ils=True, internal_dnu=dnu, source_function=src),
                     eps=0.9)
+
+
+def test_adjoint_with_a_long_state(pkg, ctx):
+    """The adjoint's sums of a state near the accepted 6,144 elements lie beside the tables in
+    shared memory: dx = K^T dy of irs_vjp_batch against K of irs_jacobian_batch (K rounded to
+    FP32 by column, 13 channels: 1e-6 of sum |K| |dy|, 2e-5 for the FP32 channel sums)."""
+    nlev = 3000
+    ll = {1: pkg.synthetic.synthetic_linelist(3, 1, 5, 700.0, 704.0)}
+    prof = profile(pkg, nlev, lambda p: {1: 0.01 * np.exp(-3.0 * (1000.0 - p) / 800.0)})
+    spec = pkg.StateVectorSpec(nlev, [1])
+    snd = pkg.Sounder.make(699.0, 705.0, 0.5, opd_max=2.0, fwhm_gauss=0.5)
+    kw = dict(sounder=snd, backend=ctx, internal_dnu=0.1, T_sfcs=[290.0], eps_sfcs=[0.98])
+    _, K, _ = pkg.analytic_jacobian_batch([prof], ll, spec, **kw)
+    dy = np.linspace(0.5, 1.5, K.shape[1])
+    _, dx = pkg.vjp_batch([prof], ll, spec, dy, **kw)
+    assert np.all(np.abs(dx[0] - dy @ K[0]) <= 2.1e-5 * (dy @ np.abs(K[0])) + 1e-12)
