@@ -208,6 +208,9 @@ int irs_state_size(const irs_state_spec* spec, int n_lev, int64_t* n_state);
  * ignored); transmittances and radiance derivatives are FP64. */
 int irs_jacobian_batch(irs_ctx* ctx, const irs_profile* profs, int n_prof, const irs_sounder* s,
                        const irs_fm_options* o, const irs_state_spec* spec, double* K, double* y);
+/* the same with K as [n_prof][n_channels][n_state] (row-major callers) */
+int irs_jacobian_batch_rows(irs_ctx* ctx, const irs_profile* profs, int n_prof, const irs_sounder* s,
+                            const irs_fm_options* o, const irs_state_spec* spec, double* K, double* y);
 
 /* forward_model for one batch spread over n_ctx contexts (one per GPU; every context
  * must hold the same line lists and tables).  No counterpart in the reference, whose

@@ -354,7 +354,7 @@ def sounder_grid(s: Sounder) -> np.ndarray:
     n_nu, n_ch = C.c_int64(), C.c_int64()
     o = fm_options(with_ils=False, high_res_factor=1)
     check(_lib.load().irs_grid_size(C.byref(s.c_struct()), C.byref(o), C.byref(n_nu), C.byref(n_ch)))
-    return np.array([s.nu_min + i * s.dnu for i in range(n_ch.value)])
+    return s.nu_min + np.arange(n_ch.value) * s.dnu
 
 
 def _prepare(ctx, linelists, line_mixing):

@@ -109,6 +109,8 @@ SIGNATURES = {
     "irs_state_size": ([C.POINTER(StateSpec), C.c_int, C.POINTER(C.c_int64)], C.c_int),
     "irs_jacobian_batch": ([_P, C.POINTER(Profile), C.c_int, C.POINTER(Sounder), C.POINTER(FMOptions),
                             C.POINTER(StateSpec), _PD, _PD], C.c_int),
+    "irs_jacobian_batch_rows": ([_P, C.POINTER(Profile), C.c_int, C.POINTER(Sounder), C.POINTER(FMOptions),
+                                 C.POINTER(StateSpec), _PD, _PD], C.c_int),
     "irs_vjp_batch": ([_P, C.POINTER(Profile), C.c_int, C.POINTER(Sounder), C.POINTER(FMOptions),
                        C.POINTER(StateSpec), _PD, _PD, _PD], C.c_int),
     "irs_oe_batch": ([_P, C.POINTER(Profile), C.c_int, C.POINTER(Sounder), C.POINTER(FMOptions),

@@ -834,16 +834,42 @@ static int64_t state_size(const irs_state_spec& sp, int n_lev) {
            (sp.include_emissivity ? 1 : 0);
 }
 
+// n floats on the device to host doubles, through two halves of a page-locked buffer that the
+// context keeps: the conversion of one half runs beside the copy of the next.  (A pageable copy
+// into a fresh vector, the conversion and the caller's transposition of K cost 16 scenes 2 of
+// their 8 ms.)
+constexpr size_t kPinHalf = (size_t)1 << 18;  // floats
+static void download_widened(irs_ctx* ctx, const float* d, size_t n, double* out) {
+    if (!ctx->pin) IRS_CUDA(cudaMallocHost((void**)&ctx->pin, 2 * kPinHalf * sizeof(float)));
+    auto copy = [&](size_t c) {
+        const size_t m = std::min(kPinHalf, n - c * kPinHalf);
+        IRS_CUDA(cudaMemcpyAsync(ctx->pin + (c & 1) * kPinHalf, d + c * kPinHalf, m * sizeof(float), cudaMemcpyDeviceToHost,
+                                 ctx->stream));
+        IRS_CUDA(cudaEventRecord(ctx->ev[9 + (c & 1)], ctx->stream));
+    };
+    const size_t nc = (n + kPinHalf - 1) / kPinHalf;
+    for (size_t c = 0; c < std::min<size_t>(nc, 2); ++c) copy(c);
+    for (size_t c = 0; c < nc; ++c) {
+        IRS_CUDA(cudaEventSynchronize(ctx->ev[9 + (c & 1)]));
+        const float* src = ctx->pin + (c & 1) * kPinHalf;
+        double* dst = out + c * kPinHalf;
+        const size_t m = std::min(kPinHalf, n - c * kPinHalf);
+        for (size_t k = 0; k < m; ++k) dst[k] = (double)src[k];
+        if (c + 2 < nc) copy(c + 2);
+    }
+}
+
 // vmr_jacobian.jl:152-505 for profiles [0, n_prof): K_h [n_prof][n_state][n_ch], y_h [n_prof][n_ch]
-// Outputs: host K_h/y_h (double), or with K_dev non-null the device K_dev (float
-// [n_prof][n_state][n_ch]) and host y_h.
+// (with rows, [n_prof][n_ch][n_state]).  Outputs: host K_h/y_h (double), or with K_dev non-null
+// the device K_dev (float [n_prof][n_state][n_ch]) and host y_h.
 // With dx_h non-null it computes the pullback dx = K^T dy instead (dy_h [n_prof][n_ch]
 // host, dx_h [n_prof][n_state] host): the derivative line sum as above, then I, R and
 // BT, the radiance cotangent on the grid by the transposed ILS, and one adjoint RTE sweep
 // that contracts each derivative term with it on the device; neither D nor K is formed.
 static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, const irs_sounder& s,
                             const irs_fm_options& o_in, const irs_state_spec& sp, double* K_h, double* y_h,
-                            float* K_dev = nullptr, const double* dy_h = nullptr, double* dx_h = nullptr) {
+                            float* K_dev = nullptr, const double* dy_h = nullptr, double* dx_h = nullptr,
+                            bool rows = false) {
     const bool adjoint = dx_h != nullptr;
     IRS_REQUIRE(n_prof >= 1 && profs, "need at least one profile");
     IRS_REQUIRE(sp.n_retrieved >= 0 && sp.n_retrieved <= 4 && (sp.n_retrieved == 0 || sp.retrieved),
@@ -887,7 +913,7 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
     const size_t per_prof = (size_t)L * total_lines * kJgLineBytes + (size_t)n_out * L * n_nu * 4 + (size_t)n_state * n_nu * 4 +
                             (size_t)n_nu * 8 + (size_t)n_state * n_ch * 4;
     const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
-    std::vector<float> Kf;
+    const long long k_state = rows ? 1 : n_ch, k_chan = rows ? n_state : 1;  // strides of K
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
         const int np = std::min(chunk, n_prof - p0);
         Plan pl;
@@ -1122,21 +1148,16 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
         if (cn.step)
             jg_channel_nodes_kernel<<<dim3((unsigned)((n_ch + kJgChan - 1) / kJgChan), (unsigned)((n_state + 1) / 2), np), kChanThreads,
                                       kJgChanSmem, st>>>(
-                d_D, (int)n_nu, (int)n_state, d_kernf, (int)n_taps, ig.dnu_hi, to_dev(ch), cn, d_RB, sp.observable, d_K);
+                d_D, (int)n_nu, (int)n_state, d_kernf, (int)n_taps, ig.dnu_hi, to_dev(ch), cn, d_RB, sp.observable, d_K, k_state, k_chan);
         else
             jg_channel_kernel<<<dim3((unsigned)((n_ch * 32 + 255) / 256), (unsigned)n_state, np), 256, 0, st>>>(
-                d_D, n_nu, (int)n_state, d_kernf ? d_kernf + kJgcPad : nullptr, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), o.with_ils, d_RB,
-                sp.observable, d_K);
+                d_D, n_nu, (int)n_state, d_kernf ? d_kernf + kJgcPad : nullptr, n_taps, ig.dnu_hi, to_dev(ig.g), to_dev(ch), o.with_ils,
+                d_RB, sp.observable, d_K, k_state, k_chan);
         check_launch(ctx);
-        if (!K_dev) {
-            Kf.resize((size_t)np * n_state * n_ch);
-            IRS_CUDA(cudaMemcpyAsync(Kf.data(), d_K, Kf.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
-        }
         IRS_CUDA(cudaMemcpyAsync(y_h + (size_t)p0 * n_ch, d_RB + (sp.observable == 0 ? (size_t)np * n_ch : 0),
                                  (size_t)np * n_ch * sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (!K_dev) download_widened(ctx, d_K, (size_t)np * n_state * n_ch, K_h + (size_t)p0 * n_state * n_ch);
         IRS_CUDA(cudaStreamSynchronize(st));
-        if (!K_dev)
-            for (size_t k = 0; k < Kf.size(); ++k) K_h[(size_t)p0 * n_state * n_ch + k] = (double)Kf[k];
     }
 }
 
@@ -1180,6 +1201,7 @@ static size_t device_budget(irs_ctx* ctx) {
 // Profiles per pass: bounded by device memory (60% of the budget) and by the grid
 // limits of the per-segment and per-(profile, layer) launches (65535 in y).
 static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof) {
+    if (n_prof == 1) return 1;  // whatever is free (asking takes 70 us, a scene 300)
     int n_lists = 0;
     for (auto& l : ctx->lists) n_lists += l.n > 0 ? 1 : 0;
     const size_t by_mem = std::max<size_t>(1, device_budget(ctx) * 6 / 10 / std::max<size_t>(per_prof, 1));
@@ -1414,10 +1436,17 @@ static void oe_batch(irs_ctx* ctx, const irs_profile* base, int n_scene, const i
         for (int64_t i = 0; i < n_ch; ++i) c += rbuf[i] * ws[i] * rbuf[i];
         std::vector<double> d(n);
         for (int i = 0; i < n; ++i) d[i] = xs[i] - xa[(size_t)sc * n + i];
-        for (int i = 0; i < n; ++i) {
-            double v = 0.0;
-            for (int j = 0; j < n; ++j) v += Sa_inv[(size_t)i * n + j] * d[j];
-            c += d[i] * v;
+        for (int i0 = 0; i0 < n; i0 += 8) {  // eight rows' sums beside each other, each in its order
+            const int m = std::min(8, n - i0);
+            const double* A = Sa_inv + (size_t)i0 * n;
+            double v[8] = {};
+            if (m == 8)
+                for (int j = 0; j < n; ++j)
+                    for (int q = 0; q < 8; ++q) v[q] += A[(size_t)q * n + j] * d[j];
+            else
+                for (int q = 0; q < m; ++q)
+                    for (int j = 0; j < n; ++j) v[q] += A[(size_t)q * n + j] * d[j];
+            for (int q = 0; q < m; ++q) c += d[i0 + q] * v[q];
         }
         return c;
     };
@@ -1427,10 +1456,12 @@ static void oe_batch(irs_ctx* ctx, const irs_profile* base, int n_scene, const i
         StateProfiles h;
         build_profiles(sp, list, x.data(), n, base, prm.eps_fixed, h);
         std::vector<double> y((size_t)list.size() * n_ch);
-        jacobian_device(ctx, h.prof.data(), (int)list.size(), s, o, sp, nullptr, y.data(), d_Kt);
+        // the first scenes in order: straight into their slots
+        const bool prefix = list.back() == (int)list.size() - 1 && std::is_sorted(list.begin(), list.end());
+        jacobian_device(ctx, h.prof.data(), (int)list.size(), s, o, sp, nullptr, y.data(), prefix ? d_K : d_Kt);
         for (size_t i = 0; i < list.size(); ++i) {
             const int sc = list[i];
-            if (sc != (int)i || d_Kt != d_K)
+            if (!prefix)
                 IRS_CUDA(cudaMemcpyAsync(d_K + (size_t)sc * n * n_ch, d_Kt + i * n * n_ch, (size_t)n * n_ch * sizeof(float),
                                          cudaMemcpyDeviceToDevice, st));
             std::copy(y.begin() + i * n_ch, y.begin() + (i + 1) * n_ch, F.begin() + (size_t)sc * n_ch);
@@ -1444,12 +1475,16 @@ static void oe_batch(irs_ctx* ctx, const irs_profile* base, int n_scene, const i
         }
     };
     auto upload_resid = [&](const std::vector<int>& list) {
-        std::vector<double> r((size_t)n_ch);
-        for (int sc : list) {
-            residual(sc, F.data() + (size_t)sc * n_ch, r.data());
-            IRS_CUDA(cudaMemcpyAsync(d_r + (size_t)sc * n_ch, r.data(), n_ch * sizeof(double), cudaMemcpyHostToDevice, st));
-            IRS_CUDA(cudaStreamSynchronize(st));
+        std::vector<double> r(list.size() * n_ch);
+        for (size_t i = 0; i < list.size();) {  // one copy per run of consecutive scenes
+            size_t e = i;
+            do residual(list[e], F.data() + (size_t)list[e] * n_ch, r.data() + e * n_ch);
+            while (++e < list.size() && list[e] == list[e - 1] + 1);
+            IRS_CUDA(cudaMemcpyAsync(d_r + (size_t)list[i] * n_ch, r.data() + i * n_ch, (e - i) * n_ch * sizeof(double),
+                                     cudaMemcpyHostToDevice, st));
+            i = e;
         }
+        IRS_CUDA(cudaStreamSynchronize(st));
     };
 
     std::vector<int> all(S);
@@ -1594,6 +1629,7 @@ int irs_destroy(irs_ctx* ctx) {
         cudaFree(l.nu);  // one allocation per list (see irs_upload_linelist)
     }
     for (auto& w : ctx->work) if (w.second.p) cudaFree(w.second.p);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     for (auto& e : ctx->ev) cudaEventDestroy(e);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -1896,6 +1932,15 @@ int irs_jacobian_batch(irs_ctx* ctx, const irs_profile* profs, int n_prof, const
     IRS_REQUIRE(ctx && s && o && spec && K && y, "invalid arguments");
     IRS_CUDA(cudaSetDevice(ctx->device));
     jacobian_device(ctx, profs, n_prof, *s, *o, *spec, K, y);
+    IRS_API_END
+}
+
+int irs_jacobian_batch_rows(irs_ctx* ctx, const irs_profile* profs, int n_prof, const irs_sounder* s,
+                            const irs_fm_options* o, const irs_state_spec* spec, double* K, double* y) {
+    IRS_API_BEGIN
+    IRS_REQUIRE(ctx && s && o && spec && K && y, "invalid arguments");
+    IRS_CUDA(cudaSetDevice(ctx->device));
+    jacobian_device(ctx, profs, n_prof, *s, *o, *spec, K, y, nullptr, nullptr, nullptr, true);
     IRS_API_END
 }
 

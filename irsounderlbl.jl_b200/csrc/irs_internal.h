@@ -162,7 +162,8 @@ void lm_poles(const RelmatHost& R, const Tables& tabs, int mode, uint32_t iso_ma
 struct irs_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev[10] = {};
+    cudaEvent_t ev[11] = {};
+    float* pin = nullptr;  // page-locked halves of download_widened
     irs::Tables tables;
     bool tips_dirty = true, cont_dirty = true;
     // device copies of tables

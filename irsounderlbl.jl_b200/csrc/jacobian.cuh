@@ -1388,7 +1388,7 @@ __device__ __forceinline__ double dbt_dr(double nu, double R) {  // vmr_jacobian
     return 1.4387769 * nu * A / ((Lg * Lg) * R * (R + A));
 }
 
-// K[x][c] = dBT/dR_c * resample(ILS(D[x]))_c, vmr_jacobian.jl:359-380.  One warp per
+// K[x][c] = dBT/dR_c * resample(ILS(D[x]))_c (strides k_state, k_chan), vmr_jacobian.jl:359-380.  One warp per
 // (state element, channel); the ILS taps (kernf: the normalised FP64 taps rounded to
 // FP32) run over lanes (FP32 products, FP32 sums).  A window that lies inside the grid,
 // as it does for every channel away from the padded ends, needs no per-tap bounds test.
@@ -1396,7 +1396,7 @@ __global__ void __launch_bounds__(256) jg_channel_kernel(const float* __restrict
                                                          const float* __restrict__ kernf, long long n_taps,
                                                          double dnu_hi, GridDev g, GridDev ch, int with_ils,
                                                          const double* __restrict__ R, int observable,
-                                                         float* __restrict__ K) {
+                                                         float* __restrict__ K, long long k_state, long long k_chan) {
     const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int x = blockIdx.y, p = blockIdx.z;
@@ -1437,7 +1437,7 @@ __global__ void __launch_bounds__(256) jg_channel_kernel(const float* __restrict
     if (lane == 0) {
         double scale = 1.0;
         if (observable == 0) scale = dbt_dr(nu, R[(size_t)p * ch.n + wid]);
-        K[((size_t)p * n_state + x) * ch.n + wid] = (float)(v * scale);
+        K[(size_t)p * n_state * ch.n + x * k_state + wid * k_chan] = (float)(v * scale);
     }
 }
 
@@ -1464,7 +1464,8 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool in)
 }
 __global__ void __launch_bounds__(kChanThreads, 3) jg_channel_nodes_kernel(
     const float* __restrict__ D, int n_nu, int n_state, const float* __restrict__ kernf, int n_taps, double dnu_hi,
-    GridDev ch, ChanNodes nodes, const double* __restrict__ R, int observable, float* __restrict__ K) {
+    GridDev ch, ChanNodes nodes, const double* __restrict__ R, int observable, float* __restrict__ K, long long k_state,
+    long long k_chan) {
     constexpr int C = kJgChan;
     extern __shared__ float jgc_smem[];
     float(*slot)[3][kChanThreads] = reinterpret_cast<float(*)[3][kChanThreads]>(jgc_smem);
@@ -1554,7 +1555,7 @@ __global__ void __launch_bounds__(kChanThreads, 3) jg_channel_nodes_kernel(
         for (int w = 0; w < kChanThreads / 32; ++w) s += part[w][threadIdx.x];
         double scale = 1.0;
         if (observable == 0) scale = dbt_dr(ch.at(c), R[(size_t)p * ch.n + c]);
-        K[((size_t)p * n_state + x) * ch.n + c] = (float)((double)s * dnu_hi * scale);
+        K[(size_t)p * n_state * ch.n + x * k_state + c * k_chan] = (float)((double)s * dnu_hi * scale);
     }
 }
 

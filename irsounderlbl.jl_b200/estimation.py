@@ -404,11 +404,10 @@ def analytic_jacobian_batch(profiles, linelists, spec: StateVectorSpec, *, sound
     nu = sounder_grid(sounder)
     n_full = C.c_int64()
     check(ctx.lib.irs_state_size(C.byref(cs), spec.n_levels, C.byref(n_full)))
-    Kc = np.empty((n, n_full.value, len(nu)))
+    K = np.empty((n, len(nu), n_full.value))
     y = np.empty((n, len(nu)))
-    check(ctx.lib.irs_jacobian_batch(ctx.h, batch.arr, n, C.byref(s), C.byref(o), C.byref(cs), dptr(Kc),
-                                     dptr(y)))
-    K = np.ascontiguousarray(np.transpose(Kc, (0, 2, 1)))  # [n_prof, n_ch, n_full]
+    check(ctx.lib.irs_jacobian_batch_rows(ctx.h, batch.arr, n, C.byref(s), C.byref(o), C.byref(cs), dptr(K),
+                                          dptr(y)))
     if reduced:
         K = _map_reduced(spec, K, profiles)
     return nu, K, y
