@@ -840,10 +840,15 @@ static int64_t state_size(const irs_state_spec& sp, int n_lev) {
 // their 8 ms.)
 constexpr size_t kPinHalf = (size_t)1 << 18;  // floats
 static void download_widened(irs_ctx* ctx, const float* d, size_t n, double* out) {
-    if (!ctx->pin) IRS_CUDA(cudaMallocHost((void**)&ctx->pin, 2 * kPinHalf * sizeof(float)));
+    if (!ctx->pin && cudaMallocHost((void**)&ctx->pin, 2 * kPinHalf * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pin = nullptr;
+    }
+    std::vector<float> pageable(ctx->pin ? 0 : 2 * kPinHalf);  // where none can be page-locked
+    float* buf = ctx->pin ? ctx->pin : pageable.data();
     auto copy = [&](size_t c) {
         const size_t m = std::min(kPinHalf, n - c * kPinHalf);
-        IRS_CUDA(cudaMemcpyAsync(ctx->pin + (c & 1) * kPinHalf, d + c * kPinHalf, m * sizeof(float), cudaMemcpyDeviceToHost,
+        IRS_CUDA(cudaMemcpyAsync(buf + (c & 1) * kPinHalf, d + c * kPinHalf, m * sizeof(float), cudaMemcpyDeviceToHost,
                                  ctx->stream));
         IRS_CUDA(cudaEventRecord(ctx->ev[9 + (c & 1)], ctx->stream));
     };
@@ -851,7 +856,7 @@ static void download_widened(irs_ctx* ctx, const float* d, size_t n, double* out
     for (size_t c = 0; c < std::min<size_t>(nc, 2); ++c) copy(c);
     for (size_t c = 0; c < nc; ++c) {
         IRS_CUDA(cudaEventSynchronize(ctx->ev[9 + (c & 1)]));
-        const float* src = ctx->pin + (c & 1) * kPinHalf;
+        const float* src = buf + (c & 1) * kPinHalf;
         double* dst = out + c * kPinHalf;
         const size_t m = std::min(kPinHalf, n - c * kPinHalf);
         for (size_t k = 0; k < m; ++k) dst[k] = (double)src[k];
