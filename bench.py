@@ -130,8 +130,8 @@ def _physical_gpu(local_rank: int) -> int:
 
 
 def _traffic_from_profiles():
-    """DRAM bytes per launch of the line-sum kernel from the committed ncu summary."""
-    p = ROOT / "profiles" / "linesum_mixed_iasi400k.txt"
+    """DRAM bytes of a step's line-sum launches from the committed ncu summary."""
+    p = ROOT / "profiles" / "linesum_iasi400k.txt"
     if not p.exists():
         return None
     for line in p.read_text().splitlines():
@@ -616,7 +616,7 @@ def main():
     launches_per_step = st.launches
     t_ls = acc["line_sum_ms"] / 1e3
     # FLOPs of the pair evaluations the kernel issued: near lines at every block point,
-    # far lines at the 8 interpolation nodes (the algorithmic pair count is larger)
+    # far lines at their blocks' 16 nodes (the algorithmic pair count is larger)
     flops = FAR_PAIR_FLOPS * (evald - core) + CORE_PAIR_FLOPS * core
     clocks = clk.summary()
     f_sm = (clocks["sm_mhz"] or 1965.0) * 1e6
@@ -688,7 +688,7 @@ def main():
             "config": workload_config(),
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "linesum_mixed_kernel<3>",
+                         "kernel": "fw_leaf_kernel<3> and fw_tree_warp_kernel",
                          "algorithmic_pairs_per_s": pairs / t_ls,
                          "peak_source": "148 SMs x 128 FP32 lanes x 2 FLOP x median sampled SM clock "
                                         "(MEASURED_PEAKS.json has no FP32 figure)",
