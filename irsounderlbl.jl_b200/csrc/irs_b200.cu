@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <numeric>
 #include <vector>
@@ -827,7 +828,7 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
 }
 
 // ------------------------------------------------------------ Jacobian
-static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof);
+static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, std::initializer_list<const char*> mine);
 
 static int64_t state_size(const irs_state_spec& sp, int n_lev) {
     return (sp.include_temperature ? n_lev : 0) + (int64_t)sp.n_retrieved * n_lev + (sp.include_tsfc ? 1 : 0) +
@@ -917,7 +918,7 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
     for (auto& l : ctx->lists) total_lines += l.n;
     const size_t per_prof = (size_t)L * total_lines * kJgLineBytes + (size_t)n_out * L * n_nu * 4 + (size_t)n_state * n_nu * 4 +
                             (size_t)n_nu * 8 + (size_t)n_state * n_ch * 4;
-    const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
+    const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof, {"jg_params", "jg_out", "jg_D", "jg_K", "jg_far", "I"});
     const long long k_state = rows ? 1 : n_ch, k_chan = rows ? n_state : 1;  // strides of K
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
         const int np = std::min(chunk, n_prof - p0);
@@ -1193,23 +1194,22 @@ static void collect_times(irs_ctx* ctx) {
     ctx->last.lm_host_ms = ctx->lm_host_pass + ctx->prior.lm_host_ms;
 }
 
-// Device bytes the library may use: what is free plus its own workspaces (reused or
-// grown in place).
-static size_t device_budget(irs_ctx* ctx) {
-    size_t free_b = 0, tot_b = 0;
-    IRS_CUDA(cudaMemGetInfo(&free_b, &tot_b));
-    size_t own = 0;
-    for (auto& w : ctx->work) own += w.second.bytes;
-    return free_b + own;
-}
-
-// Profiles per pass: bounded by device memory (60% of the budget) and by the grid
-// limits of the per-segment and per-(profile, layer) launches (65535 in y).
-static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof) {
+// Profiles per pass: bounded by device memory and by the grid limits of the per-segment and
+// per-(profile, layer) launches (65535 in y).  Memory: 60% of what is free plus the context's
+// own workspaces, and 80% of what is free plus those that this pass reuses (`mine`; what
+// another path's batch left behind stays with it).
+static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, std::initializer_list<const char*> mine) {
     if (n_prof == 1) return 1;  // whatever is free (asking takes 70 us, a scene 300)
     int n_lists = 0;
     for (auto& l : ctx->lists) n_lists += l.n > 0 ? 1 : 0;
-    const size_t by_mem = std::max<size_t>(1, device_budget(ctx) * 6 / 10 / std::max<size_t>(per_prof, 1));
+    size_t free_b = 0, tot_b = 0, own = 0, reuse = 0;
+    IRS_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+    for (auto& w : ctx->work) {
+        own += w.second.bytes;
+        for (const char* m : mine) reuse += w.first == m ? w.second.bytes : 0;
+    }
+    const size_t bytes = std::min((free_b + own) * 6 / 10, (free_b + reuse) * 8 / 10);
+    const size_t by_mem = std::max<size_t>(1, bytes / std::max<size_t>(per_prof, 1));
     const size_t by_grid = std::max<size_t>(1, 65535 / (size_t)std::max(1, L * std::max(n_lists, 1)));
     return (int)std::min<size_t>((size_t)n_prof, std::min(by_mem, by_grid));
 }
@@ -1233,7 +1233,8 @@ static void forward_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, c
     const bool mixed = o.precision != IRS_FP64;
     const size_t per_prof = (size_t)L * total_lines * (mixed ? 1 + kLpMixedBytes : 1 + kLpF64 * sizeof(double)) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
                             (size_t)ig.g.n * 8;
-    const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof);
+    const int chunk = mixed ? profiles_per_pass(ctx, n_prof, L, per_prof, {"tau", "lpmx", "keep", "I", "fw_far", "fw_cell_idx"})
+                            : profiles_per_pass(ctx, n_prof, L, per_prof, {"tau", "lp64", "keep", "I", "t64_far"});
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
         const int np = std::min(chunk, n_prof - p0);
         forward_pass(ctx, profs + p0, np, s, o, d_R + (size_t)p0 * ch.n, d_BT + (size_t)p0 * ch.n);
