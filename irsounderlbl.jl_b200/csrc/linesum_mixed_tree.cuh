@@ -495,7 +495,12 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
                     nn.y = cy ? nn.y : 1.f;
                     q.x = cx ? q.x : 1.f;
                     q.y = cy ? q.y : 1.f;
-                    const float2 den = __fmul2_rn(m, q);
+                    // m q is zero where y is lost beside x = 0 or x^2 = 3/2: points that the buffer
+                    // replaces below, but the reciprocal is their neighbours' too.  Beyond those
+                    // points it is above 1 (1e-8 with x_far = 0)
+                    float2 den = __fmul2_rn(m, q);
+                    den.x = fmaxf(den.x, 1e-18f);
+                    den.y = fmaxf(den.y, 1e-18f);
                     const float R = rcp_fast(den.x * den.y);
                     const float2 r = __fmul2_rn(make_float2(den.y, den.x), make_float2(R, R));
                     float2 v = __fmul2_rn(__fmul2_rn(nn, make_float2(p.z, p.z)), r), vd = make_float2(0.f, 0.f);
