@@ -223,7 +223,9 @@ __device__ __forceinline__ void jg_wing_coeffs(const float4& a0, const float4& a
     const float ifx = rcp_fast(fx);
     const float gg = ifx * ifx, b2 = y * y * gg, Aky = An * k * y, Akg = An * k * gg;
     const float r_fx = fxT * ifx;
-    f0 = make_float4(0.f, 0.f, b2, Aky * gg);
+    // floored: at a centre on a grid point an unbroadened line's d^2 + b2 would be 0, and the
+    // reciprocal is shared with another point (jg_offsets)
+    f0 = make_float4(0.f, 0.f, fmaxf(b2, 1e-18f), Aky * gg);
     f1 = make_float4(gg * k * (AnT * y + An * yT) - 2.f * Aky * r_fx * gg, 2.f * Aky * b2 * r_fx * gg - 2.f * Akg * yT * b2,
                      0.f, 0.f);
     P[0] = An * Hc;
