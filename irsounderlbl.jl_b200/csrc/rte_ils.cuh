@@ -166,6 +166,7 @@ __device__ __forceinline__ double planck64(double c1nu3, double nu, double c2T) 
 // _cim_correction (schwarzschild.jl:59-63) and _lit_correction (:43-47) with w = exp(-s)
 __device__ __forceinline__ double cim_w(double s, double w) {
     if (s < 0.06) return s / 6.0;
+    if (s > 1e17) return 1.0;  // 2/s is rounded away (s * r would be inf * 0 at s = inf)
     const double a = w - 1.0, r = rcp64(s * a);  // 1/s = a r, 1/(w - 1) = s r
     return 1.0 - 2.0 * fma(w, s * r, a * r);
 }
