@@ -525,6 +525,8 @@ static void ensure_ils(irs_ctx* ctx, double dnu, double opd, double fwhm, int ap
 static ChanNodes chan_nodes(const GridSpec& g, const GridSpec& ch) {
     ChanNodes c{0, 0};
     if (!g.den || !ch.den || g.n >= ((int64_t)1 << 30)) return c;
+    for (double v : {g.a_n, g.s_n, ch.a_n, ch.s_n})  // rounded numerators: nothing to compare (nor to convert)
+        if (std::fabs(v) > 9007199254740992.0) return c;
     const __int128 gs = (__int128)(int64_t)g.s_n * ch.den, cs = (__int128)(int64_t)ch.s_n * g.den;
     const __int128 off = (__int128)(int64_t)ch.a_n * g.den - (__int128)(int64_t)g.a_n * ch.den;
     if (gs <= 0 || cs % gs != 0 || off < 0 || off % gs != 0) return c;
