@@ -806,11 +806,14 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
     }
     if (o.precision != IRS_FP64) {
         const size_t sm = (size_t)L * sizeof(RteLayerF);
-        IRS_REQUIRE(sm <= 200 * 1024, "too many layers for the RTE kernel (at most 4266)");
+        // (function attributes are the device's: limits, not this call's sizes, since another
+        // context's call may set them between here and the launch)
+        constexpr int kRteSmemMax = 200 * 1024;
+        IRS_REQUIRE(sm <= kRteSmemMax, "too many layers for the RTE kernel (at most 4266)");
 #define IRS_RTE(G, CIA)                                                                                                \
     do {                                                                                                               \
         if (sm > 32 * 1024) /* beside the kernel's own 16 KB */                                                        \
-            IRS_CUDA(cudaFuncSetAttribute(rte_mixed_kernel<G, CIA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+            IRS_CUDA(cudaFuncSetAttribute(rte_mixed_kernel<G, CIA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRteSmemMax)); \
         rte_mixed_kernel<G, CIA><<<dim3((unsigned)((n_nu + RteShape<G>::points - 1) / RteShape<G>::points), n_prof), kRteThreads, sm, st>>>( \
             (const float*)d_tau, d_lrt, d_prt, L, d_grid, n_nu, o.source_function, cd, d_I);                           \
     } while (0)
@@ -866,6 +869,8 @@ static void download_widened(irs_ctx* ctx, const float* d, size_t n, double* out
         if (c + 2 < nc) copy(c + 2);
     }
 }
+
+constexpr int kVjpStateBytes = 48 * 1024;  // of the adjoint's state in shared memory
 
 // vmr_jacobian.jl:152-505 for profiles [0, n_prof): K_h [n_prof][n_state][n_ch], y_h [n_prof][n_ch]
 // (with rows, [n_prof][n_ch][n_state]).  Outputs: host K_h/y_h (double), or with K_dev non-null
@@ -1075,7 +1080,7 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
 #define IRS_JGK(MODE)                                                                                                  \
     if (modes >> MODE & 1u) {                                                                                          \
         const size_t sm = jg_smem_bytes(MODE >= kJgLm2, n_out);                                                        \
-        IRS_CUDA(cudaFuncSetAttribute(jg_linesum_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+        IRS_CUDA(cudaFuncSetAttribute(jg_linesum_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jg_smem_bytes(MODE >= kJgLm2, kJgMaxOut))); \
         jg_linesum_kernel<MODE><<<g2, kJgWarps * 32, sm, st>>>(d_segs, d_sw, d_pl, ci, go, n_nu, cut_g, n_out, store, jg_sums(lm), \
                                                                d_out, d_pert, pstride, d_tab, d_far, d_rng, n_leaves, pa, s_a);    \
         check_launch(ctx);                                                                                             \
@@ -1136,7 +1141,7 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             const size_t xsm = (size_t)n_state * sizeof(double);
             if (xsm > 32 * 1024)  // beside the kernel's own 13 KB
                 for (const void* f : {(const void*)jg_rte_kernel<true, 2>, (const void*)jg_rte_kernel<false, 2>})
-                    IRS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsm));
+                    IRS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpStateBytes));
             if (cia)
                 jg_rte_kernel<true, 2><<<gr, kJgRteThreads, xsm, st>>>(d_out, n_out, d_lrt, d_jrl, d_prt, d_jp, d_vlev, L, d_grid,
                                                              n_nu, o.source_function, cd, d_I, nullptr, d_ib, d_xb);
@@ -1958,7 +1963,7 @@ int irs_vjp_batch(irs_ctx* ctx, const irs_profile* profs, int n_prof, const irs_
     IRS_API_BEGIN
     IRS_REQUIRE(ctx && s && o && spec && dy && dx && y && profs && n_prof >= 1, "invalid arguments");
     IRS_CUDA(cudaSetDevice(ctx->device));
-    IRS_REQUIRE(state_size(*spec, profs[0].n_lev) * sizeof(double) <= 48 * 1024, "state vector too long for the adjoint");
+    IRS_REQUIRE(state_size(*spec, profs[0].n_lev) * sizeof(double) <= kVjpStateBytes, "state vector too long for the adjoint");
     jacobian_device(ctx, profs, n_prof, *s, *o, *spec, nullptr, y, nullptr, dy, dx);
     IRS_API_END
 }
