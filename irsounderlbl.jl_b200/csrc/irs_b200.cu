@@ -216,16 +216,26 @@ static CellIndex cell_index(irs_ctx* ctx, const double* d_V, const std::vector<l
     ci.idx = d_idx;
     return ci;
 }
-static const TreeTables* tree_tables(irs_ctx* ctx) {
-    const bool have = ctx->work.count("tree32") != 0;
-    TreeTables* d = (TreeTables*)workspace(ctx, "tree32", sizeof(TreeTables));
-    if (!have) {
-        std::unique_ptr<TreeTables> h(new TreeTables);
-        tree32_tables(&h->M[0][0][0], &h->L[0][0]);
-        IRS_CUDA(cudaMemcpyAsync(d, h.get(), sizeof(TreeTables), cudaMemcpyHostToDevice, ctx->stream));
-        IRS_CUDA(cudaStreamSynchronize(ctx->stream));
+// A constant table of the context, made and uploaded by its first user.  It counts as there once
+// the copy has succeeded: after a failed allocation or copy the next call starts over.
+template <typename T, typename F>
+static const T* device_table(irs_ctx* ctx, const std::string& name, F&& fill) {
+    const auto it = ctx->work.find(name);
+    if (it != ctx->work.end() && it->second.p) return (const T*)it->second.p;
+    std::unique_ptr<T> h(new T);
+    fill(*h);
+    T* d = (T*)workspace(ctx, name, sizeof(T));
+    cudaError_t e = cudaMemcpyAsync(d, h.get(), sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) {
+        cudaFree(d);
+        ctx->work.erase(name);
+        IRS_CUDA(e);
     }
     return d;
+}
+static const TreeTables* tree_tables(irs_ctx* ctx) {
+    return device_table<TreeTables>(ctx, "tree32", [](TreeTables& t) { tree32_tables(&t.M[0][0][0], &t.L[0][0]); });
 }
 
 // tree64: points per leaf (one warp).  128 points cost the least per point, but a short
@@ -250,14 +260,7 @@ static void tree64_launch(irs_ctx* ctx, const Plan& pl, const std::vector<int>& 
                           const int* d_uniform) {
     static_assert(sizeof(T64Tables) == kT64TableDoubles * sizeof(double), "table layout");
     cudaStream_t st = ctx->stream;
-    const bool have = ctx->work.count("t64_tables") != 0;
-    T64Tables* d_tab = (T64Tables*)workspace(ctx, "t64_tables", sizeof(T64Tables));
-    if (!have) {
-        std::vector<double> h(kT64TableDoubles);
-        t64_tables(h.data());
-        IRS_CUDA(cudaMemcpyAsync(d_tab, h.data(), sizeof(T64Tables), cudaMemcpyHostToDevice, st));
-        IRS_CUDA(cudaStreamSynchronize(st));
-    }
+    const T64Tables* d_tab = device_table<T64Tables>(ctx, "t64_tables", [](T64Tables& t) { t64_tables((double*)&t); });
     const bool lm = o.line_mixing == IRS_LM_PER_LINE_Y;
     const int npl = pl.n_prof * pl.L, leaf = t64_leaf_points(n_nu, pl.L);
     const int n_groups = (int)t64_groups(n_nu, leaf);
@@ -311,6 +314,7 @@ static void mixed_tree_launch(irs_ctx* ctx, const Plan& pl, const std::vector<in
                               int64_t n_nu, float cut_g, const irs_fm_options& o, float* d_tau, double* d_pert,
                               long long pstride, unsigned long long* d_eval) {
     cudaStream_t st = ctx->stream;
+    const TreeTables* d_tab = tree_tables(ctx);
     const int npl = pl.n_prof * pl.L, nseg = first[npl];
     double margin = 0.0;
     int any[2] = {0, 0};  // segments without and with per-line mixing
@@ -326,7 +330,6 @@ static void mixed_tree_launch(irs_ctx* ctx, const Plan& pl, const std::vector<in
     cell_fill_kernel<<<dim3((unsigned)(pl.max_list / 256 + 1), nseg), 256, 0, st>>>(d_segs, d_count, om.V, ci.n, 1.0 / cell,
                                                                                    off, d_idx);
     check_launch(ctx);
-    const TreeTables* d_tab = tree_tables(ctx);
     const int n_leaves = (int)tree_leaves(n_nu);
     const size_t cell_bytes = fw_cell_bytes(lm);
     const size_t max_cells = std::min((size_t)nseg * n_leaves, ctx->strip_buf_max / cell_bytes);
