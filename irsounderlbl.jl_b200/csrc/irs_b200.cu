@@ -509,6 +509,7 @@ static void ensure_ils(irs_ctx* ctx, double dnu, double opd, double fwhm, int ap
     if (std::memcmp(key, ctx->ils_key, sizeof key) == 0) return;
     const int64_t n_half = (int64_t)std::ceil(16.0 / dnu);
     const int64_t n = 2 * n_half + 1;
+    ctx->ils_key[0] = -1;  // nothing is cached until the new taps are there (an allocation may fail)
     double* k = (double*)workspace(ctx, "ils", n * sizeof(double));
     ils_taps_kernel<<<(unsigned)((n + 127) / 128), 128, 0, ctx->stream>>>(dnu, opd, fwhm, apod, n_half, k);
     check_launch(ctx);

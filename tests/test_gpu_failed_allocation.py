@@ -47,3 +47,22 @@ def test_tables_after_a_failed_allocation(precision):
             call(c, pkg.FullFaddeeva)
     assert np.array_equal(call(c, pkg.FullFaddeeva), ref)
     c.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_ils_after_a_failed_allocation(precision):
+    """A second sounder with more taps but a shorter grid: its ILS is the allocation that fails.
+    The first sounder's taps are made anew."""
+    pkg = load_package()
+    lists = {2: pkg.synthetic.synthetic_linelist(300, 2, 83, 700.0, 800.0)}
+    prof = pkg.afgl_atmosphere("us_standard")
+    snd = [pkg.Sounder.make(lo, hi, 0.25, opd_max=2.0, fwhm_gauss=0.5) for lo, hi in ((700.0, 1000.0), (750.0, 750.25))]
+    c = pkg.B200Context()
+    call = lambda k: pkg.forward_model(prof, lists, sounder=snd[k], backend=c, precision=precision,
+                                       internal_dnu=(0.0025, 0.001)[k], apply_continuum=False)[2]
+    ref = call(0)
+    with full_device():
+        with pytest.raises(pkg.IRSError, match=r"allocation of .* \(ils\)"):
+            call(1)
+    assert np.array_equal(call(0), ref)
+    c.close()
