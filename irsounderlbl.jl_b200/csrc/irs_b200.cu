@@ -216,6 +216,20 @@ static CellIndex cell_index(irs_ctx* ctx, const double* d_V, const std::vector<l
     ci.idx = d_idx;
     return ci;
 }
+// The far field's buffer, node values of up to `cells` cells: how many it holds.  No more than
+// ctx->strip_buf_max, and where the device has less left, half as often as it takes (the line sum
+// then takes more groups of profile-layers).
+static size_t far_cells(irs_ctx* ctx, const std::string& name, size_t cells, size_t cell_bytes) {
+    for (size_t c = std::min(cells, ctx->strip_buf_max / cell_bytes);; c /= 2) {
+        try {
+            workspace(ctx, name, c * cell_bytes);
+            return c;
+        } catch (const Error& e) {
+            if (e.code != IRS_E_NOMEM || c == 0) throw;
+        }
+    }
+}
+
 // A constant table of the context, made and uploaded by its first user.  It counts as there once
 // the copy has succeeded: after a failed allocation or copy the next call starts over.
 template <typename T, typename F>
@@ -265,8 +279,8 @@ static void tree64_launch(irs_ctx* ctx, const Plan& pl, const std::vector<int>& 
     const int npl = pl.n_prof * pl.L, leaf = t64_leaf_points(n_nu, pl.L);
     const int n_groups = (int)t64_groups(n_nu, leaf);
     const size_t cell_bytes = t64_cell_bytes(lm);
-    const size_t max_cells = std::min((size_t)first[npl] * n_groups, ctx->strip_buf_max / cell_bytes);
-    char* buf = (char*)workspace(ctx, "t64_far", max_cells * cell_bytes);
+    const size_t max_cells = far_cells(ctx, "t64_far", (size_t)first[npl] * n_groups, cell_bytes);
+    char* buf = (char*)ctx->work["t64_far"].p;
     for (int pa = 0; pa < npl;) {
         int pb = pa;
         const int s_a = first[pa];
@@ -302,8 +316,9 @@ static void tree64_launch(irs_ctx* ctx, const Plan& pl, const std::vector<int>& 
     }
 }
 
-// bytes of one (segment, leaf) cell of the FP32 forward far field
+// bytes of one (segment, leaf) cell of the FP32 far fields, forward and Jacobian
 static size_t fw_cell_bytes(bool lm) { return fw_sums(lm) * kTrNodes * sizeof(float) + sizeof(int4); }
+static size_t jg_cell_bytes(bool lm) { return (size_t)jg_sums(lm) * kTrNodes * sizeof(float) + sizeof(int4); }
 
 // The FP32 line sum of IRS_MIXED (linesum_mixed_tree.cuh): the cell index of the kept lines,
 // the far field's node values and the leaf kernels, in groups of profile-layers (their
@@ -332,8 +347,8 @@ static void mixed_tree_launch(irs_ctx* ctx, const Plan& pl, const std::vector<in
     check_launch(ctx);
     const int n_leaves = (int)tree_leaves(n_nu);
     const size_t cell_bytes = fw_cell_bytes(lm);
-    const size_t max_cells = std::min((size_t)nseg * n_leaves, ctx->strip_buf_max / cell_bytes);
-    char* buf = (char*)workspace(ctx, "fw_far", max_cells * cell_bytes);
+    const size_t max_cells = far_cells(ctx, "fw_far", (size_t)nseg * n_leaves, cell_bytes);
+    char* buf = (char*)ctx->work["fw_far"].p;
     // one warp or eight per (strip, segment): by the strips of one profile's segments (not the
     // batch's, so that a profile's result does not depend on it).  From 16 warps per SM on, one
     // warp is the cheaper; 9 strips x 49 segments would leave it three warps per SM, where
@@ -742,17 +757,10 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
             workspace(ctx, "chunk_count", sizeof(int) * (size_t)nseg * ((max_list + lc - 1) / lc));
         }
         workspace(ctx, "seg_count", sizeof(int) * nseg);
-        if (o.precision == IRS_MIXED && o.method != IRS_PSEUDOVOIGT) {  // the far field's buffers
-            const size_t cb = fw_cell_bytes(o.line_mixing == IRS_LM_PER_LINE_Y);
-            workspace(ctx, "fw_far", std::min((size_t)nseg * tree_leaves(n_nu), ctx->strip_buf_max / cb) * cb);
+        if (o.precision == IRS_MIXED && o.method != IRS_PSEUDOVOIGT) {
             double margin = 0.0, cell, off;
             for (auto& g : pl.segs) margin = std::max(margin, g.margin_g);
             workspace(ctx, "fw_cell_idx", (size_t)nseg * cell_layout(n_nu, o.cutoff / ig.dnu_hi + margin, cell, off).n * sizeof(int));
-        }
-        if (!mixed && o.method != IRS_PSEUDOVOIGT) {
-            const size_t cb = t64_cell_bytes(o.line_mixing == IRS_LM_PER_LINE_Y);
-            const size_t cells = (size_t)nseg * t64_groups(n_nu, t64_leaf_points(n_nu, L));
-            workspace(ctx, "t64_far", std::min(cells, ctx->strip_buf_max / cb) * cb);
         }
         workspace(ctx, "core_reach", sizeof(unsigned) * nseg);
         workspace(ctx, "lrt", std::max<size_t>(lrt.size(), 1) * sizeof(LayerRT));
@@ -775,6 +783,12 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
         workspace(ctx, "lm_sv", (size_t)n_prof * L * pstride * sizeof(double));
         workspace(ctx, "lm_coef", coef_pl.size() * sizeof(double));
         workspace(ctx, "lm_off", ((size_t)n_prof * L + 1) * sizeof(long long));
+    }
+    if (o.method != IRS_PSEUDOVOIGT && o.precision != IRS_MIXED_DIRECT) {  // the far field's buffer last: it yields
+        const size_t nseg = std::max<size_t>(pl.segs.size(), 1);
+        const bool lm = o.line_mixing == IRS_LM_PER_LINE_Y;
+        if (o.precision == IRS_MIXED) far_cells(ctx, "fw_far", nseg * tree_leaves(n_nu), fw_cell_bytes(lm));
+        else far_cells(ctx, "t64_far", nseg * t64_groups(n_nu, t64_leaf_points(n_nu, L)), t64_cell_bytes(lm));
     }
     IRS_CUDA(cudaEventRecord(ctx->ev[0], st));
     double* d_grid = (double*)workspace(ctx, "grid", n_nu * sizeof(double));
@@ -837,7 +851,8 @@ static void forward_pass(irs_ctx* ctx, const irs_profile* profs, int n_prof, con
 }
 
 // ------------------------------------------------------------ Jacobian
-static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, std::initializer_list<const char*> mine);
+static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, size_t far_prof,
+                             std::initializer_list<const char*> mine);
 
 static int64_t state_size(const irs_state_spec& sp, int n_lev) {
     return (sp.include_temperature ? n_lev : 0) + (int64_t)sp.n_retrieved * n_lev + (sp.include_tsfc ? 1 : 0) +
@@ -927,9 +942,13 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
     for (auto& l : ctx->lists) max_list = std::max<int64_t>(max_list, l.n);
     int64_t total_lines = 0;
     for (auto& l : ctx->lists) total_lines += l.n;
-    const size_t per_prof = (size_t)L * total_lines * kJgLineBytes + (size_t)n_out * L * n_nu * 4 + (size_t)n_state * n_nu * 4 +
-                            (size_t)n_nu * 8 + (size_t)n_state * n_ch * 4;
-    const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof, {"jg_params", "jg_out", "jg_D", "jg_K", "jg_far", "I"});
+    size_t per_prof = (size_t)L * total_lines * kJgLineBytes + (size_t)n_out * L * n_nu * 4 + (size_t)n_state * n_nu * 4 +
+                      (size_t)n_nu * 8 + (size_t)n_state * n_ch * 4, n_lists = 0;
+    for (auto& l : ctx->lists) n_lists += l.n > 0 ? 1 : 0;
+    if (o.line_mixing == IRS_LM_RELMAT_VPY || o.line_mixing == IRS_LM_RELMAT_VPW) per_prof += (size_t)L * n_nu * 24;
+    const size_t far_prof = L * n_lists * tree_leaves(n_nu) * jg_cell_bytes(o.line_mixing == IRS_LM_PER_LINE_Y);
+    const int chunk = profiles_per_pass(ctx, n_prof, L, per_prof, far_prof,
+                                        {"jg_params", "jg_out", "jg_D", "jg_K", "jg_far", "I", "lm_pert"});
     const long long k_state = rows ? 1 : n_ch, k_chan = rows ? n_state : 1;  // strides of K
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
         const int np = std::min(chunk, n_prof - p0);
@@ -1053,9 +1072,9 @@ static void jacobian_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, 
             const int npl = np * L, n_strips = (int)((n_nu + kTrStrip - 1) / kTrStrip), n_leaves = n_strips * kTrLeaves;
             std::vector<int> first(npl + 1, 0);
             for (int q = 0; q < npl; ++q) first[q + 1] = first[q] + pl.pl_segs[q].y;
-            const size_t cell_bytes = (size_t)jg_sums(lm) * kTrNodes * sizeof(float) + sizeof(int4);
-            const size_t max_cells = std::min((size_t)nseg * n_leaves, ctx->strip_buf_max / cell_bytes);
-            char* fbuf = (char*)workspace(ctx, "jg_far", max_cells * cell_bytes);
+            const size_t cell_bytes = jg_cell_bytes(lm);
+            const size_t max_cells = far_cells(ctx, "jg_far", (size_t)nseg * n_leaves, cell_bytes);
+            char* fbuf = (char*)ctx->work["jg_far"].p;
             for (int pa = 0; pa < npl;) {
                 int pb = pa;
                 const int s_a = first[pa];
@@ -1208,8 +1227,10 @@ static void collect_times(irs_ctx* ctx) {
 // Profiles per pass: bounded by device memory and by the grid limits of the per-segment and
 // per-(profile, layer) launches (65535 in y).  Memory: 60% of what is free plus the context's
 // own workspaces, and 80% of what is free plus those that this pass reuses (`mine`; what
-// another path's batch left behind stays with it).
-static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, std::initializer_list<const char*> mine) {
+// another path's batch left behind stays with it).  A profile takes per_prof bytes, and far_prof
+// of the far field's buffer until that has its largest size.
+static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, size_t far_prof,
+                             std::initializer_list<const char*> mine) {
     if (n_prof == 1) return 1;  // whatever is free (asking takes 70 us, a scene 300)
     int n_lists = 0;
     for (auto& l : ctx->lists) n_lists += l.n > 0 ? 1 : 0;
@@ -1220,7 +1241,9 @@ static int profiles_per_pass(irs_ctx* ctx, int n_prof, int L, size_t per_prof, s
         for (const char* m : mine) reuse += w.first == m ? w.second.bytes : 0;
     }
     const size_t bytes = std::min((free_b + own) * 6 / 10, (free_b + reuse) * 8 / 10);
-    const size_t by_mem = std::max<size_t>(1, bytes / std::max<size_t>(per_prof, 1));
+    const size_t growing = bytes / std::max<size_t>(per_prof + far_prof, 1);
+    const size_t full = bytes > ctx->strip_buf_max ? (bytes - ctx->strip_buf_max) / std::max<size_t>(per_prof, 1) : 0;
+    const size_t by_mem = std::max<size_t>(1, std::max(growing, full));
     const size_t by_grid = std::max<size_t>(1, 65535 / (size_t)std::max(1, L * std::max(n_lists, 1)));
     return (int)std::min<size_t>((size_t)n_prof, std::min(by_mem, by_grid));
 }
@@ -1242,10 +1265,28 @@ static void forward_device(irs_ctx* ctx, const irs_profile* profs, int n_prof, c
     int64_t total_lines = 0;
     for (auto& l : ctx->lists) total_lines += l.n;
     const bool mixed = o.precision != IRS_FP64;
-    const size_t per_prof = (size_t)L * total_lines * (mixed ? 1 + kLpMixedBytes : 1 + kLpF64 * sizeof(double)) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
-                            (size_t)ig.g.n * 8;
-    const int chunk = mixed ? profiles_per_pass(ctx, n_prof, L, per_prof, {"tau", "lpmx", "keep", "I", "fw_far", "fw_cell_idx"})
-                            : profiles_per_pass(ctx, n_prof, L, per_prof, {"tau", "lp64", "keep", "I", "t64_far"});
+    size_t per_prof = (size_t)L * total_lines * (mixed ? 1 + kLpMixedBytes : 1 + kLpF64 * sizeof(double)) + (size_t)L * ig.g.n * (mixed ? 4 : 8) +
+                      (size_t)ig.g.n * 8, far_prof = 0;
+    if (o.line_mixing == IRS_LM_RELMAT_VPY || o.line_mixing == IRS_LM_RELMAT_VPW) per_prof += (size_t)L * ig.g.n * 16;
+    if (o.method != IRS_PSEUDOVOIGT && o.precision != IRS_MIXED_DIRECT) {
+        size_t n_lists = 0;
+        double shift = 0.0, cell, off;
+        for (auto& l : ctx->lists) {
+            n_lists += l.n > 0 ? 1 : 0;
+            shift = std::max(shift, l.max_abs_shift);
+        }
+        const bool lm = o.line_mixing == IRS_LM_PER_LINE_Y;
+        if (mixed) {
+            per_prof += L * n_lists * cell_layout(ig.g.n, (o.cutoff + shift) / ig.dnu_hi + 2.0, cell, off).n * sizeof(int);
+            far_prof = L * n_lists * tree_leaves(ig.g.n) * fw_cell_bytes(lm);
+        } else {
+            far_prof = L * n_lists * t64_groups(ig.g.n, t64_leaf_points(ig.g.n, L)) * t64_cell_bytes(lm);
+        }
+    }
+    const int chunk = mixed ? profiles_per_pass(ctx, n_prof, L, per_prof, far_prof,
+                                                {"tau", "lpmx", "keep", "I", "fw_far", "fw_cell_idx", "lm_pert", "lm_sv"})
+                            : profiles_per_pass(ctx, n_prof, L, per_prof, far_prof,
+                                                {"tau", "lp64", "keep", "I", "t64_far", "lm_pert", "lm_sv"});
     for (int p0 = 0; p0 < n_prof; p0 += chunk) {
         const int np = std::min(chunk, n_prof - p0);
         forward_pass(ctx, profs + p0, np, s, o, d_R + (size_t)p0 * ch.n, d_BT + (size_t)p0 * ch.n);
