@@ -488,6 +488,7 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
                 linesum_f64_kernel<2><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride, du);
             else
                 linesum_f64_kernel<3><<<g2, 256, 0, st>>>(d_segs, d_count, d_pl, o64, d_grid, n_nu, o.cutoff, o.x_far, (double*)d_tau, d_pert, pstride, du);
+            check_launch(ctx);
         }
     } else {
         const float cut_g = (float)(o.cutoff / dnu_g);
@@ -508,9 +509,9 @@ static void* run_linesum(irs_ctx* ctx, Plan& pl, const double* d_grid, int64_t n
             else if (d_pert) IRS_MX(3, false, true);
             else IRS_MX(3, false, false);
 #undef IRS_MX
+            check_launch(ctx);
         }
     }
-    check_launch(ctx);
     return d_tau;
 }
 
