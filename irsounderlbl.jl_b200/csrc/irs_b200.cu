@@ -141,7 +141,7 @@ static void validate_options(const irs_fm_options& o) {
     IRS_REQUIRE(o.method >= 1 && o.method <= 3, "method must be 1 (Weideman), 2 (PseudoVoigt) or 3 (FullFaddeeva)");
     IRS_REQUIRE(o.precision == IRS_FP64 || o.precision == IRS_MIXED || o.precision == IRS_MIXED_DIRECT,
                 "precision must be IRS_FP64, IRS_MIXED or IRS_MIXED_DIRECT");
-    IRS_REQUIRE(o.cutoff > 0.0, "cutoff must be positive");
+    IRS_REQUIRE(o.cutoff > 0.0 && std::isfinite(o.cutoff), "cutoff must be positive and finite");
     IRS_REQUIRE(o.apodization >= 0 && o.apodization <= 3, "unknown apodization");
     IRS_REQUIRE(o.T_method == 0 || o.T_method == 1, "T_method must be :logp_at_pcg or :mass_weighted");
     IRS_REQUIRE(o.source_function == 0 || o.source_function == 1, "source_function must be :cim or :toon");
