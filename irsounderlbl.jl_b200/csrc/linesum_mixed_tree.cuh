@@ -471,20 +471,24 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
                 const float4 f = T.fu[k], p = T.p0[k], p1 = T.p1[k];
                 const int4 cr = T.cr[k];
                 const int rl = cr.w & 255, rh = cr.w >> 8;  // rh = -1: none (arithmetic shift)
-                const float d0 = (pl0 - f.x) - f.y, g = LM ? T.fg[k] : 0.f;
+                const float g = LM ? T.fg[k] : 0.f;
                 const float c1 = fmaf(2.5f, p.y, 1.5f), c2 = fmaf(3.f, p.y, 2.25f);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
+                    // from each point's own position: the first subtraction is exact, and the second
+                    // rounds at the size of d (an offset from the lane's first point would round at
+                    // up to 128 steps: 2e-5 of the value half a step from a centre)
+                    const float2 dn = __fadd2_rn(__fadd2_rn(make_float2(pl0 + 64.f * h, pl0 + 64.f * h + 32.f), make_float2(-f.x, -f.x)),
+                                                 make_float2(-f.y, -f.y));
                     if (rh < 2 * h || rl > 2 * h + 1) {  // warp-uniform: no core point in these rows
-                        const float2 ds = __fadd2_rn(make_float2(d0, d0), make_float2(64.f * h + 32.f, 64.f * h));
+                        const float2 ds = make_float2(dn.y, dn.x);
                         const float2 es = __ffma2_rn(ds, ds, make_float2(f.z, f.z));
                         const float R = rcp_fast(es.x * es.y);
                         const float2 r = __fmul2_rn(es, make_float2(R, R));
                         acc[h] = __ffma2_rn(make_float2(f.w, f.w), r, acc[h]);
-                        if (LM) dsp[h] = __ffma2_rn(__fmul2_rn(make_float2(g, g), make_float2(ds.y, ds.x)), r, dsp[h]);
+                        if (LM) dsp[h] = __ffma2_rn(__fmul2_rn(make_float2(g, g), dn), r, dsp[h]);
                         continue;
                     }
-                    const float2 dn = __fadd2_rn(make_float2(d0, d0), make_float2(64.f * h, 64.f * h + 32.f));
                     const float2 d2 = __fmul2_rn(dn, dn);
                     const float2 X = __fmul2_rn(d2, make_float2(p.x, p.x));
                     const float2 m = __fadd2_rn(X, make_float2(p.y, p.y));
