@@ -37,8 +37,11 @@ import numpy as np
 ROOT = Path(__file__).resolve().parent
 N_PROF = 6
 GLOBAL_BATCH = 4 * N_PROF  # profiles per step over all GPUs: the six AFGL profiles x 4
-FAR_PAIR_FLOPS = 10     # d (2), d^2, d^2+b^2, rcp, pedestal FMA (2), value FMA (2), accumulate
-CORE_PAIR_FLOPS = 70    # far-pair ops + FP32 Faddeeva (continued fraction / Weideman-16 branch)
+# FP32 operations (FMA 2) that the mixed line sum executes per evaluated (line, point or node) and
+# on top of that per pair within a Faddeeva core: the solution of the two windows counted in
+# profiles/linesum_iasi400k.txt
+EVAL_FLOPS = 10.78
+CORE_FLOPS = 20.6
 FP32_LANES = 148 * 128  # B200: 148 SMs x 128 FP32 lanes
 
 
@@ -141,6 +144,12 @@ def _traffic_from_profiles():
             except ValueError:
                 return None
     return None
+
+
+def line_sum_flops(evaluated, core):
+    """FP32 operations of a mixed line sum: near lines are evaluated at every point of their
+    block, far lines at their blocks' 16 nodes (the algorithmic pair count is larger)."""
+    return EVAL_FLOPS * evaluated + CORE_FLOPS * core
 
 
 def cpu_sample(seconds_target: float = 8.0):
@@ -509,7 +518,7 @@ def main():
                               method=pkg.FullFaddeeva, **_workload_kw())
             t = ctx.stage_times()
             print(json.dumps({"precision": prec, "line_sum_ms": t.line_sum_ms, "pairs": t.pairs,
-                              "core_pairs": t.core_pairs}), flush=True)
+                              "core_pairs": t.core_pairs, "evaluated_pairs": t.evaluated_pairs}), flush=True)
         ctx.close()
         return
 
@@ -615,9 +624,7 @@ def main():
     pairs, core, evald = st.pairs, st.core_pairs, st.evaluated_pairs
     launches_per_step = st.launches
     t_ls = acc["line_sum_ms"] / 1e3
-    # FLOPs of the pair evaluations the kernel issued: near lines at every block point,
-    # far lines at their blocks' 16 nodes (the algorithmic pair count is larger)
-    flops = FAR_PAIR_FLOPS * (evald - core) + CORE_PAIR_FLOPS * core
+    flops = line_sum_flops(evald, core)
     clocks = clk.summary()
     f_sm = (clocks["sm_mhz"] or 1965.0) * 1e6
     peak = FP32_LANES * 2 * f_sm / 1e12
@@ -698,7 +705,7 @@ def main():
                          "bt_rms_mixed_vs_fp64_K": bt_rms, "bt_max_mixed_vs_fp64_K": bt_max,
                          "bt_max_far_field_vs_direct_K": far_max,
                          "work": {"pairs": pairs, "evaluated_pairs": evald, "core_pairs": core,
-                                  "far_flops": FAR_PAIR_FLOPS, "core_flops": CORE_PAIR_FLOPS}},
+                                  "eval_flops": EVAL_FLOPS, "core_flops": CORE_FLOPS}},
             "cpu_baseline": cpu,
             "e2e": e2e,
             "gpu_launches": int(launches_per_step * args.steps),
