@@ -37,9 +37,10 @@ extern "C" {
 
 /* arithmetic of the line sum */
 #define IRS_FP64          0   /* FP64 everywhere (distant lines' wings interpolated to rounding) */
-#define IRS_MIXED         1   /* FP32 Faddeeva + Kahan-compensated FP32 line sum; the far
-                                 wings of lines >= 640 grid points from a 256-point block
-                                 are summed at 8 Chebyshev nodes and interpolated        */
+#define IRS_MIXED         1   /* FP32 Faddeeva + Kahan-compensated FP32 line sum; on a tree of
+                                 blocks of 4096 to 128 grid points, the wings of lines two
+                                 half-widths or more from a block's centre (and their cores
+                                 off it) are summed at 16 Chebyshev nodes and interpolated */
 #define IRS_MIXED_DIRECT  2   /* as IRS_MIXED with every (point, line) pair evaluated   */
 
 /* HITRANLine, src/HITRAN/linelist.jl:20-31 (isbits, 56 bytes): a Julia

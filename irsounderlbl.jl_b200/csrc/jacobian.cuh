@@ -9,8 +9,9 @@
 //   RTE Jacobian                 schwarzschild_jacobian.jl:66-266 (jg_rte_kernel)
 //   channel tail K = dBT/dR . resample . ILS . dI/dx      vmr_jacobian.jl:359-503
 //                                (jg_channel_kernel)
-// The line sum and the channel contraction are FP32 (Kahan-compensated tile sums);
-// the optical-depth sums, transmittances and radiance derivatives are FP64.
+// The line sum is FP32 (the tile sums of the values Kahan-compensated, those of the derivatives
+// plain), and so is the channel contraction (plain sums); the optical-depth sums,
+// transmittances and radiance derivatives are FP64.
 #pragma once
 #include <type_traits>
 

@@ -21,14 +21,14 @@
 //            the pedestal nearly cancel): per-pair tests
 // Pedestals of fast and core lines are quadratics in the point index, summed per lane.
 //
-// Bound by issue (81 % of the slots in both kernels).  Measured on a B200 (far + near lines),
+// Bound by issue (78 to 82 % of the slots in both kernels).  Measured on a B200 (far + near lines),
 // against a 2048-point strip pre-pass, each warp's 8 far nodes from 320 points, window searches
-// and per-row core evaluation: six IASI profiles, 400,000 lines 10.3 + 95.2 -> 15.0 + 60.0 ms;
-// two CrIS long-wave profiles with VP_Y 0.64 + 4.19 -> 0.87 + 1.94 ms; one scene of the
-// 5,000-line list 30 + 236 -> 67 + 122 us.  Of the 60 ms the cores take 29 (half of it the
-// points with |x| + y < 15), the cutoff edges 7, the interpolation 2, staging and the
-// segments' fixed work the rest.  64 registers at four CTAs per SM; three CTAs (80 registers, no
-// spills) 62.8 ms.
+// and per-row core evaluation: six IASI profiles, 400,000 lines 10.3 + 95.2 -> 15.0 + 61.1 ms;
+// two CrIS long-wave profiles with VP_Y 0.64 + 4.19 -> 0.87 + 1.97 ms; one scene of the
+// 5,000-line list 30 + 236 -> 67 + 124 us.  Of the 61 ms the cores take 30 (half of it the points
+// with |x| + y < 15; 1.1 the core rows' own offsets and the floor of their quotient), the cutoff
+// edges 7, the interpolation 2, staging and the segments' fixed work the rest.  64 registers at
+// four CTAs per SM; three CTAs (80 registers, no spills) 62.8 ms against 60.0.
 #pragma once
 #include "linesum_tree32.cuh"
 

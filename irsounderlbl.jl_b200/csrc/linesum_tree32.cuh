@@ -63,7 +63,8 @@ __global__ void __launch_bounds__(256) cell_index_kernel(const double* __restric
 
 // The far lines of the block of points [cb, cb + 2 h): index ranges [x, y) and [z, w)
 // (empty at the centre when the cutoff or the core leaves none).  R = max(2 h, core reach + h)
-// + m keeps every core off the block, m (>= twice the largest shift) covers U against V.
+// + m keeps every core off the block; m, the segment's largest shift and two points, covers U
+// against V (the keys are unshifted, so their order is exact) and the rounding of the bounds.
 __device__ __forceinline__ int4 tree_ranges(const CellIndex& ci, const int* row, float cb, float h, float cut, float m,
                                             float reach) {
     const float c = cb + h - 0.5f, R = fmaxf(2.f * h, reach + h) + m;
