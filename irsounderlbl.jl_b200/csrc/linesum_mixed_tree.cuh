@@ -18,7 +18,11 @@
 //            (wing: n = q = 1), packed, one reciprocal for two points; the points with
 //            |x| + y < 15 come from a buffer evaluated lane-parallel
 //   general  core and cutoff edge, or a cutoff within 8 times the core's reach (where H and
-//            the pedestal nearly cancel): per-pair tests
+//            the pedestal nearly cancel): per-pair tests, the continued fraction inline.  (With
+//            the rule at 8 times the reach and half a leaf, every core of a step of 0.05 to 0.1
+//            cm^-1 was general: 5,000 lines x 2,000 points 0.81 / 1.06 ms, now 0.72 / 0.88; with m^3
+//            of the quotient in range up to |x| = 1.4e3 only, x_far = 3000 took 0.70 ms for
+//            34,801 points, now 0.50.)
 // Pedestals of fast and core lines are quadratics in the point index, summed per lane.
 //
 // Bound by issue (78 to 82 % of the slots in both kernels).  Measured on a B200 (far + near lines),
@@ -306,11 +310,14 @@ __global__ void __launch_bounds__(kFwTreeWarps * 32, ANY_LM ? 6 : 10) fw_tree_wa
 }
 
 // ------------------------------------------------------------------ near lines
+// The core's quotient in units of s = 2^-14 (m s, q s^2, n s^2, K s: the same roundings), so that m^3
+// of two points is in range up to |x| = 1.8e5 instead of 1.4e3
+constexpr float kFwScale = 6.103515625e-05f;
 constexpr int kFwBuf = 160;  // 512 (1.1 KB more a warp) measured slower, 61.1 against 60.0 ms on the IASI case
 template <bool LM>
 struct FwTile {
     float4 fu[32];   // uh, ul, b2, a
-    float4 p0[32];   // edge: c1, c0, g, -; core: fx^2, y^2, K = a fx^2, dfar^2; general: c1, c0, dfar^2, An
+    float4 p0[32];   // edge: c1, c0, g, -; core: s fx^2, s y^2, s K (K = a fx^2), dfar^2; general: c1, c0, dfar^2, An
     float4 p1[32];   // core, general: fx, y, An, Yw
     float fg[LM ? 32 : 1];
     int4 cr[32];     // core: inner points [x, y], offset in cw (-1: not held), rows lo | hi << 8
@@ -347,13 +354,13 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
             df = lp.df[q];
             const float dist = fabsf(uh - kCentre);
             const bool wing = dist > df + kHalf, in = dist + kHalf <= cut;
-            cls = dist > cut + kHalf ? 0 : wing ? (in ? 1 : 2) : (in && cut >= 8.f * (df + kHalf) ? 3 : 4);
+            cls = dist > cut + kHalf ? 0 : wing ? (in ? 1 : 2) : (in && cut >= 8.f * (df + 0.5f) ? 3 : 4);
             if (cls) {
                 a0 = lp.p0[q];
                 if (cls >= 3) a1 = lp.p1[q];
                 if (LM) a2 = lp.p2[q];
-                // the quotient's m^3 for two points stays in range
-                if (cls == 3 && (METHOD != 3 || x_far2 + a1.w * a1.w > 2.0e6f)) cls = 4;
+                // the quotient's (m s)^3 for two points stays in range
+                if (cls == 3 && (METHOD != 3 || x_far2 + a1.w * a1.w > 2.0e6f / kFwScale)) cls = 4;
             }
         }
         const unsigned m1 = __ballot_sync(kFull, cls == 1), m2 = __ballot_sync(kFull, cls == 2);
@@ -398,7 +405,8 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
             if (cls == 2) T.p0[pos] = make_float4(a0.z, a0.w, 0.f, 0.f);
             else if (cls == 3) {
                 const float fx2 = a1.z * a1.z;
-                T.p0[pos] = make_float4(fx2, a1.w * a1.w, a1.y * a1.w * (float)kInvSqrtPi, df * df);
+                T.p0[pos] = make_float4(kFwScale * fx2, kFwScale * (a1.w * a1.w), kFwScale * (a1.y * a1.w * (float)kInvSqrtPi),
+                                        df * df);
                 T.p1[pos] = make_float4(a1.z, a1.w, a1.y, a2.y);
                 const float c = uh + ul;
                 const int rl = (int)fminf(fmaxf((c - df) * (1.f / 32.f) - 0.1f, 0.f), 4.f);  // rows the core reaches
@@ -472,7 +480,8 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
                 const int4 cr = T.cr[k];
                 const int rl = cr.w & 255, rh = cr.w >> 8;  // rh = -1: none (arithmetic shift)
                 const float g = LM ? T.fg[k] : 0.f;
-                const float c1 = fmaf(2.5f, p.y, 1.5f), c2 = fmaf(3.f, p.y, 2.25f);
+                constexpr float s1 = kFwScale, s2 = kFwScale * kFwScale;  // X, m times s; n, q times s^2
+                const float c1 = fmaf(2.5f * s1, p.y, 1.5f * s2), c2 = fmaf(3.f * s1, p.y, 2.25f * s2);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     // from each point's own position: the first subtraction is exact, and the second
@@ -492,16 +501,16 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
                     const float2 d2 = __fmul2_rn(dn, dn);
                     const float2 X = __fmul2_rn(d2, make_float2(p.x, p.x));
                     const float2 m = __fadd2_rn(X, make_float2(p.y, p.y));
-                    float2 nn = __ffma2_rn(m, m, __ffma2_rn(X, make_float2(-1.5f, -1.5f), make_float2(c1, c1)));
-                    float2 q = __ffma2_rn(m, m, __ffma2_rn(X, make_float2(-3.f, -3.f), make_float2(c2, c2)));
+                    float2 nn = __ffma2_rn(m, m, __ffma2_rn(X, make_float2(-1.5f * s1, -1.5f * s1), make_float2(c1, c1)));
+                    float2 q = __ffma2_rn(m, m, __ffma2_rn(X, make_float2(-3.f * s1, -3.f * s1), make_float2(c2, c2)));
                     const bool cx = d2.x <= p.w, cy = d2.y <= p.w;
                     nn.x = cx ? nn.x : 1.f;
                     nn.y = cy ? nn.y : 1.f;
                     q.x = cx ? q.x : 1.f;
                     q.y = cy ? q.y : 1.f;
                     // m q is zero where y is lost beside x = 0 or x^2 = 3/2: points that the buffer
-                    // replaces below, but the reciprocal is their neighbours' too.  Beyond those
-                    // points it is above 1 (1e-8 with x_far = 0)
+                    // replaces below, but the reciprocal is their neighbours' too.  Any other
+                    // point's is far above the floor (3e-7 at |x| + y = 15)
                     float2 den = __fmul2_rn(m, q);
                     den.x = fmaxf(den.x, 1e-18f);
                     den.y = fmaxf(den.y, 1e-18f);
@@ -509,8 +518,8 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
                     const float2 r = __fmul2_rn(make_float2(den.y, den.x), make_float2(R, R));
                     float2 v = __fmul2_rn(__fmul2_rn(nn, make_float2(p.z, p.z)), r), vd = make_float2(0.f, 0.f);
                     if (LM) {  // Im w = (x/sqrt(pi)) (m^2 - 5/2 x^2 + 3/2 y^2 + 3/2) / (m q); wing: x / (sqrt(pi) m)
-                        const float c3 = fmaf(1.5f, p.y, 1.5f), kd = p1.w * (float)kInvSqrtPi * p1.x;
-                        float2 ni = __ffma2_rn(m, m, __ffma2_rn(X, make_float2(-2.5f, -2.5f), make_float2(c3, c3)));
+                        const float c3 = fmaf(1.5f * s1, p.y, 1.5f * s2), kd = s1 * (p1.w * (float)kInvSqrtPi * p1.x);
+                        float2 ni = __ffma2_rn(m, m, __ffma2_rn(X, make_float2(-2.5f * s1, -2.5f * s1), make_float2(c3, c3)));
                         ni.x = cx ? ni.x : 1.f;
                         ni.y = cy ? ni.y : 1.f;
                         vd = __fmul2_rn(__fmul2_rn(__fmul2_rn(ni, make_float2(kd, kd)), dn), r);
@@ -545,25 +554,32 @@ __device__ __forceinline__ void fw_segment(const SegDev& sg, const LpOutMixed& l
         }
         for (int k = e3; k < e4; ++k) {  // general lines
             const float4 f = T.fu[k], p = T.p0[k], p1 = T.p1[k];
-            const float g = LM ? T.fg[k] : 0.f;
+            const float g = LM ? T.fg[k] : 0.f, y2 = p1.y * p1.y;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float d = ((pl0 + 32.f * q) - f.x) - f.y, d2 = d * d;
-                if (d2 > cut2) continue;
                 const float ped = fmaf(p.x, d2, p.y);
+                const bool core = d2 <= p.z;  // |x| <= x_far
                 float v, vd = 0.f;
-                if (d2 <= p.z) {  // |x| <= x_far
-                    if (METHOD == 3) {
-                        const float2 w = faddeeva32(d * p1.x, p1.y);
-                        v = fmaf(p.w, w.x, ped);
-                        if (LM) vd = p1.w * w.y;
-                    } else {
-                        v = fmaf(p.w, weideman24_32(d * p1.x, p1.y), ped);
-                    }
-                } else {
+                if (METHOD == 3) {
+                    // the wing at every lane; rows holding a core point (warp-uniform) the two-level
+                    // continued fraction too, the points nearer through the shared routine
                     const float r = rcp_fast(d2 + f.z);
                     v = fmaf(f.w, r, ped);
                     if (LM) vd = g * d * r;
+                    if (__any_sync(kFull, core)) {
+                        const float x = d * p1.x;
+                        float2 w = faddeeva_cf2(x, p1.y, y2);
+                        if (core && fabsf(x) + p1.y < 15.f) w = faddeeva32(x, p1.y);
+                        if (core) {
+                            v = fmaf(p.w, w.x, ped);
+                            if (LM) vd = p1.w * w.y;
+                        }
+                    }
+                    if (d2 > cut2) v = vd = 0.f;
+                } else {
+                    if (d2 > cut2) continue;
+                    v = core ? fmaf(p.w, weideman24_32(d * p1.x, p1.y), ped) : fmaf(f.w, rcp_fast(d2 + f.z), ped);
                 }
                 if (q & 1) {
                     acc[q >> 1].y += v;
