@@ -8,8 +8,8 @@
 //  * linesum_f64_kernel -- the plain FP64 GPU kernel: one thread per grid point,
 //    a binary search per point and species for the window on the shifted centres,
 //    FP64 arithmetic and IEEE division, exactly the reference kernel's structure.  It
-//    serves PseudoVoigt and grids that are not uniform; the FP64 sum of the other methods
-//    on a uniform grid is tree64_leaf_kernel's.
+//    serves PseudoVoigt, cross sections of short lists and grids that are not uniform; the
+//    FP64 sum of the other methods on a uniform grid is tree64_leaf_kernel's.
 //  * linesum_mixed_kernel -- FP32 + Kahan, every line of the window evaluated at every
 //    point (IRS_MIXED_DIRECT), and PseudoVoigt.  IRS_MIXED's sum is fw_leaf_kernel's
 //    (linesum_mixed_tree.cuh).
